@@ -173,7 +173,7 @@ DIRECT_NOALLOC_MAX_SOURCES = _header_define("FMM_DIRECT_NOALLOC_MAX_SOURCES")
 
 def direct_noalloc(xt, xs, qs, eps2=0.0, device=0):
     """direct() for callers that cannot allocate device memory (fmm_b200_direct_noalloc):
-    the same result, staged through a static 3.75 MiB device array instead of per-call
+    the same result, staged through a static 4.91 MiB device array instead of per-call
     allocations.  At most DIRECT_NOALLOC_MAX_TARGETS targets and DIRECT_NOALLOC_MAX_SOURCES
     sources; calls on one device share the array and must not overlap."""
     lib = load_library()

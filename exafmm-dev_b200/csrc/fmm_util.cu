@@ -4,6 +4,7 @@
 // library's kernel launches.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <mutex>
@@ -19,37 +20,57 @@ using namespace fmmb200;
 
 namespace {
 
+// FP64 direct sum: a block takes 64 targets and one slice of the sources, its four groups of
+// 64 threads every fourth source of each staged tile; the groups' sums meet in shared
+// memory, the slices' in k_direct_sum, in slice order.  Bound by the FP64 pipe (about 22
+// operations a pair with the reciprocal square root).  The slices fill the GPU whatever the
+// number of targets: with a thread per target and no slices, 1,024 targets were four blocks
+// (2^20 sources: 183 ms; the whole call now takes 4.5 ms, 2.5 ms of it the copies).
 constexpr int kDirTile = 256;
+constexpr int kDirTargets = 64;
+constexpr int kDirBlocks = 148 * 4;  // blocks wanted on the GPU: one wave at 4 per SM
 
-__global__ void __launch_bounds__(kDirTile)
+// slices of the sources for nt targets: at most one wave of blocks, no slice shorter than a
+// tile (so slices > 1 means at most kDirPartials partial sums)
+constexpr size_t kDirPartials = 4 * (size_t)kDirTargets * kDirBlocks;
+int direct_slices(int nt, int ns) {
+  const int s = std::min(kDirBlocks / ceil_div(nt, kDirTargets), ceil_div(ns, kDirTile));
+  return std::max(s, 1);
+}
+
+// the sums of slice blockIdx.y into out[4 (blockIdx.y nt + target)]
+__global__ void __launch_bounds__(kDirTile, 4)
     k_direct(int nt, const double* __restrict__ xt, int ns, const double* __restrict__ xs,
-             const double* __restrict__ qs, double eps2, double* __restrict__ out) {
-  __shared__ double sh[kDirTile][4];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+             const double* __restrict__ qs, double eps2, int slice, double* __restrict__ out) {
+  __shared__ double2 sh[kDirTile][2];
+  const int i = blockIdx.x * kDirTargets + (threadIdx.x & (kDirTargets - 1));
+  const int sub = threadIdx.x / kDirTargets;
   double x = 0, y = 0, z = 0;
   if (i < nt) {
-    x = xt[3 * i];
-    y = xt[3 * i + 1];
-    z = xt[3 * i + 2];
+    x = xt[3 * (size_t)i];
+    y = xt[3 * (size_t)i + 1];
+    z = xt[3 * (size_t)i + 2];
   }
   double pot = 0, ax = 0, ay = 0, az = 0;
-  for (int j0 = 0; j0 < ns; j0 += kDirTile) {
-    const int j = j0 + threadIdx.x;
+  const long long first = (long long)blockIdx.y * slice;
+  const int end = (int)(first + slice < ns ? first + slice : ns);
+  for (long long j0 = first; j0 < end; j0 += kDirTile) {
+    const size_t j = (size_t)j0 + threadIdx.x;
     __syncthreads();
-    if (j < ns) {
-      sh[threadIdx.x][0] = xs[3 * j];
-      sh[threadIdx.x][1] = xs[3 * j + 1];
-      sh[threadIdx.x][2] = xs[3 * j + 2];
-      sh[threadIdx.x][3] = qs[j];
+    if (j < (size_t)end) {
+      sh[threadIdx.x][0] = make_double2(xs[3 * j], xs[3 * j + 1]);
+      sh[threadIdx.x][1] = make_double2(xs[3 * j + 2], qs[j]);
     }
     __syncthreads();
-    const int cnt = min(kDirTile, ns - j0);
-    for (int k = 0; k < cnt; k++) {
-      const double dx = sh[k][0] - x, dy = sh[k][1] - y, dz = sh[k][2] - z;
+    const int cnt = (int)(end - j0 < kDirTile ? end - j0 : kDirTile);
+#pragma unroll 4
+    for (int k = sub; k < cnt; k += kDirTile / kDirTargets) {
+      const double2 a = sh[k][0], b = sh[k][1];
+      const double dx = a.x - x, dy = a.y - y, dz = b.x - z;
       const double r2 = dx * dx + dy * dy + dz * dz + eps2;
       if (r2 != 0) {
-        const double inv = 1.0 / sqrt(r2);
-        const double qi = sh[k][3] * inv;
+        const double inv = rsqrt(r2);
+        const double qi = b.y * inv;
         const double inv3 = qi * inv * inv;
         pot += qi;
         ax += dx * inv3;
@@ -58,11 +79,46 @@ __global__ void __launch_bounds__(kDirTile)
       }
     }
   }
-  if (i < nt) {
-    out[4 * i] = pot;
-    out[4 * i + 1] = ax;
-    out[4 * i + 2] = ay;
-    out[4 * i + 3] = az;
+  __syncthreads();
+  sh[threadIdx.x][0] = make_double2(pot, ax);
+  sh[threadIdx.x][1] = make_double2(ay, az);
+  __syncthreads();
+  if (sub == 0 && i < nt) {
+    for (int g = 1; g < kDirTile / kDirTargets; g++) {
+      const double2 a = sh[threadIdx.x + g * kDirTargets][0],
+                    b = sh[threadIdx.x + g * kDirTargets][1];
+      pot += a.x;
+      ax += a.y;
+      ay += b.x;
+      az += b.y;
+    }
+    double* o = out + 4 * ((size_t)blockIdx.y * nt + i);
+    o[0] = pot;
+    o[1] = ax;
+    o[2] = ay;
+    o[3] = az;
+  }
+}
+
+__global__ void k_direct_sum(int n, int slices, const double* __restrict__ part,
+                             double* __restrict__ out) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  double v = 0;
+  for (int s = 0; s < slices; s++) v += part[(size_t)s * n + t];
+  out[t] = v;
+}
+
+// device arrays in, 4 nt sums out; part: room for 4 nt `slices` doubles (slices > 1)
+void launch_direct(int nt, const double* xt, int ns, const double* xs, const double* qs,
+                   double eps2, int slices, double* part, double* out, cudaStream_t st) {
+  const int len = ceil_div(ceil_div(ns, slices), kDirTile) * kDirTile;
+  k_direct<<<dim3(ceil_div(nt, kDirTargets), slices), kDirTile, 0, st>>>(
+      nt, xt, ns, xs, qs, eps2, len, slices > 1 ? part : out);
+  FMM_LAUNCH_CHECK();
+  if (slices > 1) {
+    k_direct_sum<<<ceil_div(4LL * nt, 128), 128, 0, st>>>(4 * nt, slices, part, out);
+    FMM_LAUNCH_CHECK();
   }
 }
 
@@ -86,13 +142,13 @@ __global__ void __launch_bounds__(256) k_fma_probe(float* out, float s) {
 // The staging buffers of fmm_b200_direct (targets, sources, charges, output) live in one
 // fixed array in device memory instead of per-call cudaMalloc/cudaFree.  Layout for a call
 // (nt, ns), in doubles: targets [0, 3 nt), sources [3 nt, 3 nt + 3 ns), charges next (ns),
-// output next (4 nt): 7 nt + 4 ns doubles, at most 7 * 32768 + 4 * 65536 = 491,520
-// doubles (3.75 MiB) per device.  No part of it has to start at zero: a call copies in
+// output next (4 nt), the slices' partial sums next: at most 7 * 32768 + 4 * 65536 + 151,552
+// = 643,072 doubles (4.91 MiB) per device.  No part of it has to start at zero: a call copies in
 // every input it reads and the kernel writes every output that is copied back.
 constexpr int kNoAllocMaxTargets = FMM_DIRECT_NOALLOC_MAX_TARGETS;
 constexpr int kNoAllocMaxSources = FMM_DIRECT_NOALLOC_MAX_SOURCES;
 constexpr size_t kNoAllocDoubles =
-    7 * (size_t)kNoAllocMaxTargets + 4 * (size_t)kNoAllocMaxSources;
+    7 * (size_t)kNoAllocMaxTargets + 4 * (size_t)kNoAllocMaxSources + kDirPartials;
 static __device__ __align__(256) double g_direct_scratch[kNoAllocDoubles];
 
 constexpr int kNoAllocMaxDevices = 64;
@@ -156,8 +212,8 @@ int fmm_b200_direct_noalloc(int device, int nt, const double* xt, int ns, const 
       FMM_CUDA(cudaMemcpyAsync(dxs, xs, 24 * (size_t)ns, cudaMemcpyHostToDevice, st));
       FMM_CUDA(cudaMemcpyAsync(dqs, qs, 8 * (size_t)ns, cudaMemcpyHostToDevice, st));
     }
-    k_direct<<<ceil_div(nt, kDirTile), kDirTile, 0, st>>>(nt, dxt, ns, dxs, dqs, eps2, dout);
-    FMM_LAUNCH_CHECK();
+    double* part = dout + 4 * (size_t)nt;
+    launch_direct(nt, dxt, ns, dxs, dqs, eps2, direct_slices(nt, ns), part, dout, st);
     FMM_CUDA(cudaMemcpyAsync(out, dout, 32 * (size_t)nt, cudaMemcpyDeviceToHost, st));
     FMM_CUDA(cudaStreamSynchronize(st));
   } catch (const FmmError& e) {
@@ -178,7 +234,8 @@ int fmm_b200_direct(int device, int nt, const double* xt, int ns, const double* 
   try {
     FMM_CUDA(cudaSetDevice(device));
     DevArr<double> b;
-    b.ensure(3 * (size_t)nt + 4 * (size_t)ns + 4 * (size_t)nt);
+    const int slices = direct_slices(nt, ns);
+    b.ensure(3 * (size_t)nt + 4 * (size_t)ns + 4 * (size_t)nt * (slices > 1 ? 1 + slices : 1));
     double *dxt = b.p, *dxs = b.p + 3 * (size_t)nt, *dqs = dxs + 3 * (size_t)ns,
            *dout = dqs + ns;
     FMM_CUDA(cudaMemcpy(dxt, xt, 24 * (size_t)nt, cudaMemcpyHostToDevice));
@@ -186,8 +243,7 @@ int fmm_b200_direct(int device, int nt, const double* xt, int ns, const double* 
       FMM_CUDA(cudaMemcpy(dxs, xs, 24 * (size_t)ns, cudaMemcpyHostToDevice));
       FMM_CUDA(cudaMemcpy(dqs, qs, 8 * (size_t)ns, cudaMemcpyHostToDevice));
     }
-    k_direct<<<ceil_div(nt, kDirTile), kDirTile>>>(nt, dxt, ns, dxs, dqs, eps2, dout);
-    FMM_LAUNCH_CHECK();
+    launch_direct(nt, dxt, ns, dxs, dqs, eps2, slices, dout + 4 * (size_t)nt, dout, nullptr);
     FMM_CUDA(cudaMemcpy(out, dout, 32 * (size_t)nt, cudaMemcpyDeviceToHost));
     b.release();
   } catch (const FmmError& e) {

@@ -329,8 +329,8 @@ int fmm_b200_server_destroy(fmm_b200_server* srv);
 int fmm_b200_direct(int device, int nt, const double* xt, int ns, const double* xs,
                     const double* qs, double eps2, double* out);
 /* fmm_b200_direct without any device allocation: same arguments, kernel and (bitwise)
- * result, with the device staging buffers in a static device array of 3.75 MiB (7 nt + 4 ns
- * doubles), which every GPU that loads this library holds until the process exits, instead
+ * result, with the device staging buffers in a static device array of 4.91 MiB (7 nt + 4 ns
+ * doubles and the source slices' partial sums), which every GPU that loads this library holds until the process exits, instead
  * of a cudaMalloc/cudaFree per call.  For callers that cannot allocate device memory while
  * they run: those whose device memory is all held by their own pool allocator, and those
  * that must not take the device-wide synchronisation that cudaMalloc/cudaFree imply while
