@@ -488,13 +488,13 @@ int fmm_b200_create(const fmm_b200_config* cfg, fmm_b200_solver** out) {
       d_.bodies_in.OP(); d_.bodies.OP(); d_.trg_s.OP(); d_.trg_e.OP(); d_.trg_out.OP();    \
       d_.cX.OP(); d_.box.OP(); d_.M.OP(); d_.L.OP(); d_.nX.OP(); d_.m0.OP();               \
       d_.pM.OP(); d_.pM2.OP(); d_.pC.OP(); d_.c_root_cells.OP(); d_.minmax_part.OP();      \
-      d_.k_rows.OP(); d_.k_cx.OP(); d_.k_trg.OP();                                         \
+      d_.k_rows.OP(); d_.k_cx.OP(); d_.k_trg.OP(); d_.m2l_rows.OP();                                         \
     } else {                                                                               \
       Solver<float>& d_ = *static_cast<Solver<float>*>((h)->base);                         \
       d_.bodies_in.OP(); d_.bodies.OP(); d_.trg_s.OP(); d_.trg_e.OP(); d_.trg_out.OP();    \
       d_.cX.OP(); d_.box.OP(); d_.M.OP(); d_.L.OP(); d_.nX.OP(); d_.m0.OP();               \
       d_.pM.OP(); d_.pM2.OP(); d_.pC.OP(); d_.c_root_cells.OP(); d_.minmax_part.OP();      \
-      d_.k_rows.OP(); d_.k_cx.OP(); d_.k_trg.OP();                                         \
+      d_.k_rows.OP(); d_.k_cx.OP(); d_.k_trg.OP(); d_.m2l_rows.OP();                                         \
     }                                                                                      \
   } while (0)
 

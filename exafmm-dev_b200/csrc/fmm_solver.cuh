@@ -196,6 +196,7 @@ template <typename T> struct Solver : SolverBase {
   DevArr<vec4<T>> bodies_in, bodies, trg_s, trg_e, trg_out, cX;
   DevArr<T> box;  // per root, 16 values: X0[3], R0, Xmin[3], Xmax[3]
   DevArr<T> M, L, nX;
+  DevArr<T> m2l_rows;  // spherical M2L: the multipoles by order (sph::col_idx)
   DevArr<T> m0;  // monopole per cell (structure pass)
   DevArr<T> pM, pM2, pC;  // periodic cell multipoles and per-shift M2L terms
   DevArr<int> c_root_cells;

@@ -425,6 +425,173 @@ __host__ __device__ __forceinline__ void m2l_pair_rot_out(const T* rho, const T*
   }
 }
 
+// The real harmonic factors of local_rho (up to rounding), all degrees n < P at sidx(n, m),
+// with the radial power inside the recurrence
+//   rho[n, m] = (2n - 1) (-x / r) rho[n-1, m] - (n - 1 + m)(n - 1 - m) / r^2 rho[n-2, m],
+// three operations per term (the factors (2n - 1)(-x / r) are shared by all m).
+template <typename T, int P>
+__host__ __device__ __forceinline__ void fold_rho(const Angles<T>& a, T invr, T* rho) {
+  const T xi = -a.x * invr, w = invr * invr, yi = a.y * invr;
+  T X[P];
+#pragma unroll
+  for (int n = 1; n < P; n++) X[n] = T(2 * n - 1) * xi;
+  T d = invr;  // rho[m, m] = (-1)^m P_m^m / r^(m+1)
+#pragma unroll
+  for (int m = 0; m < P; m++) {
+    T q = d, qm1 = 0;
+    rho[sidx(m, m)] = q;
+#pragma unroll
+    for (int n = m + 1; n < P; n++) {
+      const int c = (n - 1 + m) * (n - 1 - m);
+      const T qn = c ? fma(X[n], q, T(-c) * (w * qm1)) : X[n] * q;
+      qm1 = q;
+      q = qn;
+      rho[sidx(n, m)] = q;
+    }
+    // P_{m+1}^{m+1} = -(2m + 1) sin(alpha) P_m^m
+    d *= T(2 * m + 1) * yi;
+  }
+}
+
+// a complex value (a pair of registers the packed two-wide FP32 instructions take together)
+template <typename T> struct Cx {
+  T r, i;
+};
+// a.r += u m.r, a.i += v m.i, each rounded once; FP32 on the device: one packed instruction
+template <typename T>
+__host__ __device__ __forceinline__ void fold_fma(T u, T v, const Cx<T>& m, Cx<T>& a) {
+#ifdef __CUDA_ARCH__
+  if constexpr (sizeof(T) == 4) {
+    const float2 t = __ffma2_rn(make_float2(u, v), make_float2(m.r, m.i), make_float2(a.r, a.i));
+    a.r = t.x;
+    a.i = t.y;
+    return;
+  }
+#endif
+  a.r = fma(u, m.r, a.r);
+  a.i = fma(v, m.i, a.i);
+}
+
+// The M2L of m2l_pair in the source's azimuthal frame, the terms of m = +mu and m = -mu
+// folded.  Every term of output (j, k) carries the phase e^(i (m - k) beta) of its harmonic,
+// so with M'[n, mu] = M[n, mu] e^(i mu beta)
+//   L[j, k] += (-1)^j e^(-i k beta) A[j, k],
+//   A[j, k] = sum over n of rho[j+n, k] M'[n, 0]
+//           + sum over n, mu > 0 of (s rho[j+n, |k-mu|] + rho[j+n, k+mu]) Re M'[n, mu]
+//                               + i (s rho[j+n, |k-mu|] - rho[j+n, k+mu]) Im M'[n, mu],
+// s = (-1)^min(k, mu).  The two real factors depend on (j + n, k, mu) only, so they are formed
+// once for all (j, n) of one sum: a term costs two multiply-adds (the unfolded form takes
+// four), one for k = 0, whose factors are 2 rho[j+n, mu] and 0.
+// Outputs of the orders k in [K0, K1) into A at fold_idx; the phases of the source by one
+// rotation per mu; Mj the source's row by order (col_idx).
+__host__ __device__ constexpr int fold_idx(int P, int K0, int k, int j) {
+  int t = j - k;
+  for (int q = K0; q < k; q++) t += P - q;
+  return t;
+}
+// hide where a value came from (device): the compiler then forms values that depend on it
+// again instead of keeping them in registers across a long unrolled sum
+template <typename U> __host__ __device__ __forceinline__ void launder(U& v) {
+#ifdef __CUDA_ARCH__
+  if constexpr (sizeof(U) == 4) asm volatile("" : "+f"(v));
+  else asm volatile("" : "+d"(v));
+#endif
+}
+template <typename U> __host__ __device__ __forceinline__ void launder(const U*& v) {
+#ifdef __CUDA_ARCH__
+  asm volatile("" : "+l"(v));
+#endif
+}
+
+// Source coefficients by order: the coefficients (n, mu), n = mu .. P - 1, of one order mu
+// contiguous, each order padded to an even number, so that the sum over one mu reads whole
+// 16-byte pairs.  Offset of (n, mu) in reals, and a row's length (a multiple of 16 bytes).
+__host__ __device__ constexpr int col_idx(int P, int n, int mu) {
+  int t = 0;
+  for (int q = 0; q < mu; q++) t += (P - q + 1) / 2 * 2;
+  return 2 * (t + n - mu);
+}
+__host__ __device__ constexpr int col_len(int P) { return col_idx(P, P, P); }
+// coefficients p[0], p[1] (16 bytes in FP32 from a 16-byte boundary, two such in FP64)
+template <typename T>
+__host__ __device__ __forceinline__ void load_pair2(const T* p, Cx<T>& a, Cx<T>& b) {
+#ifdef __CUDA_ARCH__
+  if constexpr (sizeof(T) == 4) {
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    a.r = v.x, a.i = v.y, b.r = v.z, b.i = v.w;
+    return;
+  }
+#endif
+  load_pair(p, a.r, a.i);
+  load_pair(p + 2, b.r, b.i);
+}
+
+// the terms of the source orders MU, MU + 1, ... (a recursion over compile-time mu, so that
+// every index below is a constant however long the unrolled sum); (er, ei) = e^(i MU beta)
+template <typename T, int P, int K0, int K1, int MU>
+__host__ __device__ __forceinline__ void m2l_fold_from(const T* rho, T cb, T sb, T er, T ei,
+                                                       const T* Mj, Cx<T>* A) {
+  constexpr int NS = P - K0;  // source degrees n < NS reach these outputs
+  if constexpr (MU < NS) {
+    Cx<T> m[NS - MU + 1];  // (and the pad of an odd column)
+#pragma unroll
+    for (int n = MU; n < NS; n += 2) {
+      if (n + 1 < NS || sizeof(T) == 4) load_pair2(Mj + col_idx(P, n, MU), m[n - MU], m[n - MU + 1]);
+      else load_pair(Mj + col_idx(P, n, MU), m[n - MU].r, m[n - MU].i);
+    }
+    if (MU > 0) {
+#pragma unroll
+      for (int n = 0; n < NS - MU; n++) {
+        const T mr = m[n].r, mi = m[n].i;
+        m[n].r = mr * er - mi * ei;
+        m[n].i = mr * ei + mi * er;
+      }
+    }
+#pragma unroll
+    for (int k = K0; k < K1; k++) {
+#pragma unroll
+      for (int a = k + MU; a < P; a++) {
+        if (MU == 0) {
+          // (k = 0: half the term, doubled below with the terms of mu > 0)
+          const T p = k == 0 ? T(0.5) * rho[sidx(a, 0)] : rho[sidx(a, k)];
+#pragma unroll
+          for (int n = 0; n <= a - k; n++) fold_fma(p, p, m[n], A[fold_idx(P, K0, k, a - n)]);
+        } else if (k == 0) {
+          const T p = rho[sidx(a, MU)];
+#pragma unroll
+          for (int n = MU; n <= a; n++) {
+            Cx<T>& o = A[fold_idx(P, K0, 0, a - n)];
+            o.r = fma(p, m[n - MU].r, o.r);
+          }
+        } else {
+          const T p1 = rho[sidx(a, k + MU)], p2 = rho[sidx(a, MU >= k ? MU - k : k - MU)];
+          const bool neg = ((k < MU ? k : MU) & 1) != 0;
+          const T u = neg ? p1 - p2 : p1 + p2, v = neg ? -p2 - p1 : p2 - p1;
+#pragma unroll
+          for (int n = MU; n <= a - k; n++)
+            fold_fma(u, v, m[n - MU], A[fold_idx(P, K0, k, a - n)]);
+        }
+      }
+    }
+    m2l_fold_from<T, P, K0, K1, MU + 1>(rho, cb, sb, er * cb - ei * sb, er * sb + ei * cb, Mj,
+                                        A);
+  }
+}
+template <typename T, int P, int K0, int K1>
+__host__ __device__ __forceinline__ void m2l_fold(const T* rho, T cb, T sb, const T* Mj,
+                                                  Cx<T>* A) {
+#pragma unroll
+  for (int t = 0; t < fold_idx(P, K0, K1, K1); t++) A[t].r = A[t].i = T(0);
+  m2l_fold_from<T, P, K0, K1, 0>(rho, cb, sb, T(1), T(0), Mj, A);
+  if (K0 == 0) {
+#pragma unroll
+    for (int j = 0; j < P; j++) {
+      A[j].r += A[j].r;
+      A[j].i += A[j].i;
+    }
+  }
+}
+
 // Y[a, b] for any sign of b from the m >= 0 store (real parts yr, imaginary parts yi)
 template <typename T>
 __host__ __device__ __forceinline__ void yget(const T* yr, const T* yi, int a, int b, T& r,

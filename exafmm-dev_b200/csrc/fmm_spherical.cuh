@@ -7,8 +7,9 @@
 //        fixed order and the monopole in the reference's child order
 //        (include/up_down_pass.h:79-80 / LaplaceSphericalCPU.cxx:143).
 //   M2L  warp per target cell, lane per source cell, each pair contracted in the source's
-//        azimuthal frame with the harmonics and the local expansion held in registers,
-//        passes over the output degrees, one warp reduction per target.
+//        azimuthal frame with the +m and -m terms folded and the harmonics in registers, the
+//        local expansion summed in shared memory (FP64 above P = 8: unfolded, in passes over
+//        the output degrees).
 //   L2L  thread per cell, the parent's local staged in the thread's row of shared memory.
 //   L2P  thread per body, harmonics generated and consumed on the fly.
 // setRmax / R /= theta (include/up_down_pass.h:51-67, :81-82) are fused into P2M and M2M.
@@ -250,23 +251,221 @@ __global__ void __launch_bounds__(tr_threads<T>())
 }
 
 // ---------------------------------------------------------------- M2L
-// Warp per target, lane per source cell, harmonics and local expansion in registers, one
-// warp reduction per target cell at the end (either precision).  Each pair is contracted in
-// the source's azimuthal frame (m2l_pair_rot: real harmonic factors, half the multiply-adds
-// of the complex form).  The outputs are split into passes over their degree (separate
-// launches) so that each pass's registers stay within its block's share.
-// Passes over the output degrees.  Registers of a pass [J0, J1) (besides the phases
-// e^(i m beta)): the real harmonic factors of degrees >= J0, the accumulators (two per
-// output), and either the pair's rotated sums A (two per output: source coefficients
-// streamed, m2l_pair_rot) or the rotated source coefficients of degrees < P - J0 (two per
-// coefficient: outputs streamed, m2l_pair_rot_out).  The last pass streams its outputs once
-// the remaining degrees fit OUT values; the passes before it stream the source and add
-// degrees while they fit IN values.
-//   FP32: 12 warps per block (3 per SM sub-partition, whose 16 K registers then allow 168
-//         per thread); P = 10 takes the passes [0, 5) and [5, 10), at 168 registers each,
-//         the second with a small spill.
-//   FP64: 8 warps per block (255 registers per thread), the budgets in values about half
-//         of FP32's in registers; P = 10 takes four passes, none spilling.
+// Two kernels.  k_m2l_fold (FP32 without periodic images, and FP64 up to P = 8) folds the +mu and -mu terms of the
+// contraction (sph::m2l_fold: 1,505 instead of 2,420 multiply-adds and additions a pair at
+// P = 10) and takes a pair in one pass.  k_m2l_reg (FP64 above P = 8) runs passes over the
+// output degrees with the unfolded terms: there the folded form's harmonics, sums and columns
+// do not fit 255 registers, and its shared memory leaves the L1 too small for the rows that
+// its groups read again (P = 10, 11.7 M pairs: 5.1 ms against 5.9-6.8 ms folded).  FP32 solves
+// with images keep k_m2l_reg too, and with it every bit of their results (30,003 bodies, P = 8:
+// 0.12 ms in either).
+//
+// k_m2l_fold: warp per target cell, lane per source cell, in the source's azimuthal frame.
+// The real harmonic factors rho and the sums A of a group of output orders k stay in
+// registers; a pair's outputs are rotated back and added to the target's local expansion in
+// shared memory, which the warp sums over its lanes once per target: lanes l and l ^ 16
+// exchange two outputs and each adds one of them to its own column, so an output has 16
+// columns.  (Held in registers beside rho and A, the local expansion would force passes that
+// form the harmonics again; 32 columns would take the L1 that serves the rows.)  The orders
+// are taken in groups: as many as leave 2 values per sum, the harmonics and one column of
+// source coefficients within m2l_words registers.  A later group costs little: its orders
+// k >= K0 take the source degrees n < P - K0 only.
+// The multipoles are read from a copy by order (k_m2l_rows), 16 bytes a load: a load from 32
+// rows occupies the L1 nine cycles whatever its width.  Plummer N = 2^20, P = 10 (11.7 M
+// pairs, FP32) 2.31 -> 1.46 ms in one pass where two passes of k_m2l_reg ran before; 256 solves
+// at P = 8 8.5 -> 6.1 ms.  At P = 10 the FMA pipe is busy 44-47 % at 8 warps per SM; loads of the
+// rows (long scoreboard) are the largest stall.
+// Measured and not kept: rows staged in shared memory by one bulk copy per lane (1.59 ms
+// against 1.47 ms), 12 warps per SM at 168 registers (2.7 ms: more columns, less L1).
+template <typename T> __host__ __device__ constexpr int m2l_words() {
+  return sizeof(T) == 4 ? 180 : 216;
+}
+template <typename T> __host__ __device__ constexpr bool m2l_folds(int P) {
+  return sizeof(T) == 4 || P <= 8;
+}
+template <typename T> __host__ __device__ constexpr int m2l_group_end(int P, int K0) {
+  const int words = (int)sizeof(T) / 4;
+  int k = K0 + 1;
+  while (k < P && words * (2 * sph::fold_idx(P, K0, k + 1, k + 1) + sph::NT(P) + 2 * (P - K0)) <=
+                      m2l_words<T>())
+    k++;
+  return k;
+}
+// shared slots (two outputs each) of the groups from K0 on
+template <typename T> __host__ __device__ constexpr int m2l_slots(int P, int K0) {
+  int n = 0;
+  while (K0 < P) {
+    const int K1 = m2l_group_end<T>(P, K0);
+    n += (sph::fold_idx(P, K0, K1, K1) + 1) / 2;
+    K0 = K1;
+  }
+  return n;
+}
+template <typename T, int P> struct M2LCfg {
+  static constexpr int SLOTS = m2l_slots<T>(P, 0);
+  static constexpr int ROW = 32 * (int)sizeof(vec2<T>) * SLOTS;  // shared bytes of a warp
+  static constexpr int W = ROW * 4 <= 49152 ? 4 : ROW * 2 <= 49152 ? 2 : 1;
+  // registers a thread: the first group's values and about 45 for addresses and temporaries
+  static constexpr int NG = sph::fold_idx(P, 0, m2l_group_end<T>(P, 0), m2l_group_end<T>(P, 0));
+  static constexpr int EST = (int)sizeof(T) / 4 * (2 * NG + sph::NT(P) + 2 * P) + 45;
+  // warps per SM sub-partition at that many (16,384 registers each), and so blocks per SM
+  static constexpr int WARPS = EST > 172 ? 2 : EST > 128 ? 3 : 4;
+  static constexpr int BLOCKS = 4 * WARPS / W;
+};
+
+// output o of the group of orders from K0 on, in the order of fold_idx: its coefficient index
+__device__ __forceinline__ int m2l_output(int P, int K0, int o) {
+  int k = K0;
+  while (o >= P - k) o -= P - k++;
+  return sph::sidx(k + o, k);
+}
+
+// (er, ei) = w e^(i K0 beta), w = 1, or 0 for a lane without a source
+template <typename T, int P, int K0>
+__device__ __forceinline__ void m2l_groups(const T* rho, T cb, T sb, T er, T ei, const T* Mj,
+                                           vec2<T>* col, bool upper) {
+  if constexpr (K0 < P) {
+    constexpr int K1 = m2l_group_end<T>(P, K0), NO = sph::fold_idx(P, K0, K1, K1);
+    sph::Cx<T> A[NO];
+    if (K0 > 0) {  // source coefficients loaded and rotated again, not kept since the last group
+      sph::launder(Mj);
+      sph::launder(cb);
+      sph::launder(sb);
+    }
+    sph::m2l_fold<T, P, K0, K1>(rho, cb, sb, Mj, A);
+    // e^(-i k beta) (-1)^j A
+#pragma unroll
+    for (int k = K0; k < K1; k++) {
+#pragma unroll
+      for (int j = k; j < P; j++) {
+        sph::Cx<T>& o = A[sph::fold_idx(P, K0, k, j)];
+        const T cr = (j & 1) ? -er : er, ci = (j & 1) ? -ei : ei;
+        const T r = k == 0 ? cr * o.r : fma(cr, o.r, ci * o.i);
+        o.i = k == 0 ? cr * o.i : fma(cr, o.i, -ci * o.r);
+        o.r = r;
+      }
+      const T t = er * cb - ei * sb;
+      ei = er * sb + ei * cb;
+      er = t;
+    }
+#pragma unroll
+    for (int q = 0; q < (NO + 1) / 2; q++) {
+      sph::Cx<T> keep = A[2 * q];
+      if (2 * q + 1 < NO) {
+        const sph::Cx<T> other = A[2 * q + 1];
+        const T sr = upper ? keep.r : other.r, si = upper ? keep.i : other.i;
+        keep.r = upper ? other.r : keep.r;
+        keep.i = upper ? other.i : keep.i;
+        keep.r += __shfl_xor_sync(0xffffffffu, sr, 16);
+        keep.i += __shfl_xor_sync(0xffffffffu, si, 16);
+      }
+      vec2<T> l = col[32 * q];
+      l.x += keep.r;
+      l.y += keep.i;
+      col[32 * q] = l;
+    }
+    m2l_groups<T, P, K1>(rho, cb, sb, er, ei, Mj, col + 32 * ((NO + 1) / 2), upper);
+  }
+}
+
+// the groups' columns summed and added to the target's local expansion
+template <typename T, int P, int K0>
+__device__ __forceinline__ void m2l_finish(const vec2<T>* slots, int lane, T* Lc) {
+  if constexpr (K0 < P) {
+    constexpr int K1 = m2l_group_end<T>(P, K0), NO = sph::fold_idx(P, K0, K1, K1);
+    // two lanes per slot, each summing 16 columns from a column of its own on
+#pragma unroll
+    for (int o0 = 0; o0 < NO; o0 += 32) {
+      const int o = o0 + lane, slot = min(o >> 1, (NO - 1) / 2);
+      const vec2<T>* row = slots + 32 * slot + 16 * (o & 1);
+      T r[2] = {0, 0}, i[2] = {0, 0};
+#pragma unroll
+      for (int u = 0; u < 16; u++) {
+        const vec2<T> v = row[((lane >> 1) + u) & 15];
+        r[u & 1] += v.x;
+        i[u & 1] += v.y;
+      }
+      T sr = r[0] + r[1], si = i[0] + i[1];
+      if (NO & 1) {  // the last output of an odd group has all 32 columns of its slot
+        const T xr = __shfl_xor_sync(0xffffffffu, sr, 1), xi = __shfl_xor_sync(0xffffffffu, si, 1);
+        if (o == NO - 1) {
+          sr += xr;
+          si += xi;
+        }
+      }
+      if (o < NO) {
+        const int t = m2l_output(P, K0, o);
+        Lc[2 * t] += sr;
+        Lc[2 * t + 1] += si;
+      }
+    }
+    m2l_finish<T, P, K1>(slots + 32 * ((NO + 1) / 2), lane, Lc);
+  }
+}
+
+// the cells' multipoles by order (sph::col_idx), for k_m2l_fold
+template <typename T, int P>
+__global__ void __launch_bounds__(128)
+    k_m2l_rows(int ncells, const T* __restrict__ M, int ncoef, T* __restrict__ rows) {
+  constexpr int LEN = sph::col_len(P) / 2;
+  const long long g = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const int c = (int)(g / LEN), e = (int)(g % LEN);
+  if (c >= ncells) return;
+  int mu = 0, o = e;
+  while (o >= (P - mu + 1) / 2 * 2) o -= (P - mu++ + 1) / 2 * 2;
+  vec2<T> v;
+  v.x = v.y = 0;
+  if (mu + o < P)
+    v = reinterpret_cast<const vec2<T>*>(M + (size_t)c * ncoef)[sph::sidx(mu + o, mu)];
+  reinterpret_cast<vec2<T>*>(rows)[(size_t)c * LEN + e] = v;
+}
+
+template <typename T, int P>
+__global__ void __launch_bounds__(32 * M2LCfg<T, P>::W, M2LCfg<T, P>::BLOCKS)
+    k_m2l_fold(int ntgt, const int* __restrict__ tgt, const int* __restrict__ off,
+          const unsigned long long* __restrict__ pairs, const vec4<T>* __restrict__ cX,
+          const T* __restrict__ rows, T* __restrict__ L, int ncoef, T cycle) {
+  constexpr int NT = sph::NT(P), W = M2LCfg<T, P>::W, SLOTS = M2LCfg<T, P>::SLOTS;
+  __shared__ vec2<T> cols[W][32 * SLOTS];
+  const int lane = lane_id(), wl = threadIdx.x >> 5;
+  const int w = blockIdx.x * W + wl;
+  if (w >= ntgt) return;
+  const int c = tgt[w];
+  const int s0 = off[c], s1 = off[c + 1];
+  const vec4<T> Xi = cX[c];
+  vec2<T>* col = cols[wl] + lane;
+#pragma unroll
+  for (int t = 0; t < SLOTS; t++) col[32 * t].x = col[32 * t].y = 0;
+  for (int sb = s0; sb < s1; sb += 32) {
+    const bool act = sb + lane < s1;  // a lane past the end repeats the last source, weight 0
+    const unsigned src = (unsigned)pairs[act ? sb + lane : s1 - 1];
+    const int j = pair_cell(src);
+    T px, py, pz;  // periodic shift of the source (0 without images)
+    img_shift<T>(pair_img(src), cycle, px, py, pz);
+    const vec4<T> Xj = cX[j];
+    T rho[NT], invr;
+    const sph::Angles<T> a =
+        sph::angles_rs(Xi.x - Xj.x - px, Xi.y - Xj.y - py, Xi.z - Xj.z - pz, invr);
+    sph::fold_rho<T, P>(a, invr, rho);
+    m2l_groups<T, P, 0>(rho, a.cb, a.sb, act ? T(1) : T(0), T(0),
+                        rows + (size_t)j * sph::col_len(P), col, lane >= 16);
+  }
+  __syncwarp();
+  m2l_finish<T, P, 0>(cols[wl], lane, L + (size_t)c * ncoef);
+}
+
+// k_m2l_reg: warp per target, lane per source cell, harmonics and local expansion in
+// registers, one warp reduction per target cell at the end.  Each pair is contracted in the
+// source's azimuthal frame (real harmonic factors, half the multiply-adds of the complex
+// form).  The outputs are split into passes over their degree (separate launches) so that
+// each pass's registers stay within its block's share: registers of a pass [J0, J1) (besides
+// the phases e^(i m beta)) are the real harmonic factors of degrees >= J0, the accumulators
+// (two per output), and either the pair's rotated sums A (two per output: source
+// coefficients streamed, m2l_pair_rot) or the rotated source coefficients of degrees < P - J0
+// (two per coefficient: outputs streamed, m2l_pair_rot_out).  The last pass streams its
+// outputs once the remaining degrees fit OUT values; the passes before it stream the source
+// and add degrees while they fit IN values.  FP64: 8 warps per block (255 registers per
+// thread), four passes at P = 10, none spilling; FP32: 12 warps at 168 registers, two passes.
 template <typename T> struct M2LBudget {
   static constexpr int W = sizeof(T) == 4 ? 12 : 8;
   static constexpr int IN = sizeof(T) == 4 ? 139 : 100;
@@ -447,7 +646,26 @@ template <typename T, int P> static void m2m_(Solver<T>& s, int lo, int hi) {
       (T)s.cfg.theta, s.write_r);
   FMM_LAUNCH_CHECK();
 }
-template <typename T, int P> static void m2l_(Solver<T>& s) { launch_m2l_passes<T, P, 0>(s); }
+template <typename T, int P> static void m2l_(Solver<T>& s) {
+  if (!s.m2l_ntgt) return;
+  if (sizeof(T) == 4 && s.cfg.images > 0) {
+    launch_m2l_passes<T, P, 0>(s);
+    return;
+  }
+  if constexpr (m2l_folds<T>(P)) {
+    constexpr int W = M2LCfg<T, P>::W, LEN = sph::col_len(P) / 2;
+    s.m2l_rows.ensure((size_t)s.ncells * 2 * LEN);
+    k_m2l_rows<T, P><<<ceil_div((long long)s.ncells * LEN, 128), 128, 0, s.stream>>>(
+        s.ncells, s.M.p, s.ncoef, s.m2l_rows.p);
+    FMM_LAUNCH_CHECK();
+    k_m2l_fold<T, P><<<ceil_div(s.m2l_ntgt, W), 32 * W, 0, s.stream>>>(
+        s.m2l_ntgt, s.m2l_tgt.p, s.m2l_off.p, s.m2l.p, s.cX.p, s.m2l_rows.p, s.L.p, s.ncoef,
+        (T)s.cfg.cycle);
+    FMM_LAUNCH_CHECK();
+  } else {
+    launch_m2l_passes<T, P, 0>(s);
+  }
+}
 template <typename T, int P> static void l2l_(Solver<T>& s, int lo, int hi) {
   constexpr int NTH = tr_threads<T>();
   k_l2l_reg<T, P><<<ceil_div(hi - lo, NTH), NTH, 0, s.stream>>>(lo, hi, s.npos.p, s.c_iparent.p,
