@@ -142,10 +142,6 @@ template <typename T> void stage_trav(Solver<T>& s) {
   phase_begin(s, FMM_PHASE_P2P);
   s.trg_s.ensure(std::max(s.n, 1));
   s.trg_e.ensure(std::max(s.n, 1));
-  if (s.n > 0) {
-    FMM_CUDA(cudaMemsetAsync(s.trg_s.p, 0, sizeof(vec4<T>) * s.n, s.stream));
-    FMM_CUDA(cudaMemsetAsync(s.trg_e.p, 0, sizeof(vec4<T>) * s.n, s.stream));
-  }
   run_p2p(s);
   phase_end(s, FMM_PHASE_P2P);
   s.stage = ST_TRAV;
@@ -228,10 +224,6 @@ template <typename T> void solve_all(Solver<T>& s) {
   phase_begin(s, FMM_PHASE_P2P);
   s.trg_s.ensure(std::max(s.n, 1));
   s.trg_e.ensure(std::max(s.n, 1));
-  if (s.n > 0) {
-    FMM_CUDA(cudaMemsetAsync(s.trg_s.p, 0, sizeof(vec4<T>) * s.n, s.stream));
-    FMM_CUDA(cudaMemsetAsync(s.trg_e.p, 0, sizeof(vec4<T>) * s.n, s.stream));
-  }
   finish_p2p_list(s);  // grouped on the side stream while M2L ran
   run_p2p(s);
   phase_end(s, FMM_PHASE_P2P);
@@ -476,11 +468,13 @@ int fmm_b200_create(const fmm_b200_config* cfg, fmm_b200_solver** out) {
                          &s_.c_level,  &s_.order,    &s_.m2l_off,  &s_.p2p_off, &s_.seg_cnt, \
                          &s_.d_lvl,    &s_.seg_cnt2, &s_.body_leaf, &s_.d_seg,  &s_.d_root_first, \
                          &s_.d_root_count, &s_.nsid, &s_.c_root,   &s_.cbase,   &s_.fs_pos, \
-                         &s_.fs_pos2,  &s_.fs_idx,   &s_.m2l_tgt,  &s_.k_list,  &s_.k_saved_leaves}; \
+                         &s_.fs_pos2,  &s_.fs_idx,   &s_.m2l_tgt,  &s_.k_list,  &s_.k_saved_leaves, \
+                         &s_.p2p_bucket, &s_.p2p_hist, &s_.p2p_nsrc, &s_.p2p_work}; \
     for (auto* a : ia) a->OP();                                                            \
     s_.keys.OP(); s_.keys2.OP(); s_.c_icell.OP(); s_.m2l.OP(); s_.fs_keys.OP();            \
     s_.c_info.OP(); s_.fs_root.OP(); s_.fs_root2.OP();                                     \
-    s_.p2p.OP(); s_.list_tmp.OP(); s_.p2p_pairs_count.OP();                                \
+    s_.p2p.OP(); s_.list_tmp.OP(); s_.p2p_pairs_count.OP(); s_.p2p_order.OP();             \
+    s_.p2p_srcs.OP();                                                                      \
     s_.cub_tmp.OP(); s_.front.OP(); s_.front2.OP();                                        \
     s_.seg_keys2.OP(); s_.cub_tmp2.OP(); s_.dtmp.OP();                                     \
     if ((h)->precision == FMM_FP64) {                                                      \

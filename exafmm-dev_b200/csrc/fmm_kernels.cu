@@ -430,6 +430,9 @@ void op_p2p(Solver<T>& s, int n, const int* ci, const int* cj, const int* image,
   };
   try {
     s.np2p = (long long)L.pairs.size();
+    order_p2p_targets(s);
+    s.p2p_ordered = false;                        // (an order of these targets only)
+    FMM_CUDA(cudaStreamSynchronize(s.stream));  // its team counts
     run_p2p(s);
   } catch (...) {
     restore();
@@ -502,6 +505,7 @@ int fmm_b200_kernel_set_cells(fmm_b200_solver* h, int nc, const double* X, const
     s.kc_iparent.assign(iparent, iparent + nc);
     s.kc_valid = true;
     s.ncells = nc;
+    fill_cell_info(s);
     s.maxlevel = 0;
     s.nleaves = 0;
     s.nroots = 0;

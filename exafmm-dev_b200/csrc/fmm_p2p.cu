@@ -1,26 +1,46 @@
 // Near-field P2P over the per-target-leaf source lists (kernel::P2P,
 // kernels/LaplaceP2PCPU.cxx:4-170 and the self form :172-331).
 //
-// One warp owns one target leaf.  Its lanes split into groups of G (1, 2 or 4) so that a
-// small leaf still keeps the warp busy: each group holds one target body and its G lanes
-// take every G-th source; a leaf of 33..64 bodies gives each lane two targets that share
-// every staged source.  Sources stream through shared memory 32 bodies at a time (one
-// coalesced load per lane), a chunk of 32 running on across source leaves; in FP32 the
-// staged sources are taken two at a time with the packed two-wide instructions of sm_100
-// (half the issue slots of the scalar pair arithmetic).  The inner loop is FMA + one rsqrt
-// per pair (no r^2 == 0 test away from the target leaf itself).  FP32 folds each chunk's
-// plain partial sum into a compensated (TwoSum) accumulator, so the accumulation error does
-// not grow with the length of the list; FP64 sums plainly.  Pairs with r^2 == 0 are
-// skipped, as the reference does (:149); the result is per unit target charge (the
-// reference multiplies by q_i in P2P and divides again in L2P / normalize).
+// A team of 1, 2, 4 or 8 warps of one block owns a target leaf and shares out the bodies of
+// its source list evenly; the warps' sums meet in shared memory in warp order.  The size of
+// the team follows from the leaf's own list (p2p_class), so a leaf's result does not depend
+// on what else the launch holds.  (One warp per leaf left a launch of a few thousand leaves
+// with a long tail: 1.4 waves of warps at 4,096 leaves, and 512 leaves a third of the GPU:
+// cube of 16,384 bodies in FP64 0.43 ms, now 0.12 ms.)
+//
+// A warp's lanes hold up to TPL = 3 targets each (FP64: 2), spread over G = 1 .. 8 lanes that
+// take every G-th source (p2p_lanes).  Sources stream through shared memory 32 bodies at a
+// time, a chunk running on across source leaves; FP32 takes them two at a time with the
+// packed two-wide instructions of sm_100, 13 packed instructions and two MUFU rsqrt for two
+// pairs.  Every lane reads every staged source, 16 bytes a source, and the shared-memory
+// pipe returns 128 bytes a cycle and SM: at one target per lane that return path would bound
+// the kernel, not the FMA pipe (4 cycles a source and warp against 3.25), so a source has to
+// serve several targets of its lane.  FP32 folds the sums of 32 of a lane's sources into a
+// compensated (TwoSum) accumulator, so the accumulation error does not grow with the length
+// of the list; FP64 sums plainly.
+//
+// Bound: the FMA pipe (FP64: the FP64 pipe), 26 cycles a source pair and target, at 50-65 %
+// of it: the rest is idle target slots, the chunks' staging and latency at 16 warps per SM.
+// FP32, one warp per leaf and one to two targets per lane before: Plummer 2^20, P = 10
+// (0.99 G pairs, 18 bodies a leaf) 1.08 -> 0.91 ms; 256 solves (14.4 G pairs) 14.4 -> 12.0 ms;
+// cube of 200,003 (1.28 G, 49 a leaf) 1.19 -> 0.89 ms; sphere of 2^22 (1.23 G, 13 a leaf) 1.98
+// -> 1.82 ms.  Measured beside it on the 256 solves: four targets per lane 13.8 ms against
+// 13.6 (128 registers either way), two at 24 warps per SM 14.4 ms; accumulators in registers
+// 15.6 ms; chunks of 64 bodies 14.1 ms; teams twice as large 12.9 ms.
+//
+// Away from the target leaf itself the pairs take no r^2 == 0 test and an FTZ rsqrt.  If a
+// warp's potential then is not finite (two bodies of different leaves in one place, or
+// closer than the normal range), it sums its part of the list again with the exact form
+// throughout.  Pairs with r^2 == 0 are skipped, as the reference does (:149); the result is
+// per unit target charge (the reference multiplies by q_i in P2P and divides again in L2P /
+// normalize).
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "fmm_solver.cuh"
 
 namespace fmmb200 {
-
-constexpr int kP2PWarps = 4;
 
 // 1/sqrt with subnormal inputs flushed to zero (PTX rsqrt.approx.ftz.f32): no handling of
 // subnormal inputs and no r^2 == 0 test, for the source leaves where neither can occur
@@ -31,57 +51,95 @@ __device__ __forceinline__ float rsqrt_ftz(float a) {
 }
 __device__ __forceinline__ double rsqrt_ftz(double a) { return rsqrt(a); }
 
-// one pair; EXACT: skip r^2 == 0 and take subnormal r^2 as it is (the reference's
-// arithmetic); otherwise an r^2 of zero or below the normal range makes `pot` non-finite
-// SHIFT: the source is a periodic image shifted by (px, py, pz); the offset is formed as
-// (xj - xi) + p, the negation of the reference's (xi - xj) - Xperiodic
-template <typename T, bool EXACT = true, bool SHIFT = false>
-__device__ __forceinline__ void p2p_accum(const vec4<T>& sj, const vec4<T>& xi, T eps2, T& pot,
-                                          T& ax, T& ay, T& az, T px = 0, T py = 0, T pz = 0) {
-  T dx = sj.x - xi.x, dy = sj.y - xi.y, dz = sj.z - xi.z;
-  if (SHIFT) {
-    dx += px;
-    dy += py;
-    dz += pz;
-  }
-  const T r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
-  const T inv = EXACT ? (r2 > T(0) ? rsqrt_(r2) : T(0)) : rsqrt_ftz(r2);
-  const T qinv = sj.w * inv;
-  const T inv3 = qinv * inv * inv;
-  pot += qinv;
-  ax = fma(dx, inv3, ax);
-  ay = fma(dy, inv3, ay);
-  az = fma(dz, inv3, az);
+// Most targets of a lane, and the lanes G that share one: 32 TPL / G slots for the leaf's
+// targets (64 at a time).  FP32 at the default limits g4 = 8, g2 = 16: G = 8 up to 12 bodies, 4
+// up to 24, 2 up to 48, so slots come in steps of 4, 8 and 16 and few stay idle; FP64, whose
+// arithmetic and not its reads bounds it, takes G = 4, 2, 1 (fewer sums to merge).  So do solves
+// with periodic images, whose sums are also folded after every chunk by one warp per leaf: in
+// that order their results keep every bit they had (30,003 bodies: 0.05 ms either way).
+template <typename T> __host__ __device__ constexpr int p2p_tpl() { return sizeof(T) == 4 ? 3 : 2; }
+template <typename T> __device__ __forceinline__ int p2p_lanes(int nb, int g4, int g2, int images) {
+  if (sizeof(T) == 8 || images) return nb <= g4 ? 4 : nb <= g2 ? 2 : 1;
+  constexpr int X = p2p_tpl<T>();
+  return nb <= X * g4 / 2 ? 8 : nb <= X * g2 / 2 ? 4 : nb <= 16 * X ? 2 : 1;
 }
 
-// FP32 rows: the staged sources are taken two at a time with the packed two-wide
-// instructions of sm_100 (add.f32x2, mul.f32x2, fma.f32x2: one instruction for both, each
-// component rounded as the scalar operation, so each pair's terms are those of p2p_accum).
-// A warp's row holds A[i] = (x, x', y, y') and B[i] = (z, z', q, q') for the sources 2i and
-// 2i + 1 (A in float4 0..15, B in 16..31); a missing partner is a far-away zero charge,
-// which adds exactly zero.
+constexpr int kP2PWindow = 512;  // source bodies whose indices a warp lists ahead
 
-// the pairs of one staged row (np source pairs) on the lane's TPL targets, added to the
-// two-wide sums; nx, ny, nz are the negated target coordinates in both halves
+// two staged sources of a row: FP32 (x, x', y, y') and (z, z', q, q'); FP64 one source, (x, y)
+// and (z, q)
+template <typename T> struct Row;
+template <> struct Row<float> {
+  float4 a[16], b[16];
+  int idx[kP2PWindow];
+  __device__ __forceinline__ void put(int i, const float4& v) {
+    float* p = reinterpret_cast<float*>(&a[i >> 1]) + (i & 1);
+    float* q = reinterpret_cast<float*>(&b[i >> 1]) + (i & 1);
+    p[0] = v.x;
+    p[2] = v.y;
+    q[0] = v.z;
+    q[2] = v.w;
+  }
+};
+template <> struct Row<double> {
+  double2 a[32], b[32];
+  int idx[kP2PWindow];
+  __device__ __forceinline__ void put(int i, const double4& v) {
+    a[i] = make_double2(v.x, v.y);
+    b[i] = make_double2(v.z, v.w);
+  }
+};
+
+// A target and its sums over some sources.  FP32: the coordinates negated, in both halves;
+// the halves of a sum take the even and the odd sources.
+template <typename T> struct Target;
+template <> struct Target<float> {
+  float2 nx, ny, nz, p, x, y, z;
+  __device__ __forceinline__ void set(const float4& v) {
+    nx = make_float2(-v.x, -v.x);
+    ny = make_float2(-v.y, -v.y);
+    nz = make_float2(-v.z, -v.z);
+  }
+  __device__ __forceinline__ void zero() { p = x = y = z = make_float2(0.f, 0.f); }
+  __device__ __forceinline__ void sums(float* v) const {
+    v[0] = p.x + p.y;
+    v[1] = x.x + x.y;
+    v[2] = y.x + y.y;
+    v[3] = z.x + z.y;
+  }
+};
+template <> struct Target<double> {
+  double nx, ny, nz, p, x, y, z;
+  __device__ __forceinline__ void set(const double4& v) { nx = -v.x, ny = -v.y, nz = -v.z; }
+  __device__ __forceinline__ void zero() { p = x = y = z = 0; }
+  __device__ __forceinline__ void sums(double* v) const { v[0] = p, v[1] = x, v[2] = y, v[3] = z; }
+};
+
+// The first `cnt` sources of a staged row (the rest of it charges nothing) on the lane's TPL
+// targets, every G-th entry from `sub` on.
+// EXACT: skip r^2 == 0 and take subnormal r^2 as it is (the reference's arithmetic);
+// otherwise an r^2 of zero or below the normal range makes the potential non-finite.
+// SHIFT: the source is a periodic image shifted by (px, py, pz); the offset is formed as
+// (xj - xi) + p, the negation of the reference's (xi - xj) - Xperiodic
 template <int TPL, bool EXACT, bool SHIFT>
-__device__ __forceinline__ void row_pairs(const float4* row, int sub, int G, int np,
-                                          const float2* nx, const float2* ny, const float2* nz,
-                                          float2 e2, float2 p2x, float2 p2y, float2 p2z,
-                                          float2* sp, float2* sx, float2* sy, float2* sz) {
-  const float4* A = row;
-  const float4* B = row + 16;
-#pragma unroll (4 / TPL)
-  for (int i = sub; i < np; i += G) {
-    const float4 a = A[i], c = B[i];
+__device__ __forceinline__ void p2p_row(const Row<float>& row, int sub, int G, int cnt, float eps2,
+                                        const float* shift, Target<float>* t) {
+  const int np = (cnt + 1) >> 1;
+  const float2 e2 = make_float2(eps2, eps2);
+  constexpr int UNROLL = TPL <= 2 ? 2 : 1;
+#pragma unroll UNROLL
+  for (int i = 0; i < np; i += G) {
+    const float4 a = row.a[i + sub], c = row.b[i + sub];
     const float2 x2 = make_float2(a.x, a.y), y2 = make_float2(a.z, a.w);
     const float2 z2 = make_float2(c.x, c.y), q2 = make_float2(c.z, c.w);
 #pragma unroll
     for (int u = 0; u < TPL; u++) {
-      float2 dx = __fadd2_rn(x2, nx[u]), dy = __fadd2_rn(y2, ny[u]), dz = __fadd2_rn(z2, nz[u]);
+      float2 dx = __fadd2_rn(x2, t[u].nx), dy = __fadd2_rn(y2, t[u].ny),
+             dz = __fadd2_rn(z2, t[u].nz);
       if (SHIFT) {
-        dx = __fadd2_rn(dx, p2x);
-        dy = __fadd2_rn(dy, p2y);
-        dz = __fadd2_rn(dz, p2z);
+        dx = __fadd2_rn(dx, make_float2(shift[0], shift[0]));
+        dy = __fadd2_rn(dy, make_float2(shift[1], shift[1]));
+        dz = __fadd2_rn(dz, make_float2(shift[2], shift[2]));
       }
       const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
       float2 inv;
@@ -89,279 +147,450 @@ __device__ __forceinline__ void row_pairs(const float4* row, int sub, int G, int
       inv.y = EXACT ? (r2.y > 0.f ? rsqrt_(r2.y) : 0.f) : rsqrt_ftz(r2.y);
       const float2 qinv = __fmul2_rn(q2, inv);
       const float2 inv3 = __fmul2_rn(__fmul2_rn(qinv, inv), inv);
-      sp[u] = __fadd2_rn(sp[u], qinv);
-      sx[u] = __ffma2_rn(dx, inv3, sx[u]);
-      sy[u] = __ffma2_rn(dy, inv3, sy[u]);
-      sz[u] = __ffma2_rn(dz, inv3, sz[u]);
+      t[u].p = __fadd2_rn(t[u].p, qinv);
+      t[u].x = __ffma2_rn(dx, inv3, t[u].x);
+      t[u].y = __ffma2_rn(dy, inv3, t[u].y);
+      t[u].z = __ffma2_rn(dz, inv3, t[u].z);
+    }
+  }
+}
+template <int TPL, bool EXACT, bool SHIFT>
+__device__ __forceinline__ void p2p_row(const Row<double>& row, int sub, int G, int cnt,
+                                        double eps2, const double* shift, Target<double>* t) {
+#pragma unroll(4 / TPL)
+  for (int i = 0; i < cnt; i += G) {
+    const double2 a = row.a[i + sub], c = row.b[i + sub];
+#pragma unroll
+    for (int u = 0; u < TPL; u++) {
+      double dx = a.x + t[u].nx, dy = a.y + t[u].ny, dz = c.x + t[u].nz;
+      if (SHIFT) {
+        dx += shift[0];
+        dy += shift[1];
+        dz += shift[2];
+      }
+      const double r2 = fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2)));
+      const double inv = EXACT ? (r2 > 0 ? rsqrt_(r2) : 0) : rsqrt_ftz(r2);
+      const double qinv = c.y * inv;
+      const double inv3 = qinv * inv * inv;
+      t[u].p += qinv;
+      t[u].x = fma(dx, inv3, t[u].x);
+      t[u].y = fma(dy, inv3, t[u].y);
+      t[u].z = fma(dz, inv3, t[u].z);
     }
   }
 }
 
-// FP64 rows: one source per entry (x, y, z, q); the pairs of a staged row (cnt sources) on
-// the lane's TPL targets, added to the plain sums
-template <int TPL, bool EXACT, bool SHIFT>
-__device__ __forceinline__ void row_pairs(const vec4<double>* row, int sub, int G, int cnt,
-                                          const vec4<double>* xi, double eps2, double px,
-                                          double py, double pz, double* sp, double* sx,
-                                          double* sy, double* sz) {
-#pragma unroll (4 / TPL)
-  for (int k = sub; k < cnt; k += G) {
-    const vec4<double> sj = row[k];
-#pragma unroll
-    for (int u = 0; u < TPL; u++)
-      p2p_accum<double, EXACT, SHIFT>(sj, xi[u], eps2, sp[u], sx[u], sy[u], sz[u], px, py, pz);
-  }
-}
+// A lane's accumulators in shared memory: potential and gradient of target u in s[u][lane],
+// in FP32 the sums' rounding errors in e[u][lane] (in registers they would cost 8 per target
+// and spill).
+template <typename T, bool COMP> struct Accum {
+  vec4<T> s[p2p_tpl<T>()][32], e[COMP ? p2p_tpl<T>() : 1][COMP ? 32 : 1];
+};
 
-// Target leaf, either precision: the bodies of its source leaves, taken in list order, are
-// staged 32 at a time whatever the leaves' sizes (a chunk runs on into the next source leaf,
-// and ends early only where the periodic image changes or after 32 source leaves), so that
-// the rows are full and the per-chunk work (staging, the finite test, the compensated fold)
-// is shared by all of its source leaves.  The source leaves' descriptors (first body,
-// count, image) are read 32 at a time, one per lane; a lane finds the leaf of its chunk
-// position by a scan of the counts and a binary search over the lanes.  A chunk that holds
-// bodies of the target leaf itself is summed in the exact form; any other chunk in the fast
-// form, and again in the exact form (from the same row) if a sum is not finite, so the
-// results are those of the exact form throughout.  FP32 takes the staged sources two at a
-// time with the packed f32x2 instructions; FP64 one at a time.
+// the targets' sums into their accumulators, and zero again
 template <typename T, bool COMP, int TPL>
-__device__ __forceinline__ void p2p_leaf_chunked(int lane, void* rowmem, int b0, int nb,
-                                                 int base, int G, int s0, int s1,
-                                                 const unsigned long long* __restrict__ pairs,
-                                                 const int* __restrict__ ibody,
-                                                 const int* __restrict__ nbody,
-                                                 const vec4<T>* __restrict__ bodies, T eps2,
-                                                 T cycle, vec4<T>* __restrict__ trg_s,
-                                                 vec4<T>* __restrict__ trg_e) {
-  constexpr bool F32 = sizeof(T) == 4;
-  // per-lane pair sums: float2 (two halves of the packed form) or T
-  using Acc = typename std::conditional<F32, float2, T>::type;
-  const unsigned full = 0xffffffffu;
-  const int tpp = 32 / G;
-  const int sub = lane % G;
-  int ti[TPL];
-  bool act[TPL];
-  vec4<T> xi[TPL];
-  float2 nx[TPL], ny[TPL], nz[TPL];  // FP32: negated target coordinates in both halves
-  Comp<T> acc[TPL][4];
+__device__ __forceinline__ void p2p_fold(Target<T>* t, Accum<T, COMP>& acc, int lane) {
 #pragma unroll
   for (int u = 0; u < TPL; u++) {
-    ti[u] = base + u * tpp + lane / G;
-    act[u] = ti[u] < nb;
-    xi[u] = act[u] ? bodies[b0 + ti[u]] : make_v4<T>(0, 0, 0, 0);
-    if constexpr (F32) {
-      nx[u] = make_float2(-xi[u].x, -xi[u].x);
-      ny[u] = make_float2(-xi[u].y, -xi[u].y);
-      nz[u] = make_float2(-xi[u].z, -xi[u].z);
-    }
+    T v[4];
+    t[u].sums(v);
+    vec4<T> s = acc.s[u][lane];
+    if constexpr (COMP) {
+      vec4<T> e = acc.e[u][lane];
+      Comp<T> a[4] = {{s.x, e.x}, {s.y, e.y}, {s.z, e.z}, {s.w, e.w}};
 #pragma unroll
-    for (int d = 0; d < 4; d++) acc[u][d] = Comp<T>{0, 0};
+      for (int d = 0; d < 4; d++) comp_add(a[d], v[d]);
+      acc.s[u][lane] = make_v4<T>(a[0].s, a[1].s, a[2].s, a[3].s);
+      acc.e[u][lane] = make_v4<T>(a[0].e, a[1].e, a[2].e, a[3].e);
+    } else {
+      acc.s[u][lane] = make_v4<T>(s.x + v[0], s.y + v[1], s.z + v[2], s.w + v[3]);
+    }
+    t[u].zero();
   }
-  const float2 e2 = make_float2((float)eps2, (float)eps2);
-  for (int sb = s0; sb < s1; sb += 32) {
-    // lane k: source leaf sb + k (image -1 past the end of the list)
+}
+
+// A source leaf as k_p2p reads it: first body in bits 0-30, image in 31-35, bodies above.
+__device__ __forceinline__ unsigned long long p2p_leaf(int4 info, int img) {
+  return (unsigned long long)(unsigned)info.w | (unsigned long long)img << 31 |
+         (unsigned long long)(unsigned)info.z << 36;
+}
+
+// Positions [p0, p1) of the target leaf's source bodies (the bodies of its source leaves in
+// list order) on the targets of one warp.  Source leaves' descriptors (first body, count,
+// image) are read 32 at a time, one per lane, and scanned; each lane then writes the indices
+// of its leaf's bodies into the warp's window in shared memory, from which the chunks are
+// loaded, the next one while the staged one is summed.
+template <typename T, bool COMP, int TPL>
+__device__ __forceinline__ void p2p_segment(int lane, Row<T>& row, int b0, int nb, int sub, int G,
+                                            int s0, int s1, int p0, int p1, bool whole, int folds,
+                                            const unsigned long long* __restrict__ srcs,
+                                            const vec4<T>* __restrict__ bodies, T eps2, T cycle,
+                                            bool exact, Target<T>* t, Accum<T, COMP>& acc) {
+  const unsigned full = 0xffffffffu;
+  int pending = 0;  // chunks since the last fold
+  int cum = 0;
+  for (int sb = s0; sb < s1 && cum < p1; sb += 32) {
+    // lane k: source leaf sb + k
     int dj0 = 0, dnj = 0, dimg = -1;
     if (sb + lane < s1) {
-      const unsigned src = (unsigned)pairs[sb + lane];
-      dj0 = ibody[pair_cell(src)];
-      dnj = nbody[pair_cell(src)];
-      dimg = pair_img(src);
+      const unsigned long long d = srcs[sb + lane];
+      dj0 = (int)(d & 0x7fffffffu);
+      dimg = (int)(d >> 31) & 31;
+      dnj = (int)(d >> 36);
     }
-    int k = 0, o = 0;  // the chunk starts at body o of leaf k
-    while (k < 32) {
-      const int img = __shfl_sync(full, dimg, k);
+    // the leaves of one image at a time: lanes k0 .. cut - 1
+    for (int k0 = 0; k0 < 32;) {
+      const int img = __shfl_sync(full, dimg, k0);
       if (img < 0) break;
-      const unsigned other = ~__ballot_sync(full, dimg == img) & (full << k);
-      const int cut = other ? __ffs(other) - 1 : 32;  // leaves k .. cut - 1 share the image
-      const int avail = lane >= k && lane < cut ? dnj - (lane == k ? o : 0) : 0;
-      int incl = avail;
+      const unsigned other = __ballot_sync(full, dimg != img) & (full << k0);
+      const int cut = other ? __ffs(other) - 1 : 32;
+      const int cnj = lane >= k0 && lane < cut ? dnj : 0;
+      int incl = cnj;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
         const int v = __shfl_up_sync(full, incl, d);
         if (lane >= d) incl += v;
       }
-      const int total = __shfl_sync(full, incl, 31);
-      const int cnt = min(32, total);
-      // f: the leaf of chunk position `lane`.  Each leaf of the chunk sets the bit of its
-      // first position; f is k plus the number of bits at or below `lane`, less one (with
-      // an empty leaf in the range, whose start would coincide with the next one's: the
-      // number of leaves whose counts end at or before `lane`, by binary search)
-      int f;
-      if (!__any_sync(full, lane >= k && lane < cut && avail == 0)) {
-        const unsigned starts =
-            __reduce_or_sync(full, avail > 0 && incl - avail < 32 ? 1u << (incl - avail) : 0u);
-        f = k + __popc(starts & (full >> (31 - lane))) - 1;
-      } else {
-        f = 0;
-#pragma unroll
-        for (int step = 16; step >= 1; step >>= 1)
-          if (__shfl_sync(full, incl, f + step - 1) <= lane) f += step;
-      }
-      const int ex = __shfl_sync(full, incl - avail, f);
-      const int jf = __shfl_sync(full, dj0 + (lane == k ? o : 0), f);
-      const int bj = jf + lane - ex;
-      const vec4<T> b = lane < cnt ? bodies[bj] : make_v4<T>(T(1e30), T(1e30), T(1e30), T(0));
-      const bool self = __any_sync(full, lane < cnt && img == 0 && bj >= b0 && bj < b0 + nb);
-      T px = 0, py = 0, pz = 0;
-      if (img != 0) img_shift<T>(img, cycle, px, py, pz);
-      Acc sp[TPL], sx[TPL], sy[TPL], sz[TPL];
-      auto zero = [&]() {
-#pragma unroll
-        for (int u = 0; u < TPL; u++) {
-          if constexpr (F32) sp[u] = sx[u] = sy[u] = sz[u] = make_float2(0.f, 0.f);
-          else sp[u] = sx[u] = sy[u] = sz[u] = T(0);
-        }
-      };
-      auto finite = [&]() {
-        bool bad = false;
-#pragma unroll
-        for (int u = 0; u < TPL; u++) {
-          if constexpr (F32) bad |= act[u] && !isfinite(sp[u].x + sp[u].y);
-          else bad |= act[u] && !isfinite(sp[u]);
-        }
-        return !__any_sync(full, bad);
-      };
-      __syncwarp();
-      if constexpr (F32) {
-        // A[i] = (x, x', y, y'), B[i] = (z, z', q, q') for the sources 2i and 2i + 1
-        float4* A = static_cast<float4*>(rowmem);
-        float4* B = A + 16;
-        float* a = reinterpret_cast<float*>(&A[lane >> 1]);
-        float* c = reinterpret_cast<float*>(&B[lane >> 1]);
-        const int h = lane & 1;
-        a[h] = b.x;
-        a[2 + h] = b.y;
-        c[h] = b.z;
-        c[2 + h] = b.w;
-      } else {
-        static_cast<vec4<T>*>(rowmem)[lane] = b;
-      }
-      __syncwarp();
-      // evaluate the row in the fast or the exact pair form (with or without the shift)
-      auto pairs_of = [&](auto exact, auto shift) {
-        constexpr bool EX = decltype(exact)::value, SH = decltype(shift)::value;
-        if constexpr (F32) {
-          const float2 p2x = make_float2(px, px), p2y = make_float2(py, py),
-                       p2z = make_float2(pz, pz);
-          row_pairs<TPL, EX, SH>(static_cast<const float4*>(rowmem), sub, G, (cnt + 1) >> 1,
-                                 nx, ny, nz, e2, p2x, p2y, p2z, sp, sx, sy, sz);
-        } else {
-          row_pairs<TPL, EX, SH>(static_cast<const vec4<T>*>(rowmem), sub, G, cnt, xi, eps2,
-                                 px, py, pz, sp, sx, sy, sz);
-        }
-      };
-      using TT = std::true_type;
-      using FF = std::false_type;
-      zero();
-      if (img != 0) {
-        pairs_of(FF(), TT());
-        if (!finite()) {
-          zero();
-          pairs_of(TT(), TT());
-        }
-      } else if (self) {
-        pairs_of(TT(), FF());
-      } else {
-        pairs_of(FF(), FF());
-        if (!finite()) {
-          zero();
-          pairs_of(TT(), FF());
+      const int total = __shfl_sync(full, incl, 31), excl = incl - cnj;
+      const int lo = max(0, min(total, p0 - cum)), hi = max(0, min(total, p1 - cum));
+      T shift[3] = {0, 0, 0};
+      if (img > 0) img_shift<T>(img, cycle, shift[0], shift[1], shift[2]);
+      for (int w0 = lo; w0 < hi; w0 += kP2PWindow) {
+        const int w1 = min(hi, w0 + kP2PWindow);
+        // every lane lists the bodies of its leaf that lie in the window
+        for (int p = max(excl, w0); p < min(incl, w1); p++) row.idx[p - w0] = dj0 - excl + p;
+        __syncwarp();
+        vec4<T> b;
+        bool own;
+        auto load = [&](int q) {
+          const int bj = q + lane < w1 ? row.idx[q - w0 + lane] : -1;
+          b = make_v4<T>(T(1e30), T(1e30), T(1e30), T(0));
+          if (bj >= 0) b = bodies[bj];
+          own = bj >= b0 && bj < b0 + nb;
+        };
+        load(w0);
+        for (int q = w0; q < w1; q += 32) {
+          const int cnt = min(32, w1 - q);
+          const bool self = __any_sync(full, own) && img == 0;  // (orders the last reads, too)
+          row.put(lane, b);
+          __syncwarp();
+          if (q + 32 < w1) load(q + 32);
+          if (self || exact) p2p_row<TPL, true, true>(row, sub, G, cnt, eps2, shift, t);
+          else if (img > 0) p2p_row<TPL, false, true>(row, sub, G, cnt, eps2, shift, t);
+          else p2p_row<TPL, false, false>(row, sub, G, cnt, eps2, shift, t);
+          __syncwarp();
+          if (++pending >= folds) {
+            p2p_fold<T, COMP, TPL>(t, acc, lane);
+            pending = 0;
+          }
         }
       }
-#pragma unroll
-      for (int u = 0; u < TPL; u++) {
-        T pot, ax, ay, az;
-        if constexpr (F32) {
-          pot = sp[u].x + sp[u].y;
-          ax = sx[u].x + sx[u].y;
-          ay = sy[u].x + sy[u].y;
-          az = sz[u].x + sz[u].y;
-        } else {
-          pot = sp[u];
-          ax = sx[u];
-          ay = sy[u];
-          az = sz[u];
-        }
-        if (COMP) {
-          comp_add(acc[u][0], pot);
-          comp_add(acc[u][1], ax);
-          comp_add(acc[u][2], ay);
-          comp_add(acc[u][3], az);
-        } else {
-          acc[u][0].s += pot;
-          acc[u][1].s += ax;
-          acc[u][2].s += ay;
-          acc[u][3].s += az;
-        }
-      }
-      // the next chunk: past leaves k .. cut - 1, or inside the leaf holding position 32
-      if (total <= 32) {
-        k = cut;
-        o = 0;
-      } else {
-        const int kn = __popc(__ballot_sync(full, lane < cut && incl <= 32));
-        const int exn = __shfl_sync(full, incl - avail, kn);
-        o = (kn == k ? o : 0) + 32 - exn;
-        k = kn;
-      }
+      if (!whole) cum += total;  // (a whole list has no end to reach)
+      k0 = cut;
     }
   }
-  for (int o = 1; o < G; o <<= 1) {
+  if (pending) p2p_fold<T, COMP, TPL>(t, acc, lane);
+}
+
+// one warp's part of a target leaf: up to 64 targets from body b0 + base on
+struct P2PTeam {
+  int base, G, s0, s1, S, p0, p1;
+  int folds;  // chunks between folds
+};
+template <typename T, bool COMP, int TPL>
+__device__ __forceinline__ void p2p_targets(const P2PTeam& w, int lane, Row<T>& row,
+                                            Accum<T, COMP>& mem, int b0, int nb,
+                                            const unsigned long long* __restrict__ srcs,
+                                            const vec4<T>* __restrict__ bodies, T eps2, T cycle,
+                                            vec4<T>* __restrict__ trg_s,
+                                            vec4<T>* __restrict__ trg_e) {
+  const int sub = lane % w.G, step = 32 / w.G;
+  const vec4<T> zero4 = make_v4<T>(0, 0, 0, 0);
+  Target<T> t[TPL];
+#pragma unroll
+  for (int u = 0; u < TPL; u++) {
+    const int i = w.base + u * step + lane / w.G;
+    t[u].set(i < nb ? bodies[b0 + i] : zero4);
+  }
+  for (int exact = 0; exact < 2; exact++) {
+#pragma unroll
+    for (int u = 0; u < TPL; u++) {
+      t[u].zero();
+      mem.s[u][lane] = zero4;
+      if constexpr (COMP) mem.e[u][lane] = zero4;
+    }
+    p2p_segment<T, COMP, TPL>(lane, row, b0, nb, sub, w.G, w.s0, w.s1, w.p0, w.p1, w.S == 1, w.folds, srcs,
+                              bodies, eps2, cycle, exact != 0, t, mem);
+    bool bad = false;
+#pragma unroll
+    for (int u = 0; u < TPL; u++)
+      bad |= w.base + u * step + lane / w.G < nb && !isfinite(mem.s[u][lane].x);
+    if (!__any_sync(0xffffffffu, bad)) break;
+  }
+  Comp<T> acc[TPL][4];
+#pragma unroll
+  for (int u = 0; u < TPL; u++) {
+    const vec4<T> s = mem.s[u][lane];
+    vec4<T> e = zero4;
+    if constexpr (COMP) e = mem.e[u][lane];
+    acc[u][0] = Comp<T>{s.x, e.x};
+    acc[u][1] = Comp<T>{s.y, e.y};
+    acc[u][2] = Comp<T>{s.z, e.z};
+    acc[u][3] = Comp<T>{s.w, e.w};
+  }
+  for (int o = 1; o < w.G; o <<= 1) {
 #pragma unroll
     for (int u = 0; u < TPL; u++)
 #pragma unroll
       for (int d = 0; d < 4; d++) {
-        Comp<T> r;
-        r.s = __shfl_xor_sync(full, acc[u][d].s, o);
-        r.e = __shfl_xor_sync(full, acc[u][d].e, o);
-        if (COMP) comp_merge(acc[u][d], r);
-        else acc[u][d].s += r.s;
+        Comp<T> r = {0, 0};
+        r.s = __shfl_xor_sync(0xffffffffu, acc[u][d].s, o);
+        if constexpr (COMP) {
+          r.e = __shfl_xor_sync(0xffffffffu, acc[u][d].e, o);
+          comp_merge(acc[u][d], r);
+        } else {
+          acc[u][d].s += r.s;
+        }
       }
   }
+  __syncwarp();
   if (sub == 0) {
 #pragma unroll
-    for (int u = 0; u < TPL; u++)
-      if (act[u]) {
-        trg_s[b0 + ti[u]] = make_v4<T>(acc[u][0].s, acc[u][1].s, acc[u][2].s, acc[u][3].s);
-        trg_e[b0 + ti[u]] = make_v4<T>(acc[u][0].e, acc[u][1].e, acc[u][2].e, acc[u][3].e);
+    for (int u = 0; u < TPL; u++) {
+      const int i = u * step + lane / w.G;
+      const vec4<T> s = make_v4<T>(acc[u][0].s, acc[u][1].s, acc[u][2].s, acc[u][3].s),
+                    e = make_v4<T>(acc[u][0].e, acc[u][1].e, acc[u][2].e, acc[u][3].e);
+      if (w.S > 1) {
+        mem.s[i >> 5][i & 31] = s;  // (every lane has taken its own accumulators out)
+        if constexpr (COMP) mem.e[i >> 5][i & 31] = e;
+      } else if (w.base + i < nb) {
+        trg_s[b0 + w.base + i] = s;
+        trg_e[b0 + w.base + i] = e;
       }
+    }
   }
 }
 
+constexpr int kP2PWarps = 8;  // per block, and of the largest team
+
+
+// order[i]: (first body, bodies, list begin, list end) of target leaf i in launch order, the
+// leaves of teams of 8 warps first, then 4, 2 and 1 (counts n8 .. n1); nsrc[i]: its source
+// bodies; srcs: the list's source leaves (p2p_leaf)
 template <typename T, bool COMP>
-__global__ void __launch_bounds__(32 * kP2PWarps)
-    k_p2p(const int* __restrict__ leaves, int nleaves, const int* __restrict__ off,
-          const unsigned long long* __restrict__ pairs, const int* __restrict__ ibody,
-          const int* __restrict__ nbody, const vec4<T>* __restrict__ bodies, T eps2, T cycle,
-          vec4<T>* __restrict__ trg_s, vec4<T>* __restrict__ trg_e, int g4, int g2) {
-  // one row of 32 sources per warp
-  __shared__ __align__(16) unsigned char smem[kP2PWarps][32 * sizeof(vec4<T>)];
-  const int wl = threadIdx.x >> 5;
-  const int w = blockIdx.x * kP2PWarps + wl;
-  if (w >= nleaves) return;
-  const int lane = lane_id();
-  const int c = leaves[w];
-  const int b0 = ibody[c], nb = nbody[c];
-  const int G = nb <= g4 ? 4 : (nb <= g2 ? 2 : 1);
-  const int s0 = off[c], s1 = off[c + 1];
-  void* row = smem[wl];
-  if (nb <= 32) {
-    p2p_leaf_chunked<T, COMP, 1>(lane, row, b0, nb, 0, G, s0, s1, pairs, ibody, nbody, bodies,
-                                 eps2, cycle, trg_s, trg_e);
-  } else {
-    for (int base = 0; base < nb; base += 64)
-      p2p_leaf_chunked<T, COMP, 2>(lane, row, b0, nb, base, 1, s0, s1, pairs, ibody, nbody,
-                                   bodies, eps2, cycle, trg_s, trg_e);
+__global__ void __launch_bounds__(32 * kP2PWarps, sizeof(T) == 4 ? 2 : 3)
+    k_p2p(const int4* __restrict__ order, const int* __restrict__ nsrc, int n8, int n4, int n2,
+          int n1, const unsigned long long* __restrict__ srcs,
+          const vec4<T>* __restrict__ bodies, T eps2, T cycle, vec4<T>* __restrict__ trg_s,
+          vec4<T>* __restrict__ trg_e, int g4, int g2, int images) {
+  __shared__ Row<T> rows[kP2PWarps];
+  __shared__ Accum<T, COMP> mem[kP2PWarps];
+  const int wl = threadIdx.x >> 5, lane = lane_id();
+  // the block's class: S warps per leaf, kP2PWarps / S leaves of the block
+  int blk = blockIdx.x, first = 0, cls = n8, S = 8;
+  const int rest[3] = {n4, n2, n1};
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int blocks = (cls * S + kP2PWarps - 1) / kP2PWarps;
+    if (blk >= blocks) {
+      blk -= blocks;
+      first += cls;
+      cls = rest[k];
+      S >>= 1;
+    } else {
+      break;
+    }
   }
+  const int at = blk * (kP2PWarps / S) + wl / S, seg = wl % S;
+  if (at >= cls) return;  // the whole team
+  const int4 leaf = order[first + at];
+  const int b0 = leaf.x, nb = leaf.y, s0 = leaf.z, s1 = leaf.w;
+  const int G = p2p_lanes<T>(nb, g4, g2, images);
+  const int ns = nsrc[first + at];
+  const int per = (ns + 32 * S - 1) / (32 * S) * 32;
+  const int p0 = S == 1 ? 0 : min(ns, per * seg), p1 = S == 1 ? INT_MAX : min(ns, p0 + per);
+  P2PTeam w{0, G, s0, s1, S, p0, p1, images ? 1 : G};
+  const int team = wl / S, bar = 1 + team, thr = 32 * S;
+  for (int base = 0; base < nb; base += 64) {
+    w.base = base;
+    const int tpl = (min(64, nb - base) * G + 31) / 32;
+    auto run = [&](auto n) {
+      p2p_targets<T, COMP, decltype(n)::value>(w, lane, rows[wl], mem[wl], b0, nb, srcs,
+                                               bodies, eps2, cycle, trg_s, trg_e);
+    };
+    if (tpl == 1) run(std::integral_constant<int, 1>());
+    else if (tpl == 2 || p2p_tpl<T>() == 2) run(std::integral_constant<int, 2>());
+    else if constexpr (p2p_tpl<T>() > 2) {
+      run(std::integral_constant<int, 3>());
+    }
+    if (S == 1) continue;
+    // the team's warps: partial sums through shared memory, added in warp order
+    asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(thr) : "memory");
+    const int t = seg * 32 + lane;
+    if (t < 64 && base + t < nb) {
+      vec4<T> s = mem[team * S].s[t >> 5][lane], e = make_v4<T>(0, 0, 0, 0);
+      if constexpr (COMP) e = mem[team * S].e[t >> 5][lane];
+      Comp<T> a[4] = {{s.x, e.x}, {s.y, e.y}, {s.z, e.z}, {s.w, e.w}};
+      for (int k = 1; k < S; k++) {
+        const vec4<T> u = mem[team * S + k].s[t >> 5][lane];
+        if constexpr (COMP) {
+          const vec4<T> d = mem[team * S + k].e[t >> 5][lane];
+          comp_merge(a[0], Comp<T>{u.x, d.x});
+          comp_merge(a[1], Comp<T>{u.y, d.y});
+          comp_merge(a[2], Comp<T>{u.z, d.z});
+          comp_merge(a[3], Comp<T>{u.w, d.w});
+        } else {
+          a[0].s += u.x, a[1].s += u.y, a[2].s += u.z, a[3].s += u.w;
+        }
+      }
+      trg_s[b0 + base + t] = make_v4<T>(a[0].s, a[1].s, a[2].s, a[3].s);
+      trg_e[b0 + base + t] = make_v4<T>(a[0].e, a[1].e, a[2].e, a[3].e);
+    }
+    if (base + 64 < nb) asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(thr) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------- launch order
+// Target leaves by team size, within a size by descending work (the longest start first, so
+// that none is left alone at the end): a counting sort on (class, quarter octaves of source
+// bodies times targets).  The order inside a bucket follows the atomics; no result depends
+// on it.
+constexpr int kSubBuckets = 192;
+constexpr int kP2PBuckets = 4 * kSubBuckets;
+
+// Class (0 .. 3: a team of 8, 4, 2, 1 warps) of a leaf of nb bodies with `src` source bodies:
+// `share` pairs per lane of a warp or more, so that the team's start and its merge (about 500
+// instructions a warp) stay small beside its pairs.  One warp for a count that no int holds, and
+// with periodic images (see p2p_lanes).
+__device__ __forceinline__ int p2p_class(unsigned long long src, int nb, int share) {
+  if (src > INT_MAX / 2) return 3;
+  const unsigned long long w = src * (unsigned long long)min(64, (nb + 3) / 4 * 4) / 32;
+  return w >= 8ULL * share ? 0 : w >= 4ULL * share ? 1 : w >= 2ULL * share ? 2 : 3;
+}
+
+__global__ void __launch_bounds__(256)
+    k_p2p_work(int nleaves, const int* __restrict__ leaves, const int* __restrict__ off,
+               const unsigned long long* __restrict__ pairs, const int4* __restrict__ info,
+               unsigned long long* __restrict__ srcs, int* __restrict__ bucket,
+               int* __restrict__ work, int* __restrict__ hist, int share) {
+  __shared__ int h[kP2PBuckets];
+  for (int i = threadIdx.x; i < kP2PBuckets; i += blockDim.x) h[i] = 0;
+  __syncthreads();
+  const int lane = lane_id(), nw = gridDim.x * (blockDim.x >> 5);
+  for (int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nleaves; i += nw) {
+    const int c = leaves[i];
+    unsigned long long src = 0;
+    for (int k = off[c] + lane; k < off[c + 1]; k += 32) {
+      const unsigned p = (unsigned)pairs[k];
+      const int4 f = info[pair_cell(p)];
+      src += (unsigned)f.z;
+      srcs[k] = p2p_leaf(f, pair_img(p));
+    }
+    src = warp_sum(src);
+    if (lane == 0) {
+      const unsigned long long w = src * (unsigned long long)max(8, info[c].z) | 4ULL;
+      const int e = 63 - __clzll(w);
+      const int q = 4 * e + (int)((w >> (e - 2)) & 3);
+      const int b = p2p_class(src, info[c].z, share) * kSubBuckets + kSubBuckets - 1 - min(q, kSubBuckets - 1);
+      bucket[i] = b;
+      work[i] = (int)min(src, (unsigned long long)INT_MAX);
+      atomicAdd(&h[b], 1);
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < kP2PBuckets; i += blockDim.x)
+    if (h[i]) atomicAdd(&hist[i], h[i]);
+}
+
+// cursor: kP2PBuckets zeros on entry; teams[0..3]: leaves of teams of 8, 4, 2, 1 warps
+__global__ void __launch_bounds__(256)
+    k_p2p_place(int nleaves, const int* __restrict__ leaves, const int* __restrict__ bucket,
+                const int* __restrict__ work, const int* __restrict__ hist,
+                const int* __restrict__ off, const int4* __restrict__ info,
+                int* __restrict__ cursor, int* __restrict__ teams, int4* __restrict__ order,
+                int* __restrict__ nsrc) {
+  constexpr int PER = kP2PBuckets / 256;
+  __shared__ int start[kP2PBuckets], wsum[8];
+  const int lane = lane_id(), wl = threadIdx.x >> 5;
+  int v[PER], sum = 0;
+#pragma unroll
+  for (int k = 0; k < PER; k++) {
+    v[k] = hist[threadIdx.x * PER + k];
+    sum += v[k];
+  }
+  int incl = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += u;
+  }
+  if (lane == 31) wsum[wl] = incl;
+  __syncthreads();
+  int run = incl - sum;
+  for (int k = 0; k < wl; k++) run += wsum[k];
+#pragma unroll
+  for (int k = 0; k < PER; k++) {
+    start[threadIdx.x * PER + k] = run;
+    run += v[k];
+  }
+  __syncthreads();
+  if (blockIdx.x == 0 && threadIdx.x < 4) {
+    const int k = threadIdx.x;
+    teams[k] = (k < 3 ? start[(k + 1) * kSubBuckets] : nleaves) - start[k * kSubBuckets];
+  }
+  for (int i0 = blockIdx.x * blockDim.x; i0 < nleaves; i0 += gridDim.x * blockDim.x) {
+    const int i = i0 + threadIdx.x;
+    const unsigned act = __ballot_sync(0xffffffffu, i < nleaves);
+    if (i >= nleaves) continue;
+    const int b = bucket[i];
+    const unsigned grp = __match_any_sync(act, b);
+    const int leader = __ffs(grp) - 1;
+    int pos = 0;
+    if (lane == leader) pos = atomicAdd(&cursor[b], __popc(grp));
+    pos = __shfl_sync(grp, pos, leader) + start[b] + __popc(grp & ((1u << lane) - 1));
+    const int c = leaves[i];
+    order[pos] = make_int4(info[c].w, info[c].z, off[c], off[c + 1]);
+    nsrc[pos] = work[i];
+  }
+}
+
+// the launch order of the current P2P lists, on the solver's current stream; the team counts
+// reach s.scal_host (kP2PTeamsHost) once that stream has been waited for
+void order_p2p_targets(SolverBase& s) {
+  const int nl = s.nleaves;
+  if (nl <= 0) return;
+  s.p2p_srcs.ensure(std::max<long long>(s.np2p, 1));
+  s.p2p_bucket.ensure(nl);
+  s.p2p_work.ensure(nl);
+  s.p2p_order.ensure(nl);
+  s.p2p_nsrc.ensure(nl);
+  s.p2p_hist.ensure(2 * kP2PBuckets + 4);
+  int *hist = s.p2p_hist.p, *cursor = hist + kP2PBuckets, *teams = cursor + kP2PBuckets;
+  FMM_CUDA(cudaMemsetAsync(hist, 0, 2 * kP2PBuckets * sizeof(int), s.stream));
+  k_p2p_work<<<std::min(ceil_div(nl, 8), 148 * 4), 256, 0, s.stream>>>(
+      nl, s.leaves.p, s.p2p_off.p, s.p2p.p, s.c_info.p, s.p2p_srcs.p,
+      s.p2p_bucket.p, s.p2p_work.p, hist,
+      s.cfg.images > 0 ? INT_MAX : s.cfg.precision == FMM_FP32 ? 512 : 192);
+  FMM_LAUNCH_CHECK();
+  k_p2p_place<<<std::min(ceil_div(nl, 256), 148 * 4), 256, 0, s.stream>>>(
+      nl, s.leaves.p, s.p2p_bucket.p, s.p2p_work.p, hist, s.p2p_off.p, s.c_info.p, cursor, teams,
+      s.p2p_order.p, s.p2p_nsrc.p);
+  FMM_LAUNCH_CHECK();
+  FMM_CUDA(cudaMemcpyAsync(s.scal_host + kP2PTeamsHost, teams, 4 * sizeof(int),
+                           cudaMemcpyDeviceToHost, s.stream));
+  s.p2p_ordered = true;
 }
 
 template <typename T> void run_p2p(Solver<T>& s) {
   if (s.nleaves == 0) return;
   constexpr bool comp = sizeof(T) == 4;
-  k_p2p<T, comp><<<ceil_div(s.nleaves, kP2PWarps), 32 * kP2PWarps, 0, s.stream>>>(
-      s.p2p_ordered ? s.p2p_order.p : s.leaves.p, s.nleaves, s.p2p_off.p, s.p2p.p, s.c_ibody.p, s.c_nbody.p, s.bodies.p,
-      (T)s.cfg.eps2, (T)s.cfg.cycle, s.trg_s.p, s.trg_e.p, std::min(s.p2p_g4, 8),
-      std::min(s.p2p_g2, 16));
+  const int* t = s.scal_host + kP2PTeamsHost;
+  const long long blocks = (long long)t[0] + ceil_div(4LL * t[1], kP2PWarps) +
+                           ceil_div(2LL * t[2], kP2PWarps) + ceil_div(t[3], kP2PWarps);
+  k_p2p<T, comp><<<(int)blocks, 32 * kP2PWarps, 0, s.stream>>>(
+      s.p2p_order.p, s.p2p_nsrc.p, t[0], t[1], t[2], t[3], s.p2p_srcs.p,
+      s.bodies.p, (T)s.cfg.eps2, (T)s.cfg.cycle, s.trg_s.p, s.trg_e.p, std::min(s.p2p_g4, 8),
+      std::min(s.p2p_g2, 16), s.cfg.images > 0);
   FMM_LAUNCH_CHECK();
 }
 

@@ -168,10 +168,11 @@ struct SolverBase {
   bool p2p_pending = false;
   cudaEvent_t p2p_ready = nullptr;
   DevArr<int> m2l_tgt;  // M2L target cells, by descending number of 32-source batches
-  // P2P target leaves by descending body pairs (valid while p2p_ordered: the lists of the
-  // last traversal), so that the longest leaves start first and none is left alone at the end
-  DevArr<int> p2p_order, p2p_widx;
-  DevArr<unsigned> p2p_wkey, p2p_wkey2;
+  // P2P target leaves in launch order (valid while p2p_ordered: the lists of the last
+  // traversal), each with its source bodies; scratch of the ordering
+  DevArr<int4> p2p_order;
+  DevArr<int> p2p_nsrc, p2p_bucket, p2p_work, p2p_hist;
+  DevArr<unsigned long long> p2p_srcs;  // source leaves of the P2P pairs as k_p2p reads them
   bool p2p_ordered = false;
   int m2l_ntgt = 0;
   DevArr<unsigned long long> p2p_pairs_count;
@@ -216,6 +217,9 @@ template <typename T> void downward_pass(Solver<T>& s);       // fmm_passes.cu
 template <typename T> void downward_l2l(Solver<T>& s);        // fmm_passes.cu: L2L levels
 template <typename T> void downward_l2p(Solver<T>& s);        // fmm_passes.cu: L2P + output
 template <typename T> void build_lists(Solver<T>& s, bool defer_p2p = false);  // fmm_traverse.cu
+void order_p2p_targets(SolverBase& s);  // fmm_p2p.cu: launch order of the current P2P lists
+constexpr int kP2PTeamsHost = 480;      // scal_host: its four team counts, after a wait
+void fill_cell_info(SolverBase& s);     // fmm_tree.cu: c_info from the cells' index fields
 void finish_p2p_list(SolverBase& s);  // fmm_traverse.cu: after build_lists(s, true)
 template <typename T> void run_m2l(Solver<T>& s);             // fmm_passes.cu
 template <typename T> void run_p2p(Solver<T>& s);             // fmm_p2p.cu

@@ -764,42 +764,11 @@ void finish_p2p_list(SolverBase& s) {
   if (hflow[1]) {
     FMM_CUDA(cudaStreamWaitEvent(s.stream, s.p2p_ready, 0));
     global_sort_list(s, s.p2p.p, s.np2p, bits_for(s.ncells), s.cfg.images > 0 ? 5 : 0);
+    order_p2p_targets(s);
     FMM_CUDA(cudaStreamSynchronize(s.stream));
   } else {
     FMM_CUDA(cudaStreamWaitEvent(s.stream, s.p2p_ready, 0));
   }
-}
-
-// P2P work of each leaf, as a descending sort key: its bodies times the bodies of its
-// source leaves (0 without pairs)
-__global__ void k_p2p_work(int nleaves, const int* __restrict__ leaves,
-                           const int* __restrict__ off,
-                           const unsigned long long* __restrict__ pairs,
-                           const int* __restrict__ nbody, unsigned* __restrict__ key,
-                           int* __restrict__ idx) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= nleaves) return;
-  const int c = leaves[i];
-  unsigned long long src = 0;
-  for (int k = off[c]; k < off[c + 1]; k++) src += nbody[pair_cell((unsigned)pairs[k])];
-  const unsigned long long w = src * (unsigned long long)nbody[c];
-  key[i] = ~(unsigned)(w < 0xffffffffULL ? w : 0xffffffffULL);
-  idx[i] = c;
-}
-
-// the leaves in the order of k_p2p_work's keys, on the solver's current stream
-static void order_p2p_targets(SolverBase& s, DevArr<char>* tmp) {
-  const int nl = s.nleaves;
-  if (nl <= 0) return;
-  s.p2p_wkey.ensure(nl);
-  s.p2p_wkey2.ensure(nl);
-  s.p2p_widx.ensure(nl);
-  s.p2p_order.ensure(nl);
-  k_p2p_work<<<ceil_div(nl, 256), 256, 0, s.stream>>>(nl, s.leaves.p, s.p2p_off.p, s.p2p.p,
-                                                      s.c_nbody.p, s.p2p_wkey.p, s.p2p_widx.p);
-  FMM_LAUNCH_CHECK();
-  sort_pairs_u32(s, s.p2p_wkey.p, s.p2p_wkey2.p, s.p2p_widx.p, s.p2p_order.p, nl, 32, tmp);
-  s.p2p_ordered = true;
 }
 
 template <typename T> void build_lists(Solver<T>& s, bool defer_p2p) {
@@ -846,7 +815,7 @@ template <typename T> void build_lists(Solver<T>& s, bool defer_p2p) {
     try {
       group_by_target(s, s.p2p.p, np2p, b, s.p2p_off.p, overflow + 1, s.seg_cnt2.p,
                       s.seg_keys2.p, &s.cub_tmp2);
-      order_p2p_targets(s, &s.cub_tmp2);
+      order_p2p_targets(s);
       FMM_CUDA(cudaMemcpyAsync((int*)(hc + 5) + 1, overflow + 1, sizeof(int),
                                cudaMemcpyDeviceToHost, s.stream));
       FMM_CUDA(cudaEventRecord(s.p2p_ready, s.stream));
@@ -858,7 +827,7 @@ template <typename T> void build_lists(Solver<T>& s, bool defer_p2p) {
   } else {
     group_by_target(s, s.p2p.p, np2p, b, s.p2p_off.p, overflow + 1, s.seg_cnt.p,
                     (unsigned*)s.list_tmp.p, nullptr);
-    order_p2p_targets(s, nullptr);
+    order_p2p_targets(s);
   }
   // M2L target order: by descending pair count in buckets (stable in cell index)
   {
@@ -883,7 +852,10 @@ template <typename T> void build_lists(Solver<T>& s, bool defer_p2p) {
   const int* hflow = (const int*)(hc + 5);
   if (hflow[0] || (!s.p2p_pending && hflow[1])) {
     if (hflow[0]) global_sort_list(s, s.m2l.p, nm2l, b, ib);
-    if (!s.p2p_pending && hflow[1]) global_sort_list(s, s.p2p.p, np2p, b, ib);
+    if (!s.p2p_pending && hflow[1]) {
+      global_sort_list(s, s.p2p.p, np2p, b, ib);
+      order_p2p_targets(s);
+    }
     FMM_CUDA(cudaStreamSynchronize(s.stream));
   }
   s.p2p_body_pairs = -1;  // counted when asked for (count_p2p_body_pairs)

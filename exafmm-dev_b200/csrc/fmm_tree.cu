@@ -419,6 +419,13 @@ __global__ void k_cell_info(int ncells, const int* __restrict__ nchild,
   if (c < ncells) info[c] = make_int4(nchild[c], ichild[c], nbody[c], ibody[c]);
 }
 
+void fill_cell_info(SolverBase& s) {
+  s.c_info.ensure(s.ncells);
+  k_cell_info<<<ceil_div(s.ncells, 256), 256, 0, s.stream>>>(
+      s.ncells, s.c_nchild.p, s.c_ichild.p, s.c_nbody.p, s.c_ibody.p, s.c_info.p);
+  FMM_LAUNCH_CHECK();
+}
+
 // Cell records (Nodes2cells::operator(), include/build_tree_tbb.h:250-262) with the
 // Morton index of getKey (:240-249) in 64-bit arithmetic.
 template <typename T>

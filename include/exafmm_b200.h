@@ -268,8 +268,9 @@ int fmm_b200_solve_ij_device(fmm_b200_solver* s, int nt, const void* d_targets, 
 int fmm_b200_autotune_ncrit(fmm_b200_solver* s, const int* candidates, int ncand, int repeats,
                             int* best_ncrit, double* times_ms);
 /* Picks the P2P kernel's threads per target group (lanes that share one target body) on the
- * interaction lists of the handle's last solve: candidate i gives a target 4 lanes in leaves
- * of at most lanes4_max[i] bodies, 2 lanes in leaves of at most lanes2_max[i], else 1
+ * interaction lists of the handle's last solve: candidate i sets the leaf sizes up to which a
+ * target takes the most lanes (lanes4_max[i] bodies: 4, in FP32 8 up to half as many again) and
+ * half as many (lanes2_max[i]); larger leaves take fewer
  * (0 <= lanes4_max <= 8, lanes4_max <= lanes2_max <= 16; the default is 8 / 16).  Each runs the
  * P2P `repeats` times after one untimed run; the median device time goes to times_ms[i]
  * (may be NULL) and the fastest becomes the handle's (index in *best).  The split of a
