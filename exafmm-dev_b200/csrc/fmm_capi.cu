@@ -113,12 +113,12 @@ template <typename T> void set_bodies_host_t(Solver<T>& s, int n, const double* 
   s.stage = ST_BODIES;
 }
 
-template <typename T> void stage_tree(Solver<T>& s) {
+template <typename T> void stage_tree(Solver<T>& s, bool radii = false) {
   if (s.stage < ST_BODIES) throw FmmError(FMM_ERR_STATE, "bodies not set");
   for (int p = 0; p < FMM_NUM_PHASES; p++) s.ev_used[p] = false;
   phase_begin(s, FMM_PHASE_TOTAL);
   phase_begin(s, FMM_PHASE_BOUNDS);
-  build_tree(s);
+  build_tree(s, radii);
   partition_range(s);
   if (s.n == 0) phase_end(s, FMM_PHASE_BOUNDS);
   else phase_end(s, FMM_PHASE_TREE);
@@ -166,7 +166,7 @@ template <typename T> void stage_down(Solver<T>& s) {
 // soon as SMs free up.  The results are the same as stage by stage: P2P writes only the
 // bodies' sums, L2L only the local expansions, and L2P runs after both.
 template <typename T> void solve_all(Solver<T>& s) {
-  stage_tree(s);
+  stage_tree(s, true);
   if (!s.side) {
     int lo = 0, hi = 0;
     FMM_CUDA(cudaDeviceGetStreamPriorityRange(&lo, &hi));
@@ -466,8 +466,7 @@ int fmm_b200_create(const fmm_b200_config* cfg, fmm_b200_solver** out) {
                          &s_.coff,     &s_.leaves,   &s_.idx,      &s_.idx2,    &s_.scal,   \
                          &s_.c_iparent, &s_.c_ichild, &s_.c_nchild, &s_.c_ibody, &s_.c_nbody, \
                          &s_.c_level,  &s_.order,    &s_.m2l_off,  &s_.p2p_off, &s_.seg_cnt, \
-                         &s_.d_lvl,    &s_.seg_cnt2, &s_.body_leaf, &s_.d_seg,  &s_.d_root_first, \
-                         &s_.d_root_count, &s_.nsid, &s_.c_root,   &s_.cbase,   &s_.fs_pos, \
+                         &s_.tree_ctl, &s_.seg_cnt2, &s_.body_leaf, &s_.d_seg,  &s_.nsid, &s_.c_root,   &s_.cbase,   &s_.fs_pos, \
                          &s_.fs_pos2,  &s_.fs_idx,   &s_.m2l_tgt,  &s_.k_list,  &s_.k_saved_leaves, \
                          &s_.p2p_bucket, &s_.p2p_hist, &s_.p2p_nsrc, &s_.p2p_work}; \
     for (auto* a : ia) a->OP();                                                            \
@@ -480,13 +479,13 @@ int fmm_b200_create(const fmm_b200_config* cfg, fmm_b200_solver** out) {
     if ((h)->precision == FMM_FP64) {                                                      \
       Solver<double>& d_ = *static_cast<Solver<double>*>((h)->base);                       \
       d_.bodies_in.OP(); d_.bodies.OP(); d_.trg_s.OP(); d_.trg_e.OP(); d_.trg_out.OP();    \
-      d_.cX.OP(); d_.box.OP(); d_.M.OP(); d_.L.OP(); d_.nX.OP(); d_.m0.OP();               \
+      d_.cX.OP(); d_.box.OP(); d_.M.OP(); d_.L.OP(); d_.nX.OP(); d_.nM0.OP(); d_.m0.OP(); \
       d_.pM.OP(); d_.pM2.OP(); d_.pC.OP(); d_.c_root_cells.OP(); d_.minmax_part.OP();      \
       d_.k_rows.OP(); d_.k_cx.OP(); d_.k_trg.OP(); d_.m2l_rows.OP();                                         \
     } else {                                                                               \
       Solver<float>& d_ = *static_cast<Solver<float>*>((h)->base);                         \
       d_.bodies_in.OP(); d_.bodies.OP(); d_.trg_s.OP(); d_.trg_e.OP(); d_.trg_out.OP();    \
-      d_.cX.OP(); d_.box.OP(); d_.M.OP(); d_.L.OP(); d_.nX.OP(); d_.m0.OP();               \
+      d_.cX.OP(); d_.box.OP(); d_.M.OP(); d_.L.OP(); d_.nX.OP(); d_.nM0.OP(); d_.m0.OP(); \
       d_.pM.OP(); d_.pM2.OP(); d_.pC.OP(); d_.c_root_cells.OP(); d_.minmax_part.OP();      \
       d_.k_rows.OP(); d_.k_cx.OP(); d_.k_trg.OP(); d_.m2l_rows.OP();                                         \
     }                                                                                      \
@@ -515,6 +514,7 @@ int fmm_b200_destroy(fmm_b200_solver* h) {
     if (s.p2p_ready) cudaEventDestroy(s.p2p_ready);
     if (s.scal_host) cudaFreeHost(s.scal_host);
     if (s.roots_host) cudaFreeHost(s.roots_host);
+    if (s.seg_host) cudaFreeHost(s.seg_host);
     for (int2* q : s.roots_retired) cudaFreeHost(q);
     delete h->base;
   }

@@ -153,17 +153,19 @@ template <typename T> void upward_pass(Solver<T>& s) {
 template <typename T> void structure_pass(Solver<T>& s) {
   if (s.ncells == 0) return;
   const int TB = 128;
-  s.m0.ensure(s.ncells);
-  k_struct_leaves<T><<<ceil_div(32LL * s.nleaves, TB), TB, 0, s.stream>>>(
-      s.leaves.p, s.nleaves, s.c_ibody.p, s.c_nbody.p, s.cX.p, s.bodies.p, s.m0.p,
-      s.cfg.use_rmax, (T)s.cfg.theta);
-  FMM_LAUNCH_CHECK();
-  for (int l = s.maxlevel - 1; l >= 0; l--) {
-    const int lo = s.level_lo[l], hi = s.level_lo[l + 1];
-    k_struct_level<T><<<ceil_div(hi - lo, TB), TB, 0, s.stream>>>(
-        lo, hi, s.npos.p, s.c_ichild.p, s.c_nchild.p, s.cX.p, s.m0.p, s.cfg.use_rmax,
-        (T)s.cfg.theta);
+  if (!s.radii_set) {  // (the tree kernel sets them where a warp ranks every leaf)
+    s.m0.ensure(s.ncells);
+    k_struct_leaves<T><<<ceil_div(32LL * s.nleaves, TB), TB, 0, s.stream>>>(
+        s.leaves.p, s.nleaves, s.c_ibody.p, s.c_nbody.p, s.cX.p, s.bodies.p, s.m0.p,
+        s.cfg.use_rmax, (T)s.cfg.theta);
     FMM_LAUNCH_CHECK();
+    for (int l = s.maxlevel - 1; l >= 0; l--) {
+      const int lo = s.level_lo[l], hi = s.level_lo[l + 1];
+      k_struct_level<T><<<ceil_div(hi - lo, TB), TB, 0, s.stream>>>(
+          lo, hi, s.npos.p, s.c_ichild.p, s.c_nchild.p, s.cX.p, s.m0.p, s.cfg.use_rmax,
+          (T)s.cfg.theta);
+      FMM_LAUNCH_CHECK();
+    }
   }
   if (s.cfg.use_ropt) {
     k_ropt<T><<<ceil_div(s.ncells, 256), 256, 0, s.stream>>>(s.ncells, s.cX.p, s.m0.p, s.c_root.p,

@@ -102,7 +102,10 @@ struct SolverBase {
   std::vector<int> root_solve;  // solve of each root
   std::vector<int> root_cell;   // first cell of each root (host copy)
   int nroots = 0;
-  DevArr<int> d_seg, d_root_first, d_root_count, nsid, c_root, cbase;
+  DevArr<int> d_seg, nsid, c_root, cbase;
+  const int* root_first = nullptr;  // device: first body of each root, and the end (in d_seg)
+  int* seg_host = nullptr;          // pinned staging of d_seg
+  size_t seg_host_cap = 0;
   int ncoef = 0, nterm = 0;
   Stage stage = ST_NONE;
   std::string err;
@@ -139,12 +142,13 @@ struct SolverBase {
   DevArr<int2> front, front2;
   bool trav_sized = false;  // list / frontier buffers sized by a counted traversal
   int trav_steps = 0, trav_maxlevel = 0;  // the last traversal's steps, and its tree depth
-  int tree_plan = 0;        // levels of the handle's last tree (0: none; builds level by level)
+  int tree_plan = 0;        // levels of the handle's last tree (0: none)
   int write_r = 1;          // P2M / M2M set the cell radii (else the structure pass did)
   // P2P lanes per target by target leaf size: 4 up to p2p_g4 bodies, 2 up to p2p_g2, else 1
   // (p2p_g4 <= 8 and p2p_g2 <= 16: a warp holds 32 / lanes targets); fmm_b200_autotune_p2p
   int p2p_g4 = 8, p2p_g2 = 16;
-  DevArr<int> d_lvl;        // level ends of the planned node build
+  DevArr<int> tree_ctl;     // control block of the tree kernel
+  bool radii_set = false;   // the tree kernel has set the cells' radii and monopoles
   // targets and sources in two trees (segments 0 and 1) on a common box, traversed from
   // (target root, source root) only (fmm_b200_solve_ij_*)
   bool ij = false;
@@ -196,7 +200,7 @@ struct SolverBase {
 template <typename T> struct Solver : SolverBase {
   DevArr<vec4<T>> bodies_in, bodies, trg_s, trg_e, trg_out, cX;
   DevArr<T> box;  // per root, 16 values: X0[3], R0, Xmin[3], Xmax[3]
-  DevArr<T> M, L, nX;
+  DevArr<T> M, L, nX, nM0;
   DevArr<T> m2l_rows;  // spherical M2L: the multipoles by order (sph::col_idx)
   DevArr<T> m0;  // monopole per cell (structure pass)
   DevArr<T> pM, pM2, pC;  // periodic cell multipoles and per-shift M2L terms
@@ -207,7 +211,8 @@ template <typename T> struct Solver : SolverBase {
 };
 
 // ---- stage implementations (one translation unit each) ---------------------------------
-template <typename T> void build_tree(Solver<T>& s);          // fmm_tree.cu
+// fmm_tree.cu; radii: set the cells' radii and monopoles too, where it can (s.radii_set)
+template <typename T> void build_tree(Solver<T>& s, bool radii = false);
 void partition_range(SolverBase& s);                         // fmm_tree.cu: part_range
 long long count_p2p_body_pairs(SolverBase& s);              // fmm_traverse.cu
 template <typename T> void upward_pass(Solver<T>& s);         // fmm_passes.cu
@@ -218,6 +223,7 @@ template <typename T> void downward_l2l(Solver<T>& s);        // fmm_passes.cu: 
 template <typename T> void downward_l2p(Solver<T>& s);        // fmm_passes.cu: L2P + output
 template <typename T> void build_lists(Solver<T>& s, bool defer_p2p = false);  // fmm_traverse.cu
 void order_p2p_targets(SolverBase& s);  // fmm_p2p.cu: launch order of the current P2P lists
+constexpr int kTreeHost = 320;           // scal_host: control block of the tree kernel
 constexpr int kP2PTeamsHost = 480;      // scal_host: its four team counts, after a wait
 void fill_cell_info(SolverBase& s);     // fmm_tree.cu: c_info from the cells' index fields
 void finish_p2p_list(SolverBase& s);  // fmm_traverse.cu: after build_lists(s, true)

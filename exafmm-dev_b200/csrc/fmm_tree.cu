@@ -10,6 +10,7 @@
 // as the stable partitions leave them, via a second stable sort by leaf-truncated key.
 // Cells take the reference's layout (Nodes2cells :250-294): root first, the children of a
 // cell contiguous, each child's subtree after the previous child's.
+#include <algorithm>
 #include <cfloat>
 
 #include <climits>
@@ -170,244 +171,380 @@ __device__ __forceinline__ int digit_at(unsigned long long key, int level) {
   return (int)((key >> (3 * (kMaxLevel - 1 - level))) & 7ULL);
 }
 
-// one root node per non-empty solve, in solve order
-template <typename T>
-__global__ void k_roots(int nroots, const int* __restrict__ root_first, const T* __restrict__ box,
-                        int* nbegin, int* ncount, int* nparent, int* nlevel, int* nsid, T* nX) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= nroots) return;
-  nbegin[r] = root_first[r];
-  ncount[r] = root_first[r + 1] - root_first[r];
-  nparent[r] = -1;
-  nlevel[r] = 0;
-  nsid[r] = r;
-  for (int d = 0; d < 3; d++) nX[4 * r + d] = box[16 * r + d];
-  nX[4 * r + 3] = 0;
-}
+// ---------------------------------------------------------------- the tree, in one kernel
+// Everything between the key sort and the cells is a few dozen small steps, each over one
+// level of nodes and each needing the one before: as launches of their own (a split, a scan
+// and an emission per level, the subtree sizes up and the cell slots down) they were 45 to 75
+// launches of 2-4 us.  k_tree runs them as one cooperative launch with a barrier of its blocks
+// between steps (about 1.5 us).  Bound by latency throughout: a warp's split is two to three
+// dependent rounds of key reads.
+//
+// The barrier counts arrivals up; a block that waits longer than kSyncSpins polls (seconds)
+// sets *fault and every block leaves at its next barrier.
+constexpr int kSyncSpins = 1 << 24;
 
-// One level of BuildNodes (include/build_tree_tbb.h:165-218): a node with more than ncrit
-// bodies gets one child per non-empty octant; octant boundaries by binary search.
-// One warp per node: the 7 octant boundaries of its sorted key range are found together by
-// 32-ary searches (32 samples per boundary and round, all loads of a round independent), so
-// a node of c bodies needs log32(c) dependent rounds instead of the 7 log2(c) of a binary
-// search per boundary.  Node w of the level (v = lo + w): child count into cnt[w], octant
-// starts into starts[9 w ..].
-__device__ __forceinline__ void split_node(int lane, int w, int v, int level, int ncrit,
-                                           const unsigned long long* __restrict__ keys,
-                                           const int* __restrict__ nbegin,
-                                           const int* __restrict__ ncount,
-                                           int* __restrict__ cnt, int* __restrict__ starts) {
-  const int b = nbegin[v], c = ncount[v];
-  int nch = 0;
-  if (c > ncrit && level < kMaxLevel) {
-    int* st = starts + 9 * w;
-    int slo[8], shi[8];
-#pragma unroll
-    for (int o = 1; o < 8; o++) {
-      slo[o] = b;
-      shi[o] = b + c;
-    }
-    // invariant: the first index whose octant digit is >= o lies in [slo[o], shi[o]]
-    for (;;) {
-      bool open = false;
-#pragma unroll
-      for (int o = 1; o < 8; o++) open |= slo[o] < shi[o];
-      if (!open) break;
-      unsigned ball[8];
-      int step[8];
-#pragma unroll
-      for (int o = 1; o < 8; o++) {
-        const int len = shi[o] - slo[o];
-        step[o] = len <= 32 ? 1 : (len + 31) / 32;
-        const long long idx = slo[o] + (long long)lane * step[o];
-        const bool pred = len > 0 && idx < shi[o] && digit_at(keys[idx], level) < o;
-        ball[o] = __ballot_sync(0xffffffffu, pred);
-      }
-#pragma unroll
-      for (int o = 1; o < 8; o++) {
-        if (slo[o] >= shi[o]) continue;
-        const int t = __popc(ball[o]);
-        if (step[o] == 1) {
-          slo[o] = shi[o] = slo[o] + t;
-        } else if (t == 0) {
-          shi[o] = slo[o];
-        } else {
-          const long long nlo = slo[o] + (long long)(t - 1) * step[o] + 1;
-          const long long nhi = slo[o] + (long long)t * step[o];
-          shi[o] = (int)(nhi < shi[o] ? nhi : shi[o]);
-          slo[o] = (int)nlo;
+struct GridBarrier {
+  unsigned* arrived;  // zero before the launch
+  int* fault;
+  unsigned epoch;
+  // all blocks' writes before it are visible to all blocks after it; false: leave the kernel
+  __device__ __forceinline__ bool sync() {
+    __shared__ int ok;
+    __syncthreads();
+    epoch += gridDim.x;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      atomicAdd(arrived, 1u);
+      int good = 1;
+      for (int spin = 0;; spin++) {
+        unsigned seen;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
+        if (seen >= epoch) break;
+        if (spin == kSyncSpins) {
+          atomicExch(fault, 1);
+          good = 0;
+          break;
         }
       }
+      __threadfence();
+      if (good && *(volatile int*)fault) good = 0;
+      ok = good;
     }
-    if (lane == 0) {
-      st[0] = b;
-      st[8] = b + c;
+    __syncthreads();
+    return ok != 0;
+  }
+};
+
+// control block of k_tree (ints, zero before the launch except where said)
+enum {
+  TC_ARRIVED, TC_FAULT, TC_BIG,  // TC_BIG: a leaf of more than kRankBodies bodies
+  TC_LEAVES,
+  TC_COUNT = 8,       // [l]: nodes of level l (l > 0)
+  TC_FULL = 40,       // [l]: the children of level l did not fit the node arrays
+  TC_DEEP = 72,       // [l]: level l splits on a digit the keys were not sorted by
+  TC_INTS = 104
+};
+
+// largest leaf whose bodies k_tree puts in input order itself
+constexpr int kRankBodies = 128;
+
+template <typename T> struct TreeArgs {
+  const unsigned long long* keys;  // sorted within each root on their first `levels` digits
+  const int* sidx;                 // input index of each sorted key
+  const vec4<T>* bodies_in;
+  const T* box;
+  const int* root_first;
+  int nroots, ncrit, levels, ncap;
+  int rank;   // put the bodies of each leaf in input order (order, bodies)
+  int radii;  // and set the cells' final radii and monopoles (before the error-optimised ones)
+  int use_rmax;
+  T theta;
+  int* ctl;
+  int *nbegin, *ncount, *nparent, *nchildn, *nfirst, *nnode, *npos, *ncb, *nlevel, *nsid;
+  T *nX, *nM0;
+  int* cbase;
+  int *order, *iparent, *ichild, *nchild, *ibody, *nbody, *clevel, *croot, *leaves;
+  vec4<T>* bodies;
+  unsigned long long* icell;
+  int4* info;
+  vec4<T>* cX;
+  T* m0;
+};
+
+// A warp finds the 7 octant boundaries of a node's sorted key range [b, b + c) together by
+// 32-ary searches (32 samples per boundary and round, all loads of a round independent), so
+// a node needs log32(c) dependent rounds instead of the 7 log2(c) of a binary search per
+// boundary.  slo[o]: the first index whose octant digit is >= o.
+__device__ __forceinline__ void octant_starts(int lane, int b, int c, int level,
+                                              const unsigned long long* __restrict__ keys,
+                                              int* slo) {
+  int shi[8];
 #pragma unroll
-      for (int o = 1; o < 8; o++) st[o] = slo[o];
-    }
-    int prev = b;
+  for (int o = 1; o < 8; o++) {
+    slo[o] = b;
+    shi[o] = b + c;
+  }
+  // invariant: the first index whose octant digit is >= o lies in [slo[o], shi[o]]
+  for (;;) {
+    bool open = false;
+#pragma unroll
+    for (int o = 1; o < 8; o++) open |= slo[o] < shi[o];
+    if (!open) break;
+    unsigned ball[8];
+    int step[8];
 #pragma unroll
     for (int o = 1; o < 8; o++) {
-      nch += slo[o] > prev;
-      prev = slo[o];
+      const int len = shi[o] - slo[o];
+      step[o] = len <= 32 ? 1 : (len + 31) / 32;
+      const long long idx = slo[o] + (long long)lane * step[o];
+      const bool pred = len > 0 && idx < shi[o] && digit_at(keys[idx], level) < o;
+      ball[o] = __ballot_sync(0xffffffffu, pred);
     }
-    nch += b + c > prev;
+#pragma unroll
+    for (int o = 1; o < 8; o++) {
+      if (slo[o] >= shi[o]) continue;
+      const int t = __popc(ball[o]);
+      if (step[o] == 1) {
+        slo[o] = shi[o] = slo[o] + t;
+      } else if (t == 0) {
+        shi[o] = slo[o];
+      } else {
+        const long long nlo = slo[o] + (long long)(t - 1) * step[o] + 1;
+        const long long nhi = slo[o] + (long long)t * step[o];
+        shi[o] = (int)(nhi < shi[o] ? nhi : shi[o]);
+        slo[o] = (int)nlo;
+      }
+    }
   }
-  if (lane == 0) cnt[w] = nch;
 }
 
-__global__ void k_split(int lo, int hi, int level, int ncrit,
-                        const unsigned long long* __restrict__ keys,
-                        const int* __restrict__ nbegin, const int* __restrict__ ncount,
-                        int* __restrict__ cnt, int* __restrict__ starts) {
-  const int lane = lane_id();
-  const long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int m = hi - lo;
-  if (w == m && lane == 0) cnt[m] = 0;
-  if (w >= m) return;
-  split_node(lane, (int)w, lo + (int)w, level, ncrit, keys, nbegin, ncount, cnt, starts);
+// The bodies of a leaf of at most 32 K bodies (a warp): their input indices, in key order,
+// ranked and written back ascending (the stable partitions of the reference keep input
+// order), the bodies with them; with radii, the leaf's radius (setRmax, R /= theta) and the
+// sum of its charges in body order, as the P2M kernels form them.
+template <typename T, int K>
+__device__ __forceinline__ void rank_leaf(const TreeArgs<T>& a, int lane, int v, int b0, int n,
+                                          T X0, T X1, T X2, T R) {
+  int id[K], r[K];
+  T rmax = 0;
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    id[k] = lane + 32 * k < n ? a.sidx[b0 + lane + 32 * k] : INT_MAX;
+    r[k] = 0;
+  }
+#pragma unroll
+  for (int q = 0; q < K; q++)
+    for (int i = 0; i < min(32, n - 32 * q); i++) {
+      const int u = __shfl_sync(0xffffffffu, id[q], i);
+#pragma unroll
+      for (int k = 0; k < K; k++) r[k] += u < id[k];
+    }
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    if (lane + 32 * k < n) {
+      const vec4<T> b = a.bodies_in[id[k]];
+      a.order[b0 + r[k]] = id[k];
+      a.bodies[b0 + r[k]] = b;
+      const T d = sqrt_rn(norm_rn(sub_rn(X0, b.x), sub_rn(X1, b.y), sub_rn(X2, b.z)));
+      rmax = d > rmax ? d : rmax;
+    }
+  if (!a.radii) return;
+  __syncwarp();
+  T q = 0;
+  for (int base = 0; base < n; base += 32) {
+    const int cnt = min(32, n - base);
+    const T w = lane < cnt ? a.bodies[b0 + base + lane].w : T(0);
+    for (int i = 0; i < cnt; i++) q = add_rn(q, __shfl_sync(0xffffffffu, w, i));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const T u = __shfl_xor_sync(0xffffffffu, rmax, o);
+    rmax = u > rmax ? u : rmax;
+  }
+  if (lane == 0) {
+    if (a.use_rmax) R = rmax < R ? rmax : R;
+    a.nX[4 * v + 3] = div_rn(R, a.theta);
+    a.nM0[v] = q;
+  }
 }
 
-// k_split with the level's node range read on the device (lvl[level], lvl[level + 1]) for
-// the planned build: a grid-stride loop over the level's nodes.  The counts past them are
-// zero (cnt is cleared before the first level, and k_emit_planned clears the counts it has
-// used), as the scan over mcap + 1 entries that follows needs; a level of more than mcap
-// nodes flags overflow and is not split.
-__global__ void k_split_planned(const int* __restrict__ lvl, int level, int ncrit, int mcap,
-                                const unsigned long long* __restrict__ keys,
-                                const int* __restrict__ nbegin, const int* __restrict__ ncount,
-                                int* __restrict__ cnt, int* __restrict__ starts,
-                                int* __restrict__ overflow) {
-  const int lane = lane_id();
-  const int lo = lvl[level], m = lvl[level + 1] - lo;
-  const int mm = m <= mcap ? m : 0;
-  if (m > mcap && blockIdx.x == 0 && threadIdx.x == 0) atomicExch(overflow, 1);
-  const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
-  for (long long w = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < mm; w += nw)
-    split_node(lane, (int)w, lo + (int)w, level, ncrit, keys, nbegin, ncount, cnt, starts);
-}
-
-// the children of node t of the level (v = lo + t), from hi + coff[t] on
+// One node of BuildNodes (include/build_tree_tbb.h:165-218), a warp: a node with more than
+// ncrit bodies gets one child per non-empty octant, from node `next` on; any other is a leaf.
 template <typename T>
-__device__ __forceinline__ void emit_node(int t, int lo, int hi, int level,
-                                          const int* __restrict__ cnt,
-                                          const int* __restrict__ coff,
-                                          const int* __restrict__ starts,
-                                          const T* __restrict__ box, int* __restrict__ nbegin,
-                                          int* __restrict__ ncount, int* __restrict__ nparent,
-                                          int* __restrict__ nchildn, int* __restrict__ nfirst,
-                                          int* __restrict__ nlevel, int* __restrict__ nsid,
-                                          T* __restrict__ nX) {
-  int v = lo + t;
-  int nch = cnt[t];
-  nchildn[v] = nch;
-  if (nch == 0) {
-    nfirst[v] = -1;
+__device__ __forceinline__ void tree_node(const TreeArgs<T>& a, int lane, int v, int level,
+                                          int next) {
+  const int b = a.nbegin[v], c = a.ncount[v], root = a.nsid[v];
+  const T R0 = a.box[16 * root + 3];
+  const T X0 = a.nX[4 * v], X1 = a.nX[4 * v + 1], X2 = a.nX[4 * v + 2];
+  if (c > a.ncrit && level < kMaxLevel) {
+    if (level >= a.levels) {
+      if (lane == 0) atomicExch(&a.ctl[TC_DEEP + level], 1);
+      return;
+    }
+    int slo[8];
+    octant_starts(lane, b, c, level, a.keys, slo);
+    int s = b, e = b + c;  // the range of octant `lane`
+#pragma unroll
+    for (int o = 1; o < 8; o++) {
+      if (lane == o) s = slo[o];
+      if (lane == o - 1) e = slo[o];
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, lane < 8 && e > s);
+    const int nch = __popc(m);
+    int first = 0;
+    if (lane == 0) first = next + atomicAdd(&a.ctl[TC_COUNT + level + 1], nch);
+    first = __shfl_sync(0xffffffffu, first, 0);
+    if (first + nch > a.ncap) {
+      if (lane == 0) atomicExch(&a.ctl[TC_FULL + level], 1);
+      return;
+    }
+    if (m >> lane & 1) {
+      const int u = first + __popc(m & ((1u << lane) - 1));
+      const T r = div_rn(R0, (T)(1 << (level + 1)));
+      a.nbegin[u] = s;
+      a.ncount[u] = e - s;
+      a.nparent[u] = v;
+      a.nlevel[u] = level + 1;
+      a.nsid[u] = root;
+      a.nX[4 * u] = add_rn(X0, (lane & 1) ? r : -r);
+      a.nX[4 * u + 1] = add_rn(X1, (lane & 2) ? r : -r);
+      a.nX[4 * u + 2] = add_rn(X2, (lane & 4) ? r : -r);
+    }
+    if (lane == 0) {
+      a.nchildn[v] = nch;
+      a.nfirst[v] = first;
+    }
     return;
   }
-  int first = hi + coff[t];
-  nfirst[v] = first;
-  const int* st = starts + 9 * t;
-  const int root = nsid[v];
-  T r = div_rn(box[16 * root + 3], (T)(1 << (level + 1)));
-  T X0 = nX[4 * v], X1 = nX[4 * v + 1], X2 = nX[4 * v + 2];
-  int k = 0;
-  for (int o = 0; o < 8; o++) {
-    if (st[o + 1] <= st[o]) continue;
-    int u = first + k++;
-    nbegin[u] = st[o];
-    ncount[u] = st[o + 1] - st[o];
-    nparent[u] = v;
-    nlevel[u] = level + 1;
-    nsid[u] = root;
-    nX[4 * u] = add_rn(X0, (o & 1) ? r : -r);
-    nX[4 * u + 1] = add_rn(X1, (o & 2) ? r : -r);
-    nX[4 * u + 2] = add_rn(X2, (o & 4) ? r : -r);
-    nX[4 * u + 3] = 0;
+  if (lane == 0) {
+    a.nchildn[v] = 0;
+    a.nfirst[v] = -1;
+    a.nnode[v] = 1;
   }
+  if (!a.rank) return;
+  const T R = div_rn(R0, (T)(1 << level));
+  if (c <= 64) rank_leaf<T, 2>(a, lane, v, b, c, X0, X1, X2, R);
+  else if (c <= kRankBodies) rank_leaf<T, kRankBodies / 32>(a, lane, v, b, c, X0, X1, X2, R);
+  else if (lane == 0) atomicExch(&a.ctl[TC_BIG], 1);
 }
 
-template <typename T>
-__global__ void k_emit(int lo, int hi, int level, const int* __restrict__ cnt,
-                       const int* __restrict__ coff, const int* __restrict__ starts,
-                       const T* __restrict__ box, int* __restrict__ nbegin,
-                       int* __restrict__ ncount, int* __restrict__ nparent,
-                       int* __restrict__ nchildn, int* __restrict__ nfirst,
-                       int* __restrict__ nlevel, int* __restrict__ nsid, T* __restrict__ nX) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= hi - lo) return;
-  emit_node<T>(t, lo, hi, level, cnt, coff, starts, box, nbegin, ncount, nparent, nchildn,
-               nfirst, nlevel, nsid, nX);
-}
-
-// k_emit of the planned build: the level's range and its child total (coff[m]) read on the
-// device; the next level's end is written to lvl[level + 2]; children that would not fit
-// the node arrays (ncap) flag overflow and are not emitted.
-template <typename T>
-__global__ void k_emit_planned(int* __restrict__ lvl, int level, int ncap,
-                               int* __restrict__ cnt, const int* __restrict__ coff,
-                               const int* __restrict__ starts, const T* __restrict__ box,
-                               int* __restrict__ nbegin, int* __restrict__ ncount,
-                               int* __restrict__ nparent, int* __restrict__ nchildn,
-                               int* __restrict__ nfirst, int* __restrict__ nlevel,
-                               int* __restrict__ nsid, T* __restrict__ nX,
-                               int* __restrict__ overflow) {
-  const int lo = lvl[level], hi = lvl[level + 1], m = hi - lo;
-  const int total = m > 0 ? coff[m] : 0;
-  const bool fits = (long long)hi + total <= ncap && *overflow == 0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    lvl[level + 2] = fits ? hi + total : hi;
-    if (!fits) atomicExch(overflow, 1);
-  }
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
-    if (fits)
-      emit_node<T>(t, lo, hi, level, cnt, coff, starts, box, nbegin, ncount, nparent, nchildn,
-                   nfirst, nlevel, nsid, nX);
-    if (t < ncap) cnt[t] = 0;  // cleared for the next level's scan
-  }
-}
-
-// leaf nodes: chain-less nodes at the deepest level of the last pass
-__global__ void k_finish_level(int lo, int hi, int* nchildn, int* nfirst) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= hi - lo) return;
-  nchildn[lo + t] = 0;
-  nfirst[lo + t] = -1;
-}
-
-// NNODE bottom-up (include/build_tree_tbb.h:215-217)
-__global__ void k_nnode(int lo, int hi, const int* __restrict__ nchildn,
-                        const int* __restrict__ nfirst, int* __restrict__ nnode) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= hi - lo) return;
-  int v = lo + t;
-  int s = 1;
-  for (int k = 0; k < nchildn[v]; k++) s += nnode[nfirst[v] + k];
-  nnode[v] = s;
-}
-
-// Cell slots top-down (Nodes2cells, include/build_tree_tbb.h:272-286): children at CN,
-// next free slot after the child block, each child's subtree after the previous child's.
-__global__ void k_pos(int lo, int hi, const int* __restrict__ nchildn,
-                      const int* __restrict__ nfirst, const int* __restrict__ nnode,
-                      const int* __restrict__ cbase, int* __restrict__ npos,
-                      int* __restrict__ ncb) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= hi - lo) return;
-  int v = lo + t;
-  if (lo == 0) {  // roots: each root's cells start after the previous root's subtree
-    npos[v] = cbase[v];
-    ncb[v] = cbase[v] + 1;
-  }
-  int nch = nchildn[v];
+// The subtree size (NNODE, include/build_tree_tbb.h:215-217) of a split node, and with radii
+// its radius and monopole from its children's (include/up_down_pass.h:60-84).
+template <typename T> __device__ __forceinline__ void tree_up(const TreeArgs<T>& a, int v, int level) {
+  const int nch = a.nchildn[v];
   if (nch == 0) return;
-  int cb = ncb[v];
+  const int u0 = a.nfirst[v];
+  int size = 1;
+  T rr = 0, q = 0;
+  const T X0 = a.nX[4 * v], X1 = a.nX[4 * v + 1], X2 = a.nX[4 * v + 2];
+  for (int u = u0; u < u0 + nch; u++) {
+    size += a.nnode[u];
+    if (!a.radii) continue;
+    const T d = add_rn(sqrt_rn(norm_rn(sub_rn(X0, a.nX[4 * u]), sub_rn(X1, a.nX[4 * u + 1]),
+                                       sub_rn(X2, a.nX[4 * u + 2]))),
+                       a.nX[4 * u + 3]);
+    rr = d > rr ? d : rr;
+    q = add_rn(q, a.nM0[u]);
+  }
+  a.nnode[v] = size;
+  if (a.radii) {
+    T R = div_rn(a.box[16 * a.nsid[v] + 3], (T)(1 << level));
+    if (a.use_rmax) R = rr < R ? rr : R;
+    a.nX[4 * v + 3] = div_rn(R, a.theta);
+    a.nM0[v] = q;
+  }
+}
+
+// The cell of node v, and its children's slots: Nodes2cells (include/build_tree_tbb.h:250-294:
+// children at CN, the next free slot after the child block, each child's subtree after the
+// previous child's) with the Morton index of getKey (:240-249) in 64-bit arithmetic.
+template <typename T>
+__device__ __forceinline__ void tree_cell(const TreeArgs<T>& a, int v, int level) {
+  const int root = a.nsid[v];
+  const int rc = a.nroots == 1 ? 0 : a.cbase[root];
+  const int c = level == 0 ? rc : a.npos[v], cb = level == 0 ? rc + 1 : a.ncb[v];
+  const int nch = a.nchildn[v], u0 = a.nfirst[v], par = a.nparent[v];
+  if (level == 0) a.npos[v] = c;
   int acc = cb + nch;
   for (int k = 0; k < nch; k++) {
-    int u = nfirst[v] + k;
-    npos[u] = cb + k;
-    ncb[u] = acc;
-    acc += nnode[u] - 1;
+    a.npos[u0 + k] = cb + k;
+    a.ncb[u0 + k] = acc;
+    acc += a.nnode[u0 + k] - 1;
+  }
+  const T* box = a.box + 16 * root;
+  const T R0 = box[3], R = div_rn(R0, (T)(1 << level));
+  const T X[3] = {a.nX[4 * v], a.nX[4 * v + 1], a.nX[4 * v + 2]};
+  const int b = a.nbegin[v], nb = a.ncount[v], ch = nch ? cb : 0;
+  a.croot[c] = rc;
+  a.iparent[c] = level == 0 ? c : a.npos[par];
+  a.nchild[c] = nch;
+  a.ichild[c] = ch;
+  a.ibody[c] = b;
+  a.nbody[c] = nb;
+  a.clevel[c] = level;
+  a.info[c] = make_int4(nch, ch, nb, b);
+  const T diam = mul_rn((T)2, R);
+  int iX[3];
+  for (int d = 0; d < 3; d++) iX[d] = (int)div_rn(sub_rn(X[d], sub_rn(box[d], R0)), diam);
+  unsigned long long index = ((1ULL << (3 * level)) - 1) / 7;
+  for (int l = 0; l < level; l++)
+    for (int d = 0; d < 3; d++) {
+      index += (unsigned long long)(iX[d] & 1) << (3 * l + d);
+      iX[d] >>= 1;
+    }
+  a.icell[c] = index;
+  a.cX[c] = make_v4<T>(X[0], X[1], X[2], a.radii ? a.nX[4 * v + 3] : R);
+  if (a.radii) a.m0[c] = a.nM0[v];
+}
+
+constexpr int kTreeThreads = 256, kTreeBlocks = 3;  // threads of a block, blocks per SM
+
+template <typename T>
+__global__ void __launch_bounds__(kTreeThreads, kTreeBlocks) k_tree(TreeArgs<T> a) {
+  GridBarrier bar{(unsigned*)&a.ctl[TC_ARRIVED], &a.ctl[TC_FAULT], 0};
+  __shared__ int lv[kMaxLevel + 3];
+  const int lane = lane_id();
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  // one root node per non-empty solve, in solve order
+  for (int r = tid; r < a.nroots; r += nt) {
+    a.nbegin[r] = a.root_first[r];
+    a.ncount[r] = a.root_first[r + 1] - a.root_first[r];
+    a.nparent[r] = -1;
+    a.nlevel[r] = 0;
+    a.nsid[r] = r;
+    for (int d = 0; d < 3; d++) a.nX[4 * r + d] = a.box[16 * r + d];
+  }
+  if (!bar.sync()) return;
+  int lo = 0, hi = a.nroots, level = 0;
+  for (;; level++) {
+    if (threadIdx.x == 0) lv[level] = lo;
+    for (int v = lo + (tid >> 5); v < hi; v += nt >> 5) tree_node(a, lane, v, level, hi);
+    if (!bar.sync()) return;
+    // (flags and counts of this level: no block writes them any more)
+    if (*(volatile int*)&a.ctl[TC_FULL + level] || *(volatile int*)&a.ctl[TC_DEEP + level]) return;
+    const int cnt = *(volatile int*)&a.ctl[TC_COUNT + level + 1];
+    if (cnt == 0) break;
+    lo = hi;
+    hi += cnt;
+  }
+  if (threadIdx.x == 0) lv[level + 1] = hi;
+  __syncthreads();
+  for (int l = level - 1; l >= 0; l--) {
+    for (int v = lv[l] + tid; v < lv[l + 1]; v += nt) tree_up(a, v, l);
+    if (!bar.sync()) return;
+  }
+  if (a.nroots > 1) {  // first cell of each root: exclusive scan of the roots' subtree sizes
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+      int run = 0;
+      for (int r0 = 0; r0 < a.nroots; r0 += 32) {
+        const int n = r0 + lane < a.nroots ? a.nnode[r0 + lane] : 0;
+        int incl = n;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, incl, d);
+          if (lane >= d) incl += u;
+        }
+        if (r0 + lane < a.nroots) a.cbase[r0 + lane] = run + incl - n;
+        run += __shfl_sync(0xffffffffu, incl, 31);
+      }
+    }
+    if (!bar.sync()) return;
+  } else if (tid == 0) {
+    a.cbase[0] = 0;
+  }
+  for (int l = 0; l <= level; l++) {
+    // (a warp's leaves take one atomic; their order does not matter to any result)
+    for (int v0 = lv[l] + tid - lane; v0 < lv[l + 1]; v0 += nt) {
+      const int v = v0 + lane;
+      const bool in = v < lv[l + 1];
+      if (in) tree_cell(a, v, l);
+      const unsigned m = __ballot_sync(0xffffffffu, in && a.nchildn[in ? v : 0] == 0);
+      int at = 0;
+      if (lane == 0 && m) at = atomicAdd(&a.ctl[TC_LEAVES], __popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (m >> lane & 1) a.leaves[at + __popc(m & ((1u << lane) - 1))] = a.npos[v];
+    }
+    if (l < level && !bar.sync()) return;
   }
 }
 
@@ -424,45 +561,6 @@ void fill_cell_info(SolverBase& s) {
   k_cell_info<<<ceil_div(s.ncells, 256), 256, 0, s.stream>>>(
       s.ncells, s.c_nchild.p, s.c_ichild.p, s.c_nbody.p, s.c_ibody.p, s.c_info.p);
   FMM_LAUNCH_CHECK();
-}
-
-// Cell records (Nodes2cells::operator(), include/build_tree_tbb.h:250-262) with the
-// Morton index of getKey (:240-249) in 64-bit arithmetic.
-template <typename T>
-__global__ void k_cells(int nnodes, const T* __restrict__ boxes, const int* __restrict__ nbegin,
-                        const int* __restrict__ ncount, const int* __restrict__ nparent,
-                        const int* __restrict__ nchildn, const int* __restrict__ nlevel,
-                        const int* __restrict__ nsid, const int* __restrict__ cbase,
-                        const int* __restrict__ npos, const int* __restrict__ ncb,
-                        const T* __restrict__ nX, int* iparent, int* ichild, int* nchild,
-                        int* ibody, int* nbody, int* clevel, unsigned long long* icell,
-                        vec4<T>* cX, int* croot) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= nnodes) return;
-  int c = npos[v];
-  int lev = nlevel[v];
-  const T* box = boxes + 16 * nsid[v];
-  croot[c] = cbase[nsid[v]];
-  T R0 = box[3];
-  T R = div_rn(R0, (T)(1 << lev));
-  T X[3] = {nX[4 * v], nX[4 * v + 1], nX[4 * v + 2]};
-  iparent[c] = nparent[v] < 0 ? c : npos[nparent[v]];
-  int nch = nchildn[v];
-  nchild[c] = nch;
-  ichild[c] = nch ? ncb[v] : 0;
-  ibody[c] = nbegin[v];
-  nbody[c] = ncount[v];
-  clevel[c] = lev;
-  T diam = mul_rn((T)2, R);
-  int iX[3];
-  for (int d = 0; d < 3; d++) iX[d] = (int)div_rn(sub_rn(X[d], sub_rn(box[d], R0)), diam);
-  unsigned long long index = ((1ULL << (3 * lev)) - 1) / 7;
-  for (int l = 0; l < lev; l++) {
-    for (int d = 0; d < 3; d++) index += (unsigned long long)(iX[d] & 1) << (3 * l + d);
-    for (int d = 0; d < 3; d++) iX[d] >>= 1;
-  }
-  icell[c] = index;
-  cX[c] = make_v4<T>(X[0], X[1], X[2], R);
 }
 
 // leaf level of every sorted body (leaves only; ranges partition the bodies)
@@ -487,56 +585,11 @@ __global__ void k_tkey(int n, const unsigned long long* __restrict__ skeys,
   iota[b] = b;
 }
 
-// Input order inside every leaf of at most 64 bodies (warp per leaf node): the bodies'
-// original indices, currently in full-key order, are ranked and written back ascending.
-__global__ void k_leaf_reorder(int nnodes, const int* __restrict__ nchildn,
-                               const int* __restrict__ nbegin, const int* __restrict__ ncount,
-                               const int* __restrict__ sidx, int* __restrict__ order) {
-  const int v = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = lane_id();
-  if (v >= nnodes || nchildn[v] != 0) return;
-  const int b0 = nbegin[v], n = ncount[v];
-  const int a = lane < n ? sidx[b0 + lane] : 0x7fffffff;
-  const int b = lane + 32 < n ? sidx[b0 + 32 + lane] : 0x7fffffff;
-  int ra = 0, rb = 0;
-  for (int k = 0; k < n; k++) {
-    const int u = k < 32 ? __shfl_sync(0xffffffffu, a, k) : __shfl_sync(0xffffffffu, b, k - 32);
-    ra += u < a;
-    rb += u < b;
-  }
-  if (lane < n) order[b0 + ra] = a;
-  if (lane + 32 < n) order[b0 + rb] = b;
-}
-
 template <typename T>
 __global__ void k_permute(int n, const vec4<T>* __restrict__ in, const int* __restrict__ order,
                           vec4<T>* __restrict__ out) {
   int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < n) out[b] = in[order[b]];
-}
-
-__global__ void k_leaf_flags(int nnodes, const int* __restrict__ nchildn, int* __restrict__ f) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v < nnodes) f[v] = nchildn[v] == 0;
-  if (v == nnodes) f[v] = 0;
-}
-
-__global__ void k_leaf_scatter(int nnodes, const int* __restrict__ nchildn,
-                               const int* __restrict__ off, const int* __restrict__ npos,
-                               int* __restrict__ leaves) {
-  int v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v < nnodes && nchildn[v] == 0) leaves[off[v]] = npos[v];
-}
-
-// grow a node array keeping its contents (the old buffer is retired, as DevArr::ensure does)
-template <typename U> static void grow(SolverBase& s, DevArr<U>& a, size_t n) {
-  if (n <= a.cap) return;
-  DevArr<U> b;
-  b.ensure(n > 2 * a.cap ? n : 2 * a.cap);
-  if (a.p) FMM_CUDA(cudaMemcpyAsync(b.p, a.p, a.cap * sizeof(U), cudaMemcpyDeviceToDevice, s.stream));
-  FMM_CUDA(cudaStreamSynchronize(s.stream));
-  retire_into(a, b);
-  a = std::move(b);
 }
 
 // Sort (key, body) pairs by (root, key), stable: one radix sort on the key over all roots,
@@ -559,7 +612,7 @@ static void forest_sort(Solver<T>& s, const unsigned long long* kin, unsigned lo
   s.fs_pos.ensure(n);
   s.fs_pos2.ensure(n);
   sort_pairs_u64(s, kin, s.fs_keys.p, vin, s.fs_idx.p, n, end_bit, begin_bit);
-  k_root_of<<<ceil_div(n, TB), TB, 0, s.stream>>>(n, s.fs_idx.p, s.d_root_first.p, nroots,
+  k_root_of<<<ceil_div(n, TB), TB, 0, s.stream>>>(n, s.fs_idx.p, s.root_first, nroots,
                                                   s.fs_root.p, s.fs_pos.p);
   FMM_LAUNCH_CHECK();
   int bits = 1;
@@ -568,57 +621,6 @@ static void forest_sort(Solver<T>& s, const unsigned long long* kin, unsigned lo
   k_gather_kv<<<ceil_div(n, TB), TB, 0, s.stream>>>(n, s.fs_pos2.p, s.fs_keys.p, s.fs_idx.p,
                                                     kout, vout);
   FMM_LAUNCH_CHECK();
-}
-
-// The levels of the node build without a host round trip per level, for a handle whose
-// previous tree had s.tree_plan levels: tree_plan + 1 levels of k_split_planned, a scan of
-// the counts and k_emit_planned run back to back with the level ranges kept on the device,
-// then one read of the ranges.  Returns false (and the levels are built again level by
-// level) if the node arrays overflowed or the tree went deeper than planned.
-template <typename T>
-static bool planned_levels(Solver<T>& s, int nroots, DevArr<int>** narr, int nnarr) {
-  const int TB = 256;
-  const int L = s.tree_plan + 1;
-  size_t cap = s.nX.cap / 4;
-  for (int i = 0; i < nnarr; i++) cap = std::min(cap, narr[i]->cap);
-  const int ncap = (int)std::min<size_t>(cap, INT_MAX / 16);
-  const int mcap = ncap;  // a level holds no more nodes than the arrays
-  s.nsplit.ensure(9 * (size_t)(mcap + 1));
-  s.coff.ensure((size_t)mcap + 2);
-  s.idx.ensure(std::max((size_t)s.n, (size_t)mcap + 1));
-  s.d_lvl.ensure(L + 2);
-  int* cnt = s.idx.p;
-  int* lvl = s.d_lvl.p;
-  int* ovf = (int*)((unsigned long long*)s.scal.p + 6);
-  int* hl = s.scal_host + 400;  // pinned: L + 2 level ends, then the overflow flag
-  if (L + 3 > 512 - 400) return false;
-  hl[0] = 0;
-  hl[1] = nroots;
-  FMM_CUDA(cudaMemcpyAsync(lvl, hl, 2 * sizeof(int), cudaMemcpyHostToDevice, s.stream));
-  FMM_CUDA(cudaMemsetAsync(ovf, 0, sizeof(int), s.stream));
-  FMM_CUDA(cudaMemsetAsync(cnt, 0, ((size_t)mcap + 1) * sizeof(int), s.stream));
-  const int gs = (int)std::min<long long>(ceil_div(32LL * (mcap + 1), TB), 148 * 16);
-  const int ge = (int)std::min<long long>(ceil_div((long long)mcap, TB), 148 * 8);
-  for (int level = 0; level < L; level++) {
-    k_split_planned<<<gs, TB, 0, s.stream>>>(lvl, level, s.cfg.ncrit, mcap, s.keys2.p,
-                                              s.nbegin.p, s.ncount.p, cnt, s.nsplit.p, ovf);
-    FMM_LAUNCH_CHECK();
-    exclusive_sum_int(s, cnt, s.coff.p, mcap + 1);
-    k_emit_planned<T><<<ge, TB, 0, s.stream>>>(lvl, level, ncap, cnt, s.coff.p, s.nsplit.p,
-                                               s.box.p, s.nbegin.p, s.ncount.p, s.nparent.p,
-                                               s.nchildn.p, s.nfirst.p, s.nlevel.p, s.nsid.p,
-                                               s.nX.p, ovf);
-    FMM_LAUNCH_CHECK();
-  }
-  FMM_CUDA(cudaMemcpyAsync(hl, lvl, (L + 2) * sizeof(int), cudaMemcpyDeviceToHost, s.stream));
-  FMM_CUDA(cudaMemcpyAsync(hl + L + 2, ovf, sizeof(int), cudaMemcpyDeviceToHost, s.stream));
-  FMM_CUDA(cudaStreamSynchronize(s.stream));
-  if (hl[L + 2] != 0 || hl[L + 1] != hl[L]) return false;
-  // levels 0 .. d, d the first level without children
-  int d = 0;
-  while (hl[d + 2] != hl[d + 1]) d++;
-  s.level_lo.assign(hl, hl + d + 2);
-  return true;
 }
 
 // ---------------------------------------------------------------- uniform Morton tree
@@ -850,11 +852,12 @@ template <typename T> static void build_uniform(Solver<T>& s) {
   s.tree_plan = 0;
 }
 
-template <typename T> void build_tree(Solver<T>& s) {
+template <typename T> void build_tree(Solver<T>& s, bool radii) {
   const int n = s.n;
   const int TB = 256;
   s.kc_valid = false;  // the host copies of the cells' index fields are stale
   s.p2p_ordered = false;  // so is the P2P target order of the last traversal
+  s.radii_set = false;
   s.level_lo.clear();
   s.ncells = s.maxlevel = s.nleaves = 0;
   // roots: non-empty solves in order
@@ -879,28 +882,38 @@ template <typename T> void build_tree(Solver<T>& s) {
     s.root_cell.clear();
     return;
   }
-  // bounds per root over chunks of at most 4096 bodies (256 blocks at 2^20 bodies)
+  // bounds per root over chunks of at most 4096 bodies (256 blocks at 2^20 bodies); the
+  // roots' first bodies, the chunks' ranges and the roots' first chunks in one upload from
+  // pinned memory (the last solve's was waited for when its tree was read back)
   const int CH = 4096;
-  std::vector<int> hb, he, hlo{0};
-  for (int r = 0; r < nroots; r++) {
-    for (int b0 = rfirst[r]; b0 < rfirst[r + 1]; b0 += CH) {
-      hb.push_back(b0);
-      he.push_back(std::min(b0 + CH, rfirst[r + 1]));
-    }
-    hlo.push_back((int)hb.size());
+  int nch = 0;
+  for (int r = 0; r < nroots; r++) nch += ceil_div(rfirst[r + 1] - rfirst[r], CH);
+  const size_t up = 2 * (size_t)(nroots + 1) + 2 * (size_t)nch;
+  s.d_seg.ensure(up);
+  if (up > s.seg_host_cap) {
+    if (s.seg_host) s.roots_retired.push_back((int2*)s.seg_host);
+    s.seg_host = nullptr;
+    s.seg_host_cap = 0;
+    FMM_CUDA(cudaMallocHost((void**)&s.seg_host, 2 * up * sizeof(int)));
+    s.seg_host_cap = 2 * up;
   }
-  const int nch = (int)hb.size();
-  s.d_root_first.ensure(nroots + 1);
-  s.d_seg.ensure(2 * (size_t)nch + nroots + 1);
-  int* dcb = s.d_seg.p;
-  int* dce = dcb + nch;
-  int* dlo = dce + nch;
-  FMM_CUDA(cudaMemcpyAsync(s.d_root_first.p, rfirst.data(), sizeof(int) * (nroots + 1),
-                           cudaMemcpyHostToDevice, s.stream));
-  FMM_CUDA(cudaMemcpyAsync(dcb, hb.data(), sizeof(int) * nch, cudaMemcpyHostToDevice, s.stream));
-  FMM_CUDA(cudaMemcpyAsync(dce, he.data(), sizeof(int) * nch, cudaMemcpyHostToDevice, s.stream));
-  FMM_CUDA(cudaMemcpyAsync(dlo, hlo.data(), sizeof(int) * (nroots + 1), cudaMemcpyHostToDevice,
+  {
+    int *hr = s.seg_host, *hlo = hr + nroots + 1, *hb = hlo + nroots + 1, *he = hb + nch;
+    std::copy(rfirst.begin(), rfirst.end(), hr);
+    int k = 0;
+    for (int r = 0; r < nroots; r++) {
+      hlo[r] = k;
+      for (int b0 = rfirst[r]; b0 < rfirst[r + 1]; b0 += CH, k++) {
+        hb[k] = b0;
+        he[k] = std::min(b0 + CH, rfirst[r + 1]);
+      }
+    }
+    hlo[nroots] = k;
+  }
+  FMM_CUDA(cudaMemcpyAsync(s.d_seg.p, s.seg_host, up * sizeof(int), cudaMemcpyHostToDevice,
                            s.stream));
+  s.root_first = s.d_seg.p;
+  const int *dlo = s.root_first + nroots + 1, *dcb = dlo + nroots + 1, *dce = dcb + nch;
   s.minmax_part.ensure(6 * (size_t)nch);
   k_minmax_chunks<T><<<nch, TB, 0, s.stream>>>(s.bodies_in.p, dcb, dce, s.minmax_part.p);
   FMM_LAUNCH_CHECK();
@@ -913,155 +926,126 @@ template <typename T> void build_tree(Solver<T>& s) {
     build_uniform(s);
     return;
   }
-  // keys and first sort (within each root's range)
   s.keys.ensure(n);
   s.keys2.ensure(n);
   s.idx.ensure(n);
   s.idx2.ensure(n);
+  s.order.ensure(n);
+  s.bodies.ensure(n);
+  s.cbase.ensure(nroots + 1);
+  s.tree_ctl.ensure(TC_INTS);
+  const bool rank = s.cfg.ncrit <= kRankBodies;
   // With a plan of L levels to split, the keys are sorted on their top L digits only: the
   // splits read no deeper digit, and the bodies of a leaf are put in input order afterwards
-  // whatever the order of their deeper digits.  If the plan fails, they are sorted again on
-  // every digit for the level-by-level build.
-  const int plan_levels = s.tree_plan > 0 ? s.tree_plan + 1 : kMaxLevel;
-  const int begin_bit = plan_levels < kMaxLevel ? 3 * (kMaxLevel - plan_levels) : 0;
-  k_keys<T><<<ceil_div(n, TB), TB, 0, s.stream>>>(s.bodies_in.p, n, s.box.p, s.d_root_first.p,
-                                                  nroots, s.keys.p, s.idx.p);
-  FMM_LAUNCH_CHECK();
-  forest_sort(s, s.keys.p, s.keys2.p, s.idx.p, s.idx2.p, n, nroots, 3 * kMaxLevel, begin_bit);
-  // nodes, level by level
-  size_t cap0 = (size_t)std::max(1024, 4 * (n / std::max(1, s.cfg.ncrit)) + 64 + nroots);
-  DevArr<int>* narr[] = {&s.nbegin, &s.ncount, &s.nparent, &s.nchildn, &s.nfirst,
-                         &s.nnode, &s.npos, &s.ncb, &s.nlevel, &s.nsid};
-  for (auto* a : narr) a->ensure(cap0);
-  s.nX.ensure(4 * cap0);
-  k_roots<T><<<ceil_div(nroots, TB), TB, 0, s.stream>>>(nroots, s.d_root_first.p, s.box.p,
-                                                        s.nbegin.p, s.ncount.p, s.nparent.p,
-                                                        s.nlevel.p, s.nsid.p, s.nX.p);
-  FMM_LAUNCH_CHECK();
-  s.level_lo.push_back(0);
-  s.level_lo.push_back(nroots);
-  const bool planned = s.tree_plan > 0 && planned_levels(s, nroots, narr, sizeof(narr) / sizeof(*narr));
-  if (!planned && begin_bit > 0) {
-    k_keys<T><<<ceil_div(n, TB), TB, 0, s.stream>>>(s.bodies_in.p, n, s.box.p,
-                                                    s.d_root_first.p, nroots, s.keys.p, s.idx.p);
-    FMM_LAUNCH_CHECK();
-    forest_sort(s, s.keys.p, s.keys2.p, s.idx.p, s.idx2.p, n, nroots, 3 * kMaxLevel);
-    k_roots<T><<<ceil_div(nroots, TB), TB, 0, s.stream>>>(nroots, s.d_root_first.p, s.box.p,
-                                                          s.nbegin.p, s.ncount.p, s.nparent.p,
-                                                          s.nlevel.p, s.nsid.p, s.nX.p);
-    FMM_LAUNCH_CHECK();
-    s.level_lo.assign({0, nroots});
-  }
-  for (int level = 0; !planned; level++) {
-    int lo = s.level_lo[level], hi = s.level_lo[level + 1];
-    int m = hi - lo;
-    s.nsplit.ensure(9 * (size_t)m);
-    s.coff.ensure(m + 1);
-    s.idx.ensure(std::max((size_t)n, (size_t)m + 1));
-    int* cnt = s.idx.p;  // the input-order index array is free until the second sort
-    k_split<<<ceil_div(32LL * (m + 1), TB), TB, 0, s.stream>>>(lo, hi, level, s.cfg.ncrit, s.keys2.p,
-                                                       s.nbegin.p, s.ncount.p, cnt, s.nsplit.p);
-    FMM_LAUNCH_CHECK();
-    exclusive_sum_int(s, cnt, s.coff.p, m + 1);
-    FMM_CUDA(cudaMemcpyAsync(s.scal_host, s.coff.p + m, sizeof(int), cudaMemcpyDeviceToHost,
-                             s.stream));
-    FMM_CUDA(cudaStreamSynchronize(s.stream));
-    int total = s.scal_host[0];
-    if (total == 0) {
-      k_finish_level<<<ceil_div(m, TB), TB, 0, s.stream>>>(lo, hi, s.nchildn.p, s.nfirst.p);
+  // whatever the order of their deeper digits.  A tree that turns out deeper is built again
+  // with the keys sorted on every digit.
+  int levels = s.tree_plan > 0 && rank ? std::min(s.tree_plan + 1, kMaxLevel) : kMaxLevel;
+  size_t cap = (size_t)std::max(1024, 4 * (n / std::max(1, s.cfg.ncrit)) + 64 + nroots);
+  int* hc = s.scal_host + kTreeHost;
+  bool sorted = false;
+  for (;;) {
+    if (!sorted) {
+      k_keys<T><<<ceil_div(n, TB), TB, 0, s.stream>>>(s.bodies_in.p, n, s.box.p, s.root_first,
+                                                      nroots, s.keys.p, s.idx.p);
       FMM_LAUNCH_CHECK();
-      break;
+      forest_sort(s, s.keys.p, s.keys2.p, s.idx.p, s.idx2.p, n, nroots, 3 * kMaxLevel,
+                  3 * (kMaxLevel - levels));
+      sorted = true;
     }
-    size_t need = (size_t)hi + total;
-    for (auto* a : narr) grow(s, *a, need);
-    grow(s, s.nX, 4 * need);
-    k_emit<T><<<ceil_div(m, TB), TB, 0, s.stream>>>(lo, hi, level, cnt, s.coff.p, s.nsplit.p,
-                                                    s.box.p, s.nbegin.p, s.ncount.p,
-                                                    s.nparent.p, s.nchildn.p, s.nfirst.p,
-                                                    s.nlevel.p, s.nsid.p, s.nX.p);
+    DevArr<int>* narr[] = {&s.nbegin, &s.ncount, &s.nparent, &s.nchildn, &s.nfirst, &s.nnode,
+                           &s.npos, &s.ncb, &s.nlevel, &s.nsid, &s.c_iparent, &s.c_ichild,
+                           &s.c_nchild, &s.c_ibody, &s.c_nbody, &s.c_level, &s.c_root, &s.leaves};
+    size_t ncap = (size_t)INT_MAX / 16;
+    for (auto* q : narr) {
+      q->ensure(cap);
+      ncap = std::min(ncap, q->cap);
+    }
+    s.nX.ensure(4 * cap);
+    s.nM0.ensure(cap);
+    s.m0.ensure(cap);
+    s.c_icell.ensure(cap);
+    s.c_info.ensure(cap);
+    s.cX.ensure(cap);
+    ncap = std::min({ncap, s.nX.cap / 4, s.nM0.cap, s.m0.cap, s.c_icell.cap, s.c_info.cap, s.cX.cap});
+    TreeArgs<T> t{};
+    t.keys = s.keys2.p;
+    t.sidx = s.idx2.p;
+    t.bodies_in = s.bodies_in.p;
+    t.box = s.box.p;
+    t.root_first = s.root_first;
+    t.nroots = nroots;
+    t.ncrit = s.cfg.ncrit;
+    t.levels = levels;
+    t.ncap = (int)ncap;
+    t.rank = rank;
+    t.radii = rank && radii;
+    t.use_rmax = s.cfg.use_rmax;
+    t.theta = (T)s.cfg.theta;
+    t.ctl = s.tree_ctl.p;
+    t.nbegin = s.nbegin.p, t.ncount = s.ncount.p, t.nparent = s.nparent.p;
+    t.nchildn = s.nchildn.p, t.nfirst = s.nfirst.p, t.nnode = s.nnode.p, t.npos = s.npos.p;
+    t.ncb = s.ncb.p, t.nlevel = s.nlevel.p, t.nsid = s.nsid.p, t.nX = s.nX.p, t.nM0 = s.nM0.p;
+    t.cbase = s.cbase.p, t.order = s.order.p, t.iparent = s.c_iparent.p, t.ichild = s.c_ichild.p;
+    t.nchild = s.c_nchild.p, t.ibody = s.c_ibody.p, t.nbody = s.c_nbody.p;
+    t.clevel = s.c_level.p, t.croot = s.c_root.p, t.leaves = s.leaves.p, t.bodies = s.bodies.p;
+    t.icell = s.c_icell.p, t.info = s.c_info.p, t.cX = s.cX.p, t.m0 = s.m0.p;
+    // a warp for every few nodes of the widest level: fewer blocks make cheaper barriers
+    const int blocks = std::max(1, std::min(kTreeBlocks * 148, ceil_div(n, 4 * s.cfg.ncrit)));
+    FMM_CUDA(cudaMemsetAsync(s.tree_ctl.p, 0, TC_INTS * sizeof(int), s.stream));
+    void* args[] = {&t};
+    FMM_CUDA(cudaLaunchCooperativeKernel((const void*)k_tree<T>, dim3(blocks), dim3(kTreeThreads),
+                                         args, 0, s.stream));
     FMM_LAUNCH_CHECK();
-    s.level_lo.push_back(hi + total);
+    FMM_CUDA(cudaMemcpyAsync(hc, s.tree_ctl.p, TC_INTS * sizeof(int), cudaMemcpyDeviceToHost,
+                             s.stream));
+    s.root_cell.assign(nroots, 0);
+    if (nroots > 1)
+      FMM_CUDA(cudaMemcpyAsync(s.root_cell.data(), s.cbase.p, sizeof(int) * nroots,
+                               cudaMemcpyDeviceToHost, s.stream));
+    FMM_CUDA(cudaStreamSynchronize(s.stream));
+    if (hc[TC_FAULT]) throw FmmError(FMM_ERR_DEVICE, "the tree build's blocks lost one another");
+    bool full = false, deep = false;
+    for (int l = 0; l < kMaxLevel; l++) {
+      full |= hc[TC_FULL + l] != 0;
+      deep |= hc[TC_DEEP + l] != 0;
+    }
+    if (deep) {
+      levels = kMaxLevel;
+      sorted = false;
+    }
+    if (full) cap = 2 * ncap;
+    if (!deep && !full) break;
   }
-  const int nlev = (int)s.level_lo.size() - 1;
-  const int nnodes = s.level_lo.back();
+  s.level_lo.assign({0, nroots});
+  for (int l = 1; hc[TC_COUNT + l]; l++) s.level_lo.push_back(s.level_lo.back() + hc[TC_COUNT + l]);
+  const int nlev = (int)s.level_lo.size() - 1, nnodes = s.level_lo.back();
   s.tree_plan = nlev;
   s.maxlevel = nlev - 1;
   s.ncells = nnodes;
-  for (int l = nlev - 1; l >= 0; l--) {
-    int lo = s.level_lo[l], hi = s.level_lo[l + 1];
-    k_nnode<<<ceil_div(hi - lo, TB), TB, 0, s.stream>>>(lo, hi, s.nchildn.p, s.nfirst.p,
-                                                        s.nnode.p);
-    FMM_LAUNCH_CHECK();
+  s.nleaves = hc[TC_LEAVES];
+  if (rank && !hc[TC_BIG]) {
+    s.radii_set = radii;
+    return;
   }
-  // first cell of each root: exclusive scan of the roots' subtree sizes
-  s.cbase.ensure(nroots + 1);
-  s.coff.ensure(nroots + 1);
-  FMM_CUDA(cudaMemsetAsync(s.coff.p + nroots, 0, sizeof(int), s.stream));
-  FMM_CUDA(cudaMemcpyAsync(s.coff.p, s.nnode.p, sizeof(int) * nroots, cudaMemcpyDeviceToDevice,
+  // leaves of more bodies than a warp ranks: stable sort by leaf-truncated key from input order
+  if (levels < kMaxLevel) {
+    k_keys<T><<<ceil_div(n, TB), TB, 0, s.stream>>>(s.bodies_in.p, n, s.box.p, s.root_first,
+                                                    nroots, s.keys.p, s.idx.p);
+    FMM_LAUNCH_CHECK();
+    forest_sort(s, s.keys.p, s.keys2.p, s.idx.p, s.idx2.p, n, nroots, 3 * kMaxLevel);
+  }
+  int* blev = s.idx.p;
+  k_leaf_levels<<<ceil_div(nnodes, TB), TB, 0, s.stream>>>(nnodes, s.nchildn.p, s.nbegin.p,
+                                                           s.ncount.p, s.nlevel.p, blev);
+  FMM_LAUNCH_CHECK();
+  k_tkey<<<ceil_div(n, TB), TB, 0, s.stream>>>(n, s.keys2.p, s.idx2.p, blev, s.keys.p, s.order.p);
+  FMM_LAUNCH_CHECK();
+  // s.order holds 0..n-1 (input positions); sort them by truncated key within each root
+  FMM_CUDA(cudaMemcpyAsync(s.idx.p, s.order.p, n * sizeof(int), cudaMemcpyDeviceToDevice,
                            s.stream));
-  exclusive_sum_int(s, s.coff.p, s.cbase.p, nroots + 1);
-  for (int l = 0; l < nlev; l++) {
-    int lo = s.level_lo[l], hi = s.level_lo[l + 1];
-    k_pos<<<ceil_div(hi - lo, TB), TB, 0, s.stream>>>(lo, hi, s.nchildn.p, s.nfirst.p,
-                                                      s.nnode.p, s.cbase.p, s.npos.p, s.ncb.p);
-    FMM_LAUNCH_CHECK();
-  }
-  // cells
-  s.c_iparent.ensure(nnodes); s.c_ichild.ensure(nnodes); s.c_nchild.ensure(nnodes);
-  s.c_ibody.ensure(nnodes); s.c_nbody.ensure(nnodes); s.c_level.ensure(nnodes);
-  s.c_icell.ensure(nnodes);
-  s.cX.ensure(nnodes);
-  s.c_root.ensure(nnodes);
-  k_cells<T><<<ceil_div(nnodes, TB), TB, 0, s.stream>>>(
-      nnodes, s.box.p, s.nbegin.p, s.ncount.p, s.nparent.p, s.nchildn.p, s.nlevel.p, s.nsid.p,
-      s.cbase.p, s.npos.p, s.ncb.p, s.nX.p, s.c_iparent.p, s.c_ichild.p, s.c_nchild.p,
-      s.c_ibody.p, s.c_nbody.p, s.c_level.p, s.c_icell.p, s.cX.p, s.c_root.p);
-  FMM_LAUNCH_CHECK();
-  s.c_info.ensure(nnodes);
-  k_cell_info<<<ceil_div(nnodes, TB), TB, 0, s.stream>>>(nnodes, s.c_nchild.p, s.c_ichild.p,
-                                                         s.c_nbody.p, s.c_ibody.p, s.c_info.p);
-  FMM_LAUNCH_CHECK();
-  // bodies inside a leaf in input order (the stable partitions of the reference keep it)
-  s.order.ensure(n);
-  if (s.cfg.ncrit <= 64 && s.maxlevel < kMaxLevel) {
-    // every leaf holds at most ncrit <= 64 bodies: rank them per leaf
-    k_leaf_reorder<<<ceil_div(32LL * nnodes, TB), TB, 0, s.stream>>>(
-        nnodes, s.nchildn.p, s.nbegin.p, s.ncount.p, s.idx2.p, s.order.p);
-    FMM_LAUNCH_CHECK();
-  } else {
-    // general case: stable sort by leaf-truncated key from input order
-    int* blev = s.idx.p;
-    k_leaf_levels<<<ceil_div(nnodes, TB), TB, 0, s.stream>>>(nnodes, s.nchildn.p, s.nbegin.p,
-                                                             s.ncount.p, s.nlevel.p, blev);
-    FMM_LAUNCH_CHECK();
-    k_tkey<<<ceil_div(n, TB), TB, 0, s.stream>>>(n, s.keys2.p, s.idx2.p, blev, s.keys.p, s.order.p);
-    FMM_LAUNCH_CHECK();
-    // s.order holds 0..n-1 (input positions); sort them by truncated key within each root
-    FMM_CUDA(cudaMemcpyAsync(s.idx.p, s.order.p, n * sizeof(int), cudaMemcpyDeviceToDevice,
-                             s.stream));
-    forest_sort(s, s.keys.p, s.keys2.p, s.idx.p, s.order.p, n, nroots, 3 * kMaxLevel);
-  }
-  s.bodies.ensure(n);
+  forest_sort(s, s.keys.p, s.keys2.p, s.idx.p, s.order.p, n, nroots, 3 * kMaxLevel);
   k_permute<T><<<ceil_div(n, TB), TB, 0, s.stream>>>(n, s.bodies_in.p, s.order.p, s.bodies.p);
   FMM_LAUNCH_CHECK();
-  // leaf cell list
-  s.nsplit.ensure(nnodes + 1);
-  int* flags = s.nsplit.p;
-  s.coff.ensure(nnodes + 1);
-  k_leaf_flags<<<ceil_div(nnodes + 1, TB), TB, 0, s.stream>>>(nnodes, s.nchildn.p, flags);
-  FMM_LAUNCH_CHECK();
-  exclusive_sum_int(s, flags, s.coff.p, nnodes + 1);
-  FMM_CUDA(cudaMemcpyAsync(s.scal_host, s.coff.p + nnodes, sizeof(int), cudaMemcpyDeviceToHost,
-                           s.stream));
-  s.leaves.ensure(nnodes);
-  k_leaf_scatter<<<ceil_div(nnodes, TB), TB, 0, s.stream>>>(nnodes, s.nchildn.p, s.coff.p,
-                                                            s.npos.p, s.leaves.p);
-  FMM_LAUNCH_CHECK();
-  s.root_cell.resize(nroots);
-  FMM_CUDA(cudaMemcpyAsync(s.root_cell.data(), s.cbase.p, sizeof(int) * nroots,
-                           cudaMemcpyDeviceToHost, s.stream));
-  FMM_CUDA(cudaStreamSynchronize(s.stream));
-  s.nleaves = s.scal_host[0];
 }
 
 // The bodies of part `part` of nparts: [t0, t1) with t = floor(k n / nparts), each bound
@@ -1095,7 +1079,7 @@ void partition_range(SolverBase& s) {
   FMM_LAUNCH_CHECK();
 }
 
-template void build_tree<float>(Solver<float>&);
-template void build_tree<double>(Solver<double>&);
+template void build_tree<float>(Solver<float>&, bool);
+template void build_tree<double>(Solver<double>&, bool);
 
 }  // namespace fmmb200
