@@ -298,46 +298,54 @@ __global__ void k_cper_reduce(int nroots, int nt, const int* __restrict__ root_c
   if (t >= nroots * nt) return;
   const int r = t / nt, e = t % nt;
   T acc = L[(size_t)root_cell[r] * ncoef + e];
+#pragma unroll 27
   for (int q = 0; q < kCPerShifts; q++) acc += contrib[((size_t)r * kCPerShifts + q) * nt + e];
   L[(size_t)root_cell[r] * ncoef + e] = acc;
 }
 
+// the 26 copies' terms, a warp each (block o, root r), then their sums in the reference's
+// order
 template <typename T, int P>
 __global__ void __launch_bounds__(32)
     k_cper_m2m(const T* __restrict__ Mp, const int* __restrict__ root_cell,
-               const vec4<T>* __restrict__ cX, T cycle, int ncoef, T* __restrict__ Mout) {
+               const vec4<T>* __restrict__ cX, T cycle, int ncoef, T* __restrict__ contrib) {
   constexpr int NT = cart::NT(P), KO = (NT + 31) / 32;
   __shared__ T sc[NT], sm[NT];
-  const int lane = lane_id(), r = blockIdx.x;
+  const int lane = lane_id(), o = blockIdx.x, r = blockIdx.y;
   const vec4<T> X = cX[root_cell[r]];
   for (int t = lane; t < NT; t += 32) sm[t] = Mp[(size_t)r * ncoef + t];
-  T acc[KO];
-  int ox[KO], oy[KO], oz[KO];
+  int ix, iy, iz;
+  cper_outer(o, ix, iy, iz);
+  // child centre X + (ix, iy, iz) cycle, then dX = Xparent - Xchild as the reference rounds
+  const T xc = X.x + (T)ix * cycle, yc = X.y + (T)iy * cycle, zc = X.z + (T)iz * cycle;
+  {
+    T C[NT];
+    C[0] = 1;
+    cart::power<T, P>(C, X.x - xc, X.y - yc, X.z - zc);
+    spread_c<T, NT>(C, sc, lane);
+  }
+  __syncwarp();
 #pragma unroll
   for (int i = 0; i < KO; i++) {
-    acc[i] = 0;
-    cart::mi_of(lane + 32 * i, ox[i], oy[i], oz[i]);
-  }
-  for (int o = 0; o < 26; o++) {
-    int ix, iy, iz;
-    cper_outer(o, ix, iy, iz);
-    // child centre X + (ix, iy, iz) cycle, then dX = Xparent - Xchild as the reference rounds
-    const T xc = X.x + (T)ix * cycle, yc = X.y + (T)iy * cycle, zc = X.z + (T)iz * cycle;
-    {
-      T C[NT];
-      C[0] = 1;
-      cart::power<T, P>(C, X.x - xc, X.y - yc, X.z - zc);
-      __syncwarp();
-      spread_c<T, NT>(C, sc, lane);
+    const int t = lane + 32 * i;
+    if (t < NT) {
+      int nx, ny, nz;
+      cart::mi_of(t, nx, ny, nz);
+      contrib[((size_t)r * 26 + o) * NT + t] = cart::m2m_term<T>(nx, ny, nz, sc, sm);
     }
-    __syncwarp();
-#pragma unroll
-    for (int i = 0; i < KO; i++)
-      if (lane + 32 * i < NT) acc[i] += cart::m2m_term<T>(ox[i], oy[i], oz[i], sc, sm);
   }
+}
+
+template <typename T>
+__global__ void k_cper_m2m_sum(int nroots, int nt, const T* __restrict__ contrib, int ncoef,
+                               T* __restrict__ Mout) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nroots * nt) return;
+  const int r = t / nt, e = t % nt;
+  T acc = 0;
 #pragma unroll
-  for (int i = 0; i < KO; i++)
-    if (lane + 32 * i < NT) Mout[(size_t)r * ncoef + lane + 32 * i] = acc[i];
+  for (int o = 0; o < 26; o++) acc += contrib[((size_t)r * 26 + o) * nt + e];
+  Mout[(size_t)r * ncoef + e] = acc;
 }
 
 template <typename T>
@@ -370,8 +378,11 @@ template <typename T, int P> static void cperiodic_(Solver<T>& s) {
     k_cper_reduce<T><<<ceil_div((long long)R * NT, 128), 128, 0, s.stream>>>(
         R, NT, s.c_root_cells.p, s.pC.p, s.L.p, s.ncoef);
     FMM_LAUNCH_CHECK();
-    k_cper_m2m<T, P><<<R, 32, 0, s.stream>>>(s.pM.p, s.c_root_cells.p, s.cX.p, cycle, s.ncoef,
-                                             s.pM2.p);
+    k_cper_m2m<T, P><<<dim3(26, R), 32, 0, s.stream>>>(s.pM.p, s.c_root_cells.p, s.cX.p, cycle,
+                                                       s.ncoef, s.pC.p);
+    FMM_LAUNCH_CHECK();
+    k_cper_m2m_sum<T><<<ceil_div((long long)R * NT, 128), 128, 0, s.stream>>>(R, NT, s.pC.p,
+                                                                              s.ncoef, s.pM2.p);
     FMM_LAUNCH_CHECK();
     std::swap(s.pM, s.pM2);
     cycle = cycle * (T)3;
