@@ -253,7 +253,6 @@ static int autotune_ncrit_t(Solver<T>& s, const int* cand, int ncand, int repeat
   try {
     for (int i = 0; i < ncand; i++) {
       s.cfg.ncrit = cand[i];
-      s.trav_sized = false;  // list sizes change with the tree
       solve_all(s);
       std::vector<float> ms;
       for (int r = 0; r < repeats; r++) {
@@ -282,7 +281,6 @@ static int autotune_ncrit_t(Solver<T>& s, const int* cand, int ncand, int repeat
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   s.cfg.ncrit = best_nc;
-  s.trav_sized = false;
   s.stage = ST_BODIES;
   if (best) *best = best_nc;
   return FMM_OK;
@@ -350,7 +348,6 @@ static void solve_ij_t(fmm_b200_solver* h, Solver<T>& s, int nt, int ns, int com
   if (!set_segments(*h->base, 2, counts, &n)) throw FmmError(FMM_ERR_INVALID, "sizes");
   s.ij = true;
   s.ij_common_box = common_box != 0;
-  s.trav_sized = false;  // the frontier holds one pair, not one per root
   try {
     solve_all(s);
   } catch (...) {
@@ -471,7 +468,7 @@ int fmm_b200_create(const fmm_b200_config* cfg, fmm_b200_solver** out) {
                          &s_.p2p_bucket, &s_.p2p_hist, &s_.p2p_nsrc, &s_.p2p_work}; \
     for (auto* a : ia) a->OP();                                                            \
     s_.keys.OP(); s_.keys2.OP(); s_.c_icell.OP(); s_.m2l.OP(); s_.fs_keys.OP();            \
-    s_.c_info.OP(); s_.fs_root.OP(); s_.fs_root2.OP();                                     \
+    s_.c_info.OP(); s_.fs_root.OP(); s_.fs_root2.OP(); s_.tgt_key.OP();                                   \
     s_.p2p.OP(); s_.list_tmp.OP(); s_.p2p_pairs_count.OP(); s_.p2p_order.OP();             \
     s_.p2p_srcs.OP();                                                                      \
     s_.cub_tmp.OP(); s_.front.OP(); s_.front2.OP();                                        \
@@ -525,7 +522,6 @@ int fmm_b200_destroy(fmm_b200_solver* h) {
 int fmm_b200_set_mutual(fmm_b200_solver* h, int mutual) {
   if (!h || !h->base || (mutual != 0 && mutual != 1)) return FMM_ERR_INVALID;
   h->base->cfg.mutual = mutual;
-  h->base->trav_sized = false;
   return FMM_OK;
 }
 

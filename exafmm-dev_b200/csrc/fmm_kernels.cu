@@ -157,7 +157,6 @@ template <typename T> void prepare(Solver<T>& s) {
 // downward pass stale
 void finish(SolverBase& s) {
   if (s.stage > ST_UP) s.stage = ST_UP;
-  s.trav_sized = false;
 }
 
 void check_list(const SolverBase& s, int n, const int* cells, const char* what) {
@@ -513,7 +512,6 @@ int fmm_b200_kernel_set_cells(fmm_b200_solver* h, int nc, const double* X, const
     s.level_lo.assign({0, nc});
     s.nm2l = s.np2p = 0;
     s.p2p_ordered = false;
-    s.trav_sized = false;
     s.stage = ST_TREE;
     prepare(s);  // expansions and targets zero
     FMM_CUDA(cudaMemsetAsync(s.trg_s.p, 0, sizeof(vec4<T>) * std::max(n, 1), s.stream));

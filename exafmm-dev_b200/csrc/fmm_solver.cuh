@@ -140,8 +140,7 @@ struct SolverBase {
   DevArr<unsigned long long> fs_keys;
   DevArr<int> fs_idx;
   DevArr<int2> front, front2;
-  bool trav_sized = false;  // list / frontier buffers sized by a counted traversal
-  int trav_steps = 0, trav_maxlevel = 0;  // the last traversal's steps, and its tree depth
+  int trav_steps = 0, trav_maxlevel = 0;  // the last traversal's steps (0: none), its tree depth
   int tree_plan = 0;        // levels of the handle's last tree (0: none)
   int write_r = 1;          // P2M / M2M set the cell radii (else the structure pass did)
   // P2P lanes per target by target leaf size: 4 up to p2p_g4 bodies, 2 up to p2p_g2, else 1
@@ -171,7 +170,8 @@ struct SolverBase {
   DevArr<char> cub_tmp2;
   bool p2p_pending = false;
   cudaEvent_t p2p_ready = nullptr;
-  DevArr<int> m2l_tgt;  // M2L target cells, by descending number of 32-source batches
+  DevArr<int> m2l_tgt;       // M2L target cells by descending pair count
+  DevArr<unsigned> tgt_key;  // scratch of their ordering
   // P2P target leaves in launch order (valid while p2p_ordered: the lists of the last
   // traversal), each with its source bodies; scratch of the ordering
   DevArr<int4> p2p_order;

@@ -15,6 +15,7 @@
 
 #include <climits>
 
+#include "fmm_grid.cuh"
 #include "fmm_solver.cuh"
 
 namespace fmmb200 {
@@ -179,42 +180,6 @@ __device__ __forceinline__ int digit_at(unsigned long long key, int level) {
 // between steps (about 1.5 us).  Bound by latency throughout: a warp's split is two to three
 // dependent rounds of key reads.
 //
-// The barrier counts arrivals up; a block that waits longer than kSyncSpins polls (seconds)
-// sets *fault and every block leaves at its next barrier.
-constexpr int kSyncSpins = 1 << 24;
-
-struct GridBarrier {
-  unsigned* arrived;  // zero before the launch
-  int* fault;
-  unsigned epoch;
-  // all blocks' writes before it are visible to all blocks after it; false: leave the kernel
-  __device__ __forceinline__ bool sync() {
-    __shared__ int ok;
-    __syncthreads();
-    epoch += gridDim.x;
-    if (threadIdx.x == 0) {
-      __threadfence();
-      atomicAdd(arrived, 1u);
-      int good = 1;
-      for (int spin = 0;; spin++) {
-        unsigned seen;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrived) : "memory");
-        if (seen >= epoch) break;
-        if (spin == kSyncSpins) {
-          atomicExch(fault, 1);
-          good = 0;
-          break;
-        }
-      }
-      __threadfence();
-      if (good && *(volatile int*)fault) good = 0;
-      ok = good;
-    }
-    __syncthreads();
-    return ok != 0;
-  }
-};
-
 // control block of k_tree (ints, zero before the launch except where said)
 enum {
   TC_ARRIVED, TC_FAULT, TC_BIG,  // TC_BIG: a leaf of more than kRankBodies bodies
