@@ -66,6 +66,9 @@ SIGNATURES = {
     "fmm_b200_supported_orders": (_i, [_i, _vp, _i]),
     "fmm_b200_solve_device": (_i, [_vp, _i, _vp, _vp]),
     "fmm_b200_solve_host": (_i, [_vp, _i, _vp, _vp, _vp, _vp]),
+    "fmm_b200_solve_host_trg": (_i, [_vp, _i, _vp, _vp, _vp]),
+    "fmm_b200_solve_batch_host_trg": (_i, [_vp, _i, _vp, _vp, _vp, _vp]),
+    "fmm_b200_solve_ij_host_trg": (_i, [_vp, _i, _vp, _vp, _i, _vp, _vp, _i, _vp]),
     "fmm_b200_set_bodies_host": (_i, [_vp, _i, _vp, _vp]),
     "fmm_b200_solve_batch_device": (_i, [_vp, _i, _vp, _vp, _vp]),
     "fmm_b200_solve_batch_host": (_i, [_vp, _i, _vp, _vp, _vp, _vp, _vp]),
@@ -336,7 +339,7 @@ class Solver:
         self._check(self.lib.fmm_b200_downward_pass(self.h))
 
     def trg(self):
-        out = np.zeros((self.n, 4))
+        out = np.empty((self.n, 4))
         if self.n:
             self._check(self.lib.fmm_b200_get_trg_host(self.h, _p(out)))
         return out
@@ -347,11 +350,10 @@ class Solver:
         x = np.ascontiguousarray(x, np.float64).reshape(-1, 3)
         q = np.ascontiguousarray(q, np.float64).reshape(-1)
         n = len(q)
-        p = np.zeros(n)
-        f = np.zeros((n, 3))
-        self._check(self.lib.fmm_b200_solve_host(self.h, n, _p(x), _p(q), _p(p), _p(f)))
+        out = np.empty((n, 4))
+        self._check(self.lib.fmm_b200_solve_host_trg(self.h, n, _p(x), _p(q), _p(out)))
         self.n = n
-        return np.concatenate([p[:, None], f], axis=1)
+        return out
 
     def solve_ij(self, xt, qt, xs, qs, common_box=True):
         """Targets (xt, qt) against sources (xs, qs) in two trees (examples/serial.cxx IneJ
@@ -361,13 +363,12 @@ class Solver:
         qt = np.ascontiguousarray(qt, np.float64).reshape(-1)
         xs = np.ascontiguousarray(xs, np.float64).reshape(-1, 3)
         qs = np.ascontiguousarray(qs, np.float64).reshape(-1)
-        p = np.zeros(len(qt))
-        f = np.zeros((len(qt), 3))
-        self._check(self.lib.fmm_b200_solve_ij_host(self.h, len(qt), _p(xt), _p(qt), len(qs),
-                                                     _p(xs), _p(qs), int(common_box), _p(p),
-                                                     _p(f)))
+        out = np.empty((len(qt), 4))
+        self._check(self.lib.fmm_b200_solve_ij_host_trg(self.h, len(qt), _p(xt), _p(qt), len(qs),
+                                                         _p(xs), _p(qs), int(common_box),
+                                                         _p(out)))
         self.n = len(qt) + len(qs)
-        return np.concatenate([p[:, None], f], axis=1)
+        return out
 
     def solve_batch(self, xs, qs):
         """Several independent solves in one batch: lists of (n_s, 3) positions and (n_s,)
@@ -376,12 +377,10 @@ class Solver:
         x = np.ascontiguousarray(np.concatenate([np.asarray(a, np.float64).reshape(-1, 3) for a in xs]))
         q = np.ascontiguousarray(np.concatenate([np.asarray(a, np.float64).reshape(-1) for a in qs]))
         n = len(q)
-        p = np.zeros(n)
-        f = np.zeros((n, 3))
-        self._check(self.lib.fmm_b200_solve_batch_host(self.h, len(counts), _p(counts), _p(x),
-                                                       _p(q), _p(p), _p(f)))
+        out = np.empty((n, 4))
+        self._check(self.lib.fmm_b200_solve_batch_host_trg(self.h, len(counts), _p(counts), _p(x),
+                                                           _p(q), _p(out)))
         self.n = n
-        out = np.concatenate([p[:, None], f], axis=1)
         return np.split(out, np.cumsum(counts)[:-1])
 
     def solve_batch_device(self, counts, bodies_ptr, trg_ptr):

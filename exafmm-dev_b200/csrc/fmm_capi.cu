@@ -97,20 +97,47 @@ bool set_segments(SolverBase& s, int nsolves, const int* counts, int* total) {
   return true;
 }
 
-template <typename T> void set_bodies_host_t(Solver<T>& s, int n, const double* x, const double* q,
-                                             DevArr<double>& tmp) {
-  s.n = n;
-  s.bodies_in.ensure(std::max(n, 1));
-  if (n > 0) {
-    tmp.ensure(4 * (size_t)n);
-    FMM_CUDA(cudaMemcpyAsync(tmp.p, x, 3 * sizeof(double) * n, cudaMemcpyHostToDevice, s.stream));
-    FMM_CUDA(cudaMemcpyAsync(tmp.p + 3 * (size_t)n, q, sizeof(double) * n,
-                             cudaMemcpyHostToDevice, s.stream));
-    k_pack<T><<<ceil_div(n, 256), 256, 0, s.stream>>>(n, tmp.p, tmp.p + 3 * (size_t)n,
-                                                      s.bodies_in.p);
+// host positions and charges to bodies_in: n bodies, then n2 of a second set
+template <typename T>
+void set_bodies_host_t(Solver<T>& s, int n, const double* x, const double* q, int n2 = 0,
+                       const double* x2 = nullptr, const double* q2 = nullptr) {
+  const size_t m = (size_t)n + n2;
+  s.n = (int)m;
+  s.bodies_in.ensure(std::max<size_t>(m, 1));
+  if (m > 0) {
+    DevArr<double>& tmp = s.dtmp;
+    tmp.ensure(4 * m);
+    auto up = [&](double* dst, const double* src, size_t k) {
+      if (k) FMM_CUDA(cudaMemcpyAsync(dst, src, sizeof(double) * k, cudaMemcpyHostToDevice, s.stream));
+    };
+    up(tmp.p, x, 3 * (size_t)n);
+    up(tmp.p + 3 * (size_t)n, x2, 3 * (size_t)n2);
+    up(tmp.p + 3 * m, q, n);
+    up(tmp.p + 3 * m + n, q2, n2);
+    k_pack<T><<<ceil_div(m, 256), 256, 0, s.stream>>>((int)m, tmp.p, tmp.p + 3 * m, s.bodies_in.p);
     FMM_LAUNCH_CHECK();
   }
   s.stage = ST_BODIES;
+}
+
+// the first n results to the host, as p (n) and f (3 n) or, with f null, as 4 n rows; waits
+template <typename T> void results_host(Solver<T>& s, int n, double* p, double* f) {
+  if (n > 0) {
+    DevArr<double>& tmp = s.dtmp;
+    tmp.ensure(4 * (size_t)n);
+    if (f) {
+      k_unpack_pf<T><<<ceil_div(n, 256), 256, 0, s.stream>>>(n, s.trg_out.p, tmp.p, tmp.p + n);
+      FMM_LAUNCH_CHECK();
+      FMM_CUDA(cudaMemcpyAsync(p, tmp.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s.stream));
+      FMM_CUDA(cudaMemcpyAsync(f, tmp.p + n, 3 * sizeof(double) * n, cudaMemcpyDeviceToHost,
+                               s.stream));
+    } else {
+      k_unpack<T><<<ceil_div(n, 256), 256, 0, s.stream>>>(n, s.trg_out.p, tmp.p);
+      FMM_LAUNCH_CHECK();
+      FMM_CUDA(cudaMemcpyAsync(p, tmp.p, 4 * sizeof(double) * n, cudaMemcpyDeviceToHost, s.stream));
+    }
+  }
+  FMM_CUDA(cudaStreamSynchronize(s.stream));
 }
 
 template <typename T> void stage_tree(Solver<T>& s, bool radii = false) {
@@ -574,7 +601,7 @@ int fmm_b200_set_bodies_host(fmm_b200_solver* h, int n, const double* x, const d
   if (n < 0 || (n > 0 && (!x || !q))) return FMM_ERR_INVALID;
   if (!h || !h->base) return FMM_ERR_INVALID;
   h->base->seg = {0, n};
-  return FMM_DISPATCH(h, set_bodies_host_t(s, n, x, q, h->base->dtmp));
+  return FMM_DISPATCH(h, set_bodies_host_t(s, n, x, q));
 }
 
 int fmm_b200_set_bodies_device(fmm_b200_solver* h, int n, const void* d_bodies) {
@@ -634,25 +661,25 @@ int fmm_b200_solve_device(fmm_b200_solver* h, int n, const void* d_bodies, void*
   });
 }
 
-int fmm_b200_solve_host(fmm_b200_solver* h, int n, const double* x, const double* q, double* p,
-                        double* f) {
-  if (n < 0 || (n > 0 && (!x || !q || !p || !f))) return FMM_ERR_INVALID;
+static int solve_host(fmm_b200_solver* h, int n, const double* x, const double* q, double* p,
+                      double* f) {
   if (!h || !h->base) return FMM_ERR_INVALID;
   h->base->seg = {0, n};
   return FMM_DISPATCH(h, {
-    DevArr<double>& tmp = h->base->dtmp;
-    set_bodies_host_t(s, n, x, q, tmp);
+    set_bodies_host_t(s, n, x, q);
     solve_all(s);
-    if (n > 0) {
-      tmp.ensure(4 * (size_t)n);
-      k_unpack_pf<T><<<ceil_div(n, 256), 256, 0, s.stream>>>(n, s.trg_out.p, tmp.p, tmp.p + n);
-      FMM_LAUNCH_CHECK();
-      FMM_CUDA(cudaMemcpyAsync(p, tmp.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s.stream));
-      FMM_CUDA(cudaMemcpyAsync(f, tmp.p + n, 3 * sizeof(double) * n, cudaMemcpyDeviceToHost,
-                               s.stream));
-    }
-    FMM_CUDA(cudaStreamSynchronize(s.stream));
+    results_host(s, n, p, f);
   });
+}
+int fmm_b200_solve_host(fmm_b200_solver* h, int n, const double* x, const double* q, double* p,
+                        double* f) {
+  if (n < 0 || (n > 0 && (!x || !q || !p || !f))) return FMM_ERR_INVALID;
+  return solve_host(h, n, x, q, p, f);
+}
+int fmm_b200_solve_host_trg(fmm_b200_solver* h, int n, const double* x, const double* q,
+                            double* trg) {
+  if (n < 0 || (n > 0 && (!x || !q || !trg))) return FMM_ERR_INVALID;
+  return solve_host(h, n, x, q, trg, nullptr);
 }
 
 int fmm_b200_solve_batch_device(fmm_b200_solver* h, int nsolves, const int* counts,
@@ -675,55 +702,49 @@ int fmm_b200_solve_batch_device(fmm_b200_solver* h, int nsolves, const int* coun
   });
 }
 
-int fmm_b200_solve_batch_host(fmm_b200_solver* h, int nsolves, const int* counts,
-                              const double* x, const double* q, double* p, double* f) {
+static int solve_batch_host(fmm_b200_solver* h, int nsolves, const int* counts, const double* x,
+                            const double* q, double* p, double* f, bool rows) {
   if (!h || !h->base) return FMM_ERR_INVALID;
   int n = 0;
   if (!set_segments(*h->base, nsolves, counts, &n)) return FMM_ERR_INVALID;
-  if (n > 0 && (!x || !q || !p || !f)) return FMM_ERR_INVALID;
+  if (n > 0 && (!x || !q || !p || (!f && !rows))) return FMM_ERR_INVALID;
   return FMM_DISPATCH(h, {
-    DevArr<double>& tmp = h->base->dtmp;
-    std::vector<int> seg = s.seg;
-    set_bodies_host_t(s, n, x, q, tmp);
-    s.seg = seg;
+    set_bodies_host_t(s, n, x, q);
     solve_all(s);
-    if (n > 0) {
-      tmp.ensure(4 * (size_t)n);
-      k_unpack_pf<T><<<ceil_div(n, 256), 256, 0, s.stream>>>(n, s.trg_out.p, tmp.p, tmp.p + n);
-      FMM_LAUNCH_CHECK();
-      FMM_CUDA(cudaMemcpyAsync(p, tmp.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s.stream));
-      FMM_CUDA(cudaMemcpyAsync(f, tmp.p + n, 3 * sizeof(double) * n, cudaMemcpyDeviceToHost,
-                               s.stream));
-    }
-    FMM_CUDA(cudaStreamSynchronize(s.stream));
+    results_host(s, n, p, f);
   });
 }
+int fmm_b200_solve_batch_host(fmm_b200_solver* h, int nsolves, const int* counts,
+                              const double* x, const double* q, double* p, double* f) {
+  return solve_batch_host(h, nsolves, counts, x, q, p, f, false);
+}
+int fmm_b200_solve_batch_host_trg(fmm_b200_solver* h, int nsolves, const int* counts,
+                                  const double* x, const double* q, double* trg) {
+  return solve_batch_host(h, nsolves, counts, x, q, trg, nullptr, true);
+}
 
+static int solve_ij_host(fmm_b200_solver* h, int nt, const double* xt, const double* qt, int ns,
+                         const double* xs, const double* qs, int common_box, double* p, double* f,
+                         bool rows) {
+  if (!h || !h->base || nt < 0 || ns < 0) return FMM_ERR_INVALID;
+  if ((nt > 0 && (!xt || !qt || !p || (!f && !rows))) || (ns > 0 && (!xs || !qs)))
+    return FMM_ERR_INVALID;
+  if (nt == 0) return FMM_OK;
+  return FMM_DISPATCH(h, {
+    set_bodies_host_t(s, nt, xt, qt, ns, xs, qs);
+    solve_ij_t(h, s, nt, ns, common_box);
+    results_host(s, nt, p, f);
+  });
+}
 int fmm_b200_solve_ij_host(fmm_b200_solver* h, int nt, const double* xt, const double* qt,
                            int ns, const double* xs, const double* qs, int common_box, double* p,
                            double* f) {
-  if (!h || !h->base || nt < 0 || ns < 0) return FMM_ERR_INVALID;
-  if ((nt > 0 && (!xt || !qt || !p || !f)) || (ns > 0 && (!xs || !qs))) return FMM_ERR_INVALID;
-  if (nt == 0) return FMM_OK;
-  std::vector<double> x(3 * ((size_t)nt + ns)), q((size_t)nt + ns);
-  std::memcpy(x.data(), xt, sizeof(double) * 3 * nt);
-  std::memcpy(q.data(), qt, sizeof(double) * nt);
-  if (ns) {
-    std::memcpy(x.data() + 3 * (size_t)nt, xs, sizeof(double) * 3 * ns);
-    std::memcpy(q.data() + nt, qs, sizeof(double) * ns);
-  }
-  return FMM_DISPATCH(h, {
-    DevArr<double>& tmp = h->base->dtmp;
-    set_bodies_host_t(s, nt + ns, x.data(), q.data(), tmp);
-    solve_ij_t(h, s, nt, ns, common_box);
-    tmp.ensure(4 * (size_t)nt);
-    k_unpack_pf<T><<<ceil_div(nt, 256), 256, 0, s.stream>>>(nt, s.trg_out.p, tmp.p, tmp.p + nt);
-    FMM_LAUNCH_CHECK();
-    FMM_CUDA(cudaMemcpyAsync(p, tmp.p, sizeof(double) * nt, cudaMemcpyDeviceToHost, s.stream));
-    FMM_CUDA(cudaMemcpyAsync(f, tmp.p + nt, 3 * sizeof(double) * nt, cudaMemcpyDeviceToHost,
-                             s.stream));
-    FMM_CUDA(cudaStreamSynchronize(s.stream));
-  });
+  return solve_ij_host(h, nt, xt, qt, ns, xs, qs, common_box, p, f, false);
+}
+int fmm_b200_solve_ij_host_trg(fmm_b200_solver* h, int nt, const double* xt, const double* qt,
+                               int ns, const double* xs, const double* qs, int common_box,
+                               double* trg) {
+  return solve_ij_host(h, nt, xt, qt, ns, xs, qs, common_box, trg, nullptr, true);
 }
 
 int fmm_b200_solve_ij_device(fmm_b200_solver* h, int nt, const void* d_targets, int ns,
@@ -777,15 +798,7 @@ int fmm_b200_get_roots(fmm_b200_solver* h, int* nroots, int* root_cells, int* ro
 int fmm_b200_get_trg_host(fmm_b200_solver* h, double* trg) {
   return FMM_DISPATCH(h, {
     if (s.stage < ST_DOWN) throw FmmError(FMM_ERR_STATE, "downward pass not done");
-    if (s.n > 0) {
-      DevArr<double>& tmp = h->base->dtmp;
-      tmp.ensure(4 * (size_t)s.n);
-      k_unpack<T><<<ceil_div(s.n, 256), 256, 0, s.stream>>>(s.n, s.trg_out.p, tmp.p);
-      FMM_LAUNCH_CHECK();
-      FMM_CUDA(cudaMemcpyAsync(trg, tmp.p, 4 * sizeof(double) * s.n, cudaMemcpyDeviceToHost,
-                               s.stream));
-    }
-    FMM_CUDA(cudaStreamSynchronize(s.stream));
+    results_host(s, s.n, trg, nullptr);
   });
 }
 

@@ -146,6 +146,15 @@ int fmm_b200_solve_device(fmm_b200_solver* s, int n, const void* d_bodies, void*
  * call; synchronous. */
 int fmm_b200_solve_host(fmm_b200_solver* s, int n, const double* x, const double* q,
                         double* p, double* f);
+/* The host solves (this one, the batch and the separate sets below) with the results as
+ * fmm_b200_get_trg_host lays them out: trg receives 4 values (phi, grad phi) per body. */
+int fmm_b200_solve_host_trg(fmm_b200_solver* s, int n, const double* x, const double* q,
+                            double* trg);
+int fmm_b200_solve_batch_host_trg(fmm_b200_solver* s, int nsolves, const int* counts,
+                                  const double* x, const double* q, double* trg);
+int fmm_b200_solve_ij_host_trg(fmm_b200_solver* s, int nt, const double* xt, const double* qt,
+                               int ns, const double* xs, const double* qs, int common_box,
+                               double* trg);
 
 /* ---- batches of independent solves --------------------------------------------------- *
  * nsolves solves with counts[s] bodies each, bodies concatenated in solve order (device
