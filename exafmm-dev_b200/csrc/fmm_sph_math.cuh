@@ -592,6 +592,107 @@ __host__ __device__ __forceinline__ void m2l_fold(const T* rho, T cb, T sb, cons
   }
 }
 
+// The regular harmonics' real factors: Y[n, m] of multipole() = reg[n, m] e^(i m beta).
+template <typename T, int P>
+__host__ __device__ __forceinline__ void multipole_rho(const Angles<T>& a, T rho, T* reg) {
+  T fact = 1, pn = 1, rhom = 1;
+#pragma unroll
+  for (int m = 0; m < P; m++) {
+    T p = pn, p1 = p;
+    reg[sidx(m, m)] = rhom * p;
+    p = a.x * (2 * m + 1) * p1;
+    rhom *= rho;
+    T rhon = rhom;
+#pragma unroll
+    for (int n = m + 1; n < P; n++) {
+      rhon *= T(-1) / T(n + m);
+      reg[sidx(n, m)] = rhon * p;
+      const T p2 = p1;
+      p1 = p;
+      p = (a.x * (2 * n + 1) * p1 - (n + m) * p2) * (T(1) / T(n - m + 1));
+      rhon *= rho;
+    }
+    rhom *= T(-1) / T((2 * m + 2) * (2 * m + 1));
+    pn = -pn * fact * a.y;
+    fact += 2;
+  }
+}
+
+// M2M (UP) and L2L of m2m_term / l2l_term in the azimuthal frame of the shift, folded as
+// m2l_fold: with the source (the child's M, the parent's L) rotated, S'[l, mu] = S[l, mu]
+// e^(i mu beta), each output is e^(-i k beta) A[j, k] and
+//   A[j, k] = sum over mu and d of (s2 reg[d, |k-mu|] + s1 reg[d, k+mu]) Re S'[l, mu]
+//                             + i (s2 reg[d, |k-mu|] - s1 reg[d, k+mu]) Im S'[l, mu],
+// l = j - d (M2M) or j + d (L2L), a harmonic of order above its degree d being none, and the
+// two real factors shared by all (j, l) of one d.  M2M: s2 = (-1)^d, times (-1)^(k-mu) for
+// k < mu (none at mu = 0), s1 = (-1)^(d+mu); L2L: s2 = (-1)^(k-mu) for mu < k, else 1,
+// s1 = (-1)^k (none at mu = 0).  S: the row in the layout of the expansions.
+template <typename T, int P, int K0, int K1, int MU, bool UP>
+__host__ __device__ __forceinline__ void shift_fold_from(const T* reg, T cb, T sb, T er, T ei,
+                                                         const T* S, Cx<T>* A) {
+  if constexpr (MU < P) {
+    Cx<T> m[P - MU];
+#pragma unroll
+    for (int l = MU; l < P; l++) {
+      const T mr = S[2 * sidx(l, MU)], mi = S[2 * sidx(l, MU) + 1];
+      m[l - MU].r = MU > 0 ? mr * er - mi * ei : mr;
+      m[l - MU].i = MU > 0 ? mr * ei + mi * er : mi;
+    }
+#pragma unroll
+    for (int k = K0; k < K1; k++) {
+#pragma unroll
+      for (int d = 0; d < P; d++) {
+        const int q = MU >= k ? MU - k : k - MU;
+        const bool has2 = q <= d && !(UP && MU == 0), has1 = k + MU <= d && !(!UP && MU == 0);
+        if (!has2 && !has1) continue;
+        const bool neg2 = UP ? (d & 1) != (k < MU && (q & 1)) : MU < k && (q & 1);
+        const bool neg1 = UP ? ((d + MU) & 1) != 0 : (k & 1) != 0;
+        T u = T(0), v = T(0);  // factors of the real and the imaginary part
+        if (has2) u = v = neg2 ? -reg[sidx(d, q)] : reg[sidx(d, q)];
+        if (has1) {
+          const T p1 = neg1 ? -reg[sidx(d, k + MU)] : reg[sidx(d, k + MU)];
+          v = has2 ? v - p1 : -p1;
+          u = has2 ? u + p1 : p1;
+        }
+        // k = 0, mu > 0: both terms are there with the same sign, and v is zero
+        const bool real = k == 0 && MU > 0;
+#pragma unroll
+        for (int l = MU; l < P; l++) {
+          const int j = UP ? l + d : l - d;
+          if (j < k || j >= P) continue;
+          Cx<T>& o = A[fold_idx(P, K0, k, j)];
+          if (real) o.r = fma(u, m[l - MU].r, o.r);
+          else fold_fma(u, v, m[l - MU], o);
+        }
+      }
+    }
+    shift_fold_from<T, P, K0, K1, MU + 1, UP>(reg, cb, sb, er * cb - ei * sb, er * sb + ei * cb,
+                                              S, A);
+  }
+}
+// the outputs of the orders [K0, K1), rotated back, at fold_idx
+template <typename T, int P, int K0, int K1, bool UP>
+__host__ __device__ __forceinline__ void shift_fold(const T* reg, T cb, T sb, const T* S,
+                                                    Cx<T>* A) {
+#pragma unroll
+  for (int t = 0; t < fold_idx(P, K0, K1, K1); t++) A[t].r = A[t].i = T(0);
+  shift_fold_from<T, P, K0, K1, 0, UP>(reg, cb, sb, T(1), T(0), S, A);
+  T er = T(1), ei = T(0);
+#pragma unroll
+  for (int k = 0; k < K1; k++) {
+#pragma unroll
+    for (int j = k; j < P && k >= K0 && k > 0; j++) {
+      Cx<T>& o = A[fold_idx(P, K0, k, j)];
+      const T r = fma(er, o.r, ei * o.i);
+      o.i = fma(er, o.i, -ei * o.r);
+      o.r = r;
+    }
+    const T t = er * cb - ei * sb;
+    ei = er * sb + ei * cb;
+    er = t;
+  }
+}
+
 // Y[a, b] for any sign of b from the m >= 0 store (real parts yr, imaginary parts yi)
 template <typename T>
 __host__ __device__ __forceinline__ void yget(const T* yr, const T* yi, int a, int b, T& r,

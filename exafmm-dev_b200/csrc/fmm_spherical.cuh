@@ -148,7 +148,8 @@ __device__ __forceinline__ void m2m_passes(const T* yr, const T* yi, const T* Mc
   }
 }
 
-// M2M (either precision): 8 lanes per parent (one per child slot), 4 parents per warp;
+// M2M, unfolded (FP32 with images, which keeps every bit of its results, and FP64 above P = 8;
+// the others take k_m2m_fold): 8 lanes per parent (one per child slot), 4 parents per warp;
 // each lane translates its child with compile-time indices, the group sums in a fixed
 // order, and the monopole is re-summed in child order (the reference's sequence) so that
 // the radii of the error-optimised MAC see the same M[0] bits.
@@ -225,7 +226,7 @@ __device__ __forceinline__ void l2l_passes(const T* yr, const T* yi, const T* Lp
   }
 }
 
-// L2L (either precision): thread per cell, compile-time indices, the parent's local staged
+// L2L, unfolded (for the solves of k_m2m_reg): thread per cell, compile-time indices, the parent's local staged
 // in the thread's shared row.
 template <typename T, int P>
 __global__ void __launch_bounds__(tr_threads<T>())
@@ -250,9 +251,140 @@ __global__ void __launch_bounds__(tr_threads<T>())
   l2l_passes<T, P, 0>(yr, yi, row, L + (size_t)c * ncoef);
 }
 
+// ---------------------------------------------------------------- folded M2M / L2L
+// The translations with the +m and -m terms folded (sph::shift_fold), for the solves whose M2L
+// folds (see there).  A small level's time is one warp's walk through the unrolled code, whose
+// instructions arrive at about one in eight cycles (35-45 us a level at P = 10 whatever its
+// cells): the folded form is under half as long.  One warp per block, so that a level of few
+// cells spreads over the SMs; the output orders in groups as the M2L's.  Upward phase of
+// 31,250 bodies at P = 10 0.10 -> 0.058 ms, M2M and P2M beside the traversal of 2^20 bodies
+// 0.49-0.61 -> 0.28 ms, of 256 solves at P = 8 2.4-2.9 -> 2.05 ms; FP64 (P = 8) within the
+// spread.
+template <typename T> __host__ __device__ constexpr bool m2l_folds(int P) {
+  return sizeof(T) == 4 || P <= 8;
+}
+template <typename T> __host__ __device__ constexpr int shift_group_end(int P, int K0) {
+  const int words = (int)sizeof(T) / 4;
+  int k = K0 + 1;
+  while (k < P && words * (2 * sph::fold_idx(P, K0, k + 1, k + 1) + sph::NT(P) + 2 * P) <=
+                      (sizeof(T) == 4 ? 184 : 200))
+    k++;
+  return k;
+}
+template <typename T, int P, int K0, bool UP, typename F>
+__device__ __forceinline__ void shift_groups(const T* reg, T cb, T sb, const T* S, F&& store) {
+  if constexpr (K0 < P) {
+    constexpr int K1 = shift_group_end<T>(P, K0);
+    sph::Cx<T> A[sph::fold_idx(P, K0, K1, K1)];
+    if (K0 > 0) {  // source coefficients read and rotated again, not kept since the last group
+      sph::launder(S);
+      sph::launder(cb);
+      sph::launder(sb);
+    }
+    sph::shift_fold<T, P, K0, K1, UP>(reg, cb, sb, S, A);
+#pragma unroll
+    for (int k = K0; k < K1; k++)
+#pragma unroll
+      for (int j = k; j < P; j++) store(sph::sidx(j, k), A[sph::fold_idx(P, K0, k, j)]);
+    shift_groups<T, P, K1, UP>(reg, cb, sb, S, store);
+  }
+}
+
+// M2M: 8 lanes per parent (one per child slot); each writes its child's terms to its own row
+// of shared memory, then the 8 lanes share out the coefficients and add them in child order,
+// the monopole with the rounding of the reference's sequence.
+template <typename T, int P>
+__global__ void __launch_bounds__(32)
+    k_m2m_fold(int lo, int hi, const int* __restrict__ npos, const int* __restrict__ ichild,
+               const int* __restrict__ nchild, vec4<T>* __restrict__ cX, T* __restrict__ M,
+               int ncoef, int use_rmax, T theta, int write_r) {
+  constexpr int NT = sph::NT(P), STR = (2 * NT) | 1;  // odd row stride: no bank conflicts
+  __shared__ T rows[32 * STR], outs[32 * STR];
+  T* row = rows + threadIdx.x * STR;
+  T* mine = outs + threadIdx.x * STR;
+  const int v = lo + blockIdx.x * 4 + (threadIdx.x >> 3), slot = threadIdx.x & 7;
+  int c = 0, nch = 0, c0 = 0;
+  if (v < hi) {
+    c = npos[v];
+    nch = nchild[c];
+    c0 = ichild[c];
+  }
+  T rr = 0;
+  vec4<T> Xp = make_v4<T>(0, 0, 0, 0);
+  if (v < hi) Xp = cX[c];
+  if (slot < nch) {
+    const int cc = c0 + slot;
+    const T* src = M + (size_t)cc * ncoef;
+#pragma unroll
+    for (int t = 0; t < NT; t++) sph::load_pair(src + 2 * t, row[2 * t], row[2 * t + 1]);
+    const vec4<T> Xc = cX[cc];
+    const sph::Angles<T> a = sph::angles(Xp.x - Xc.x, Xp.y - Xc.y, Xp.z - Xc.z);
+    T reg[NT];
+    sph::multipole_rho<T, P>(a, a.r, reg);
+    shift_groups<T, P, 0, true>(reg, a.cb, a.sb, row, [&](int t, const sph::Cx<T>& o) {
+      mine[2 * t] = o.r;
+      mine[2 * t + 1] = o.i;
+    });
+    rr = add_rn(sqrt_rn(norm_rn(sub_rn(Xp.x, Xc.x), sub_rn(Xp.y, Xc.y), sub_rn(Xp.z, Xc.z))),
+                Xc.w);
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    const T x = __shfl_xor_sync(0xffffffffu, rr, o);
+    rr = x > rr ? x : rr;
+  }
+  __syncwarp();
+  if (nch == 0) return;
+  const T* first = outs + (threadIdx.x & ~7) * STR;
+  for (int t = slot; t < 2 * NT; t += 8) {
+    T acc = 0;
+    if (t == 0) {
+      for (int k = 0; k < nch; k++) acc = add_rn(acc, rows[(threadIdx.x & ~7) * STR + k * STR]);
+    } else {
+      for (int k = 0; k < nch; k++) acc += first[k * STR + t];
+    }
+    M[(size_t)c * ncoef + t] = acc;
+  }
+  if (slot == 0 && write_r) {
+    T R = Xp.w;
+    if (use_rmax) R = rr < R ? rr : R;
+    cX[c].w = div_rn(R, theta);
+  }
+}
+
+// L2L: thread per cell, the parent's local staged in the thread's shared row.
+template <typename T, int P>
+__global__ void __launch_bounds__(32)
+    k_l2l_fold(int lo, int hi, const int* __restrict__ npos, const int* __restrict__ iparent,
+               const vec4<T>* __restrict__ cX, T* __restrict__ L, int ncoef,
+               const int4* __restrict__ info, const int* __restrict__ range) {
+  constexpr int NT = sph::NT(P), STR = (2 * NT) | 1;
+  __shared__ T rows[32 * STR];
+  T* row = rows + threadIdx.x * STR;
+  const int v = lo + blockIdx.x * 32 + threadIdx.x;
+  if (v >= hi) return;
+  const int c = npos[v];
+  if (range && !part_holds(info[c], range)) return;  // no body of this part below the cell
+  const int p = iparent[c];
+  const T* src = L + (size_t)p * ncoef;
+#pragma unroll
+  for (int t = 0; t < NT; t++) sph::load_pair(src + 2 * t, row[2 * t], row[2 * t + 1]);
+  const vec4<T> Xc = cX[c], Xp = cX[p];
+  const sph::Angles<T> a = sph::angles(Xc.x - Xp.x, Xc.y - Xp.y, Xc.z - Xp.z);
+  T reg[NT];
+  sph::multipole_rho<T, P>(a, a.r, reg);
+  vec2<T>* Lc = reinterpret_cast<vec2<T>*>(L + (size_t)c * ncoef);
+  shift_groups<T, P, 0, false>(reg, a.cb, a.sb, row, [&](int t, const sph::Cx<T>& o) {
+    vec2<T> l = Lc[t];
+    l.x += o.r;
+    l.y += o.i;
+    Lc[t] = l;
+  });
+}
+
 // ---------------------------------------------------------------- M2L
-// Two kernels.  k_m2l_fold (FP32 without periodic images, and FP64 up to P = 8) folds the +mu and -mu terms of the
-// contraction (sph::m2l_fold: 1,505 instead of 2,420 multiply-adds and additions a pair at
+// Two kernels.  k_m2l_fold (FP32 without periodic images, and FP64 up to P = 8) folds the
+// +mu and -mu terms of the contraction (sph::m2l_fold: 1,505 instead of 2,420 multiply-adds and additions a pair at
 // P = 10) and takes a pair in one pass.  k_m2l_reg (FP64 above P = 8) runs passes over the
 // output degrees with the unfolded terms: there the folded form's harmonics, sums and columns
 // do not fit 255 registers, and its shared memory leaves the L1 too small for the rows that
@@ -279,9 +411,6 @@ __global__ void __launch_bounds__(tr_threads<T>())
 // against 1.47 ms), 12 warps per SM at 168 registers (2.7 ms: more columns, less L1).
 template <typename T> __host__ __device__ constexpr int m2l_words() {
   return sizeof(T) == 4 ? 180 : 216;
-}
-template <typename T> __host__ __device__ constexpr bool m2l_folds(int P) {
-  return sizeof(T) == 4 || P <= 8;
 }
 template <typename T> __host__ __device__ constexpr int m2l_group_end(int P, int K0) {
   const int words = (int)sizeof(T) / 4;
@@ -639,38 +768,58 @@ template <typename T, int P> static void p2m_(Solver<T>& s) {
       s.cfg.use_rmax, (T)s.cfg.theta, s.write_r, s.body_leaf.p);
   FMM_LAUNCH_CHECK();
 }
+// Solves whose M2M, M2L and L2L take the folded forms: all where they fit, but FP32 with
+// images (FOLD_ALL: no solve of this type and order needs the other kernels).
+template <typename T, int P> constexpr bool FOLD_ALL = m2l_folds<T>(P) && sizeof(T) == 8;
+template <typename T, int P> static bool folds(const Solver<T>& s) {
+  return m2l_folds<T>(P) && (FOLD_ALL<T, P> || s.cfg.images == 0);
+}
 template <typename T, int P> static void m2m_(Solver<T>& s, int lo, int hi) {
-  constexpr int NTH = tr_threads<T>();
-  k_m2m_reg<T, P><<<ceil_div(8LL * (hi - lo), NTH), NTH, 0, s.stream>>>(
-      lo, hi, s.npos.p, s.c_ichild.p, s.c_nchild.p, s.cX.p, s.M.p, s.ncoef, s.cfg.use_rmax,
-      (T)s.cfg.theta, s.write_r);
+  if constexpr (m2l_folds<T>(P)) {
+    if (folds<T, P>(s))
+      k_m2m_fold<T, P><<<ceil_div(hi - lo, 4), 32, 0, s.stream>>>(
+          lo, hi, s.npos.p, s.c_ichild.p, s.c_nchild.p, s.cX.p, s.M.p, s.ncoef, s.cfg.use_rmax,
+          (T)s.cfg.theta, s.write_r);
+  }
+  if constexpr (!FOLD_ALL<T, P>) {
+    constexpr int NTH = tr_threads<T>();
+    if (!folds<T, P>(s))
+      k_m2m_reg<T, P><<<ceil_div(8LL * (hi - lo), NTH), NTH, 0, s.stream>>>(
+          lo, hi, s.npos.p, s.c_ichild.p, s.c_nchild.p, s.cX.p, s.M.p, s.ncoef, s.cfg.use_rmax,
+          (T)s.cfg.theta, s.write_r);
+  }
   FMM_LAUNCH_CHECK();
 }
 template <typename T, int P> static void m2l_(Solver<T>& s) {
   if (!s.m2l_ntgt) return;
-  if (sizeof(T) == 4 && s.cfg.images > 0) {
-    launch_m2l_passes<T, P, 0>(s);
-    return;
-  }
   if constexpr (m2l_folds<T>(P)) {
-    constexpr int W = M2LCfg<T, P>::W, LEN = sph::col_len(P) / 2;
-    s.m2l_rows.ensure((size_t)s.ncells * 2 * LEN);
-    k_m2l_rows<T, P><<<ceil_div((long long)s.ncells * LEN, 128), 128, 0, s.stream>>>(
-        s.ncells, s.M.p, s.ncoef, s.m2l_rows.p);
-    FMM_LAUNCH_CHECK();
-    k_m2l_fold<T, P><<<ceil_div(s.m2l_ntgt, W), 32 * W, 0, s.stream>>>(
-        s.m2l_ntgt, s.m2l_tgt.p, s.m2l_off.p, s.m2l.p, s.cX.p, s.m2l_rows.p, s.L.p, s.ncoef,
-        (T)s.cfg.cycle);
-    FMM_LAUNCH_CHECK();
-  } else {
-    launch_m2l_passes<T, P, 0>(s);
+    if (folds<T, P>(s)) {
+      constexpr int W = M2LCfg<T, P>::W, LEN = sph::col_len(P) / 2;
+      s.m2l_rows.ensure((size_t)s.ncells * 2 * LEN);
+      k_m2l_rows<T, P><<<ceil_div((long long)s.ncells * LEN, 128), 128, 0, s.stream>>>(
+          s.ncells, s.M.p, s.ncoef, s.m2l_rows.p);
+      FMM_LAUNCH_CHECK();
+      k_m2l_fold<T, P><<<ceil_div(s.m2l_ntgt, W), 32 * W, 0, s.stream>>>(
+          s.m2l_ntgt, s.m2l_tgt.p, s.m2l_off.p, s.m2l.p, s.cX.p, s.m2l_rows.p, s.L.p, s.ncoef,
+          (T)s.cfg.cycle);
+      FMM_LAUNCH_CHECK();
+    }
   }
+  if constexpr (!FOLD_ALL<T, P>)
+    if (!folds<T, P>(s)) launch_m2l_passes<T, P, 0>(s);
 }
 template <typename T, int P> static void l2l_(Solver<T>& s, int lo, int hi) {
-  constexpr int NTH = tr_threads<T>();
-  k_l2l_reg<T, P><<<ceil_div(hi - lo, NTH), NTH, 0, s.stream>>>(lo, hi, s.npos.p, s.c_iparent.p,
-                                                                s.cX.p, s.L.p, s.ncoef,
-                                                                s.c_info.p, s.part_ptr());
+  if constexpr (m2l_folds<T>(P)) {
+    if (folds<T, P>(s))
+      k_l2l_fold<T, P><<<ceil_div(hi - lo, 32), 32, 0, s.stream>>>(
+          lo, hi, s.npos.p, s.c_iparent.p, s.cX.p, s.L.p, s.ncoef, s.c_info.p, s.part_ptr());
+  }
+  if constexpr (!FOLD_ALL<T, P>) {
+    constexpr int NTH = tr_threads<T>();
+    if (!folds<T, P>(s))
+      k_l2l_reg<T, P><<<ceil_div(hi - lo, NTH), NTH, 0, s.stream>>>(
+          lo, hi, s.npos.p, s.c_iparent.p, s.cX.p, s.L.p, s.ncoef, s.c_info.p, s.part_ptr());
+  }
   FMM_LAUNCH_CHECK();
 }
 template <typename T, int P> static void l2p_(Solver<T>& s) {

@@ -1,6 +1,7 @@
 // Host build of the folded M2L contraction (exafmm-dev_b200/csrc/fmm_sph_math.cuh: fold_rho,
-// m2l_fold) for tests/test_fold_math.py: one pair's M2L in FP64 with the output orders taken
-// in one group or split at K, the source row laid out by order as the kernel reads it.
+// m2l_fold, shift_fold) for tests/test_fold_math.py: one pair's M2L in FP64 with the output
+// orders taken in one group or split, the source row laid out by order as the kernel reads it,
+// and one shift of an M2M or an L2L.
 #include <vector>
 
 #include "fmm_sph_math.cuh"
@@ -49,6 +50,33 @@ template <int P> void pair(int split, const double* Xi, const double* Xj, const 
   }
 }
 
+// The folded M2M (up) and L2L of one shift, the outputs in one group or split at order 1 or P / 2.
+template <int P, int K0, int K1, bool UP>
+void shift_group(const double* reg, const sph::Angles<double>& a, const double* in, double* out) {
+  sph::Cx<double> A[sph::fold_idx(P, K0, K1, K1)];
+  sph::shift_fold<double, P, K0, K1, UP>(reg, a.cb, a.sb, in, A);
+  for (int k = K0; k < K1; k++)
+    for (int j = k; j < P; j++) {
+      out[2 * sph::sidx(j, k)] += A[sph::fold_idx(P, K0, k, j)].r;
+      out[2 * sph::sidx(j, k) + 1] += A[sph::fold_idx(P, K0, k, j)].i;
+    }
+}
+template <int P, bool UP>
+void shift(int split, const double* d, const double* in, double* out) {
+  double reg[sph::NT(P)];
+  const sph::Angles<double> a = sph::angles(d[0], d[1], d[2]);
+  sph::multipole_rho<double, P>(a, a.r, reg);
+  if (split == 0) {
+    shift_group<P, 0, P, UP>(reg, a, in, out);
+  } else if (split == 1) {
+    shift_group<P, 0, 1, UP>(reg, a, in, out);
+    shift_group<P, 1, P, UP>(reg, a, in, out);
+  } else {
+    shift_group<P, 0, P / 2, UP>(reg, a, in, out);
+    shift_group<P, P / 2, P, UP>(reg, a, in, out);
+  }
+}
+
 }  // namespace
 
 extern "C" int fold_m2l(int P, int split, const double* Xi, const double* Xj, const double* Mj,
@@ -59,5 +87,18 @@ extern "C" int fold_m2l(int P, int split, const double* Xi, const double* Xj, co
     return 0;                         \
   }
   CASE(4) CASE(5) CASE(6) CASE(7) CASE(8) CASE(9) CASE(10) CASE(12)
+  return 1;
+}
+
+// d: parent - child (M2M, up) or child - parent (L2L)
+extern "C" int fold_shift(int P, int up, int split, const double* d, const double* in,
+                          double* out) {
+#define SHIFT(p)                                  \
+  if (P == p) {                                   \
+    if (up) shift<p, true>(split, d, in, out);    \
+    else shift<p, false>(split, d, in, out);      \
+    return 0;                                     \
+  }
+  SHIFT(4) SHIFT(5) SHIFT(6) SHIFT(7) SHIFT(8) SHIFT(9) SHIFT(10) SHIFT(12)
   return 1;
 }
