@@ -52,7 +52,7 @@ __device__ __forceinline__ float rsqrt_ftz(float a) {
 __device__ __forceinline__ double rsqrt_ftz(double a) { return rsqrt(a); }
 
 // Most targets of a lane, and the lanes G that share one: 32 TPL / G slots for the leaf's
-// targets (64 at a time).  FP32 at the default limits g4 = 8, g2 = 16: G = 8 up to 12 bodies, 4
+// targets (64 at a time; FP32 without images: p2p_width).  FP32 at the default limits g4 = 8, g2 = 16: G = 8 up to 12 bodies, 4
 // up to 24, 2 up to 48, so slots come in steps of 4, 8 and 16 and few stay idle; FP64, whose
 // arithmetic and not its reads bounds it, takes G = 4, 2, 1 (fewer sums to merge).  So do solves
 // with periodic images, whose sums are also folded after every chunk by one warp per leaf: in
@@ -62,6 +62,16 @@ template <typename T> __device__ __forceinline__ int p2p_lanes(int nb, int g4, i
   if (sizeof(T) == 8 || images) return nb <= g4 ? 4 : nb <= g2 ? 2 : 1;
   constexpr int X = p2p_tpl<T>();
   return nb <= X * g4 / 2 ? 8 : nb <= X * g2 / 2 ? 4 : nb <= 16 * X ? 2 : 1;
+}
+
+// FP32: targets of the next pass of a leaf with `left` to go, 96 at most, and as many as fill
+// their slots (48 at G = 2, the rest by its own size, where one pass at G = 1 would hold
+// 96 slots: leaves of 65-80 bodies take 65-80 slots instead of 96; uniform tree of 250,007
+// bodies, 61 a leaf, 0.79 -> 0.70 ms).  Up to 64 bodies stay one pass: 48 and the rest apart
+// for leaves of 49-56 made the 256 solves 1 % slower.
+__device__ __forceinline__ int p2p_width(int left) {
+  constexpr int X = p2p_tpl<float>();
+  return left >= 32 * X ? 32 * X : left > 64 ? 16 * X : left;
 }
 
 constexpr int kP2PWindow = 512;  // source bodies whose indices a warp lists ahead
@@ -292,7 +302,7 @@ __device__ __forceinline__ void p2p_segment(int lane, Row<T>& row, int b0, int n
   if (pending) p2p_fold<T, COMP, TPL>(t, acc, lane);
 }
 
-// one warp's part of a target leaf: up to 64 targets from body b0 + base on
+// one warp's part of a target leaf: its targets from body b0 + base on
 struct P2PTeam {
   int base, G, s0, s1, S, p0, p1;
   int folds;  // chunks between folds
@@ -405,15 +415,19 @@ __global__ void __launch_bounds__(32 * kP2PWarps, sizeof(T) == 4 ? 2 : 3)
   if (at >= cls) return;  // the whole team
   const int4 leaf = order[first + at];
   const int b0 = leaf.x, nb = leaf.y, s0 = leaf.z, s1 = leaf.w;
-  const int G = p2p_lanes<T>(nb, g4, g2, images);
   const int ns = nsrc[first + at];
   const int per = (ns + 32 * S - 1) / (32 * S) * 32;
   const int p0 = S == 1 ? 0 : min(ns, per * seg), p1 = S == 1 ? INT_MAX : min(ns, p0 + per);
+  const int G = p2p_lanes<T>(nb, g4, g2, images);
   P2PTeam w{0, G, s0, s1, S, p0, p1, images ? 1 : G};
   const int team = wl / S, bar = 1 + team, thr = 32 * S;
-  for (int base = 0; base < nb; base += 64) {
+  for (int base = 0, width = 64; base < nb; base += width) {
+    if (sizeof(T) == 4 && !images && nb > 64) {
+      width = p2p_width(nb - base);
+      w.folds = w.G = p2p_lanes<T>(width, g4, g2, 0);
+    }
     w.base = base;
-    const int tpl = (min(64, nb - base) * G + 31) / 32;
+    const int tpl = (min(width, nb - base) * w.G + 31) / 32;
     auto run = [&](auto n) {
       p2p_targets<T, COMP, decltype(n)::value>(w, lane, rows[wl], mem[wl], b0, nb, srcs,
                                                bodies, eps2, cycle, trg_s, trg_e);
@@ -426,8 +440,7 @@ __global__ void __launch_bounds__(32 * kP2PWarps, sizeof(T) == 4 ? 2 : 3)
     if (S == 1) continue;
     // the team's warps: partial sums through shared memory, added in warp order
     asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(thr) : "memory");
-    const int t = seg * 32 + lane;
-    if (t < 64 && base + t < nb) {
+    for (int t = seg * 32 + lane; t < min(width, nb - base); t += thr) {
       vec4<T> s = mem[team * S].s[t >> 5][lane], e = make_v4<T>(0, 0, 0, 0);
       if constexpr (COMP) e = mem[team * S].e[t >> 5][lane];
       Comp<T> a[4] = {{s.x, e.x}, {s.y, e.y}, {s.z, e.z}, {s.w, e.w}};
@@ -446,7 +459,7 @@ __global__ void __launch_bounds__(32 * kP2PWarps, sizeof(T) == 4 ? 2 : 3)
       trg_s[b0 + base + t] = make_v4<T>(a[0].s, a[1].s, a[2].s, a[3].s);
       trg_e[b0 + base + t] = make_v4<T>(a[0].e, a[1].e, a[2].e, a[3].e);
     }
-    if (base + 64 < nb) asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(thr) : "memory");
+    if (base + width < nb) asm volatile("bar.sync %0, %1;" ::"r"(bar), "r"(thr) : "memory");
   }
 }
 

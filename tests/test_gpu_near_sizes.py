@@ -28,7 +28,8 @@ def pair_sums(xt, xs, qs):
 
 
 @pytest.mark.parametrize("prec", ["f32", "f64"])
-@pytest.mark.parametrize("nb", [1, 4, 5, 8, 9, 12, 13, 16, 17, 24, 25, 32, 33, 48, 49, 64, 65, 129])
+@pytest.mark.parametrize("nb", [1, 4, 5, 8, 9, 12, 13, 16, 17, 24, 25, 32, 33, 48, 49, 64, 65, 72, 80, 95, 96, 97,
+                                129, 145])
 @pytest.mark.parametrize("src", [(1,), (31, 0, 1), (33, 0, 0, 5, 64), (700, 41), (40,) * 130])
 def test_near_field_sizes(prec, nb, src):
     """One target cell against itself and source cells of the given sizes (empty ones among
