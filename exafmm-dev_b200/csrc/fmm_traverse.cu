@@ -5,16 +5,15 @@
 // otherwise splitCell (:188-212) descends into the children of the leaf-less side, of both
 // sides when NBODY_i + NBODY_j >= nspawn (TraverseRange :65-124, which for mutual = false
 // visits every child pair), or of the larger cell (ties split Ci).  The set of emitted
-// pairs depends only on each pair, so here the recursion runs breadth first: every
-// iteration classifies a frontier of pairs in parallel (count pass + write pass, exact
-// sizes, no overflow) and emits M2L pairs, P2P pairs and the next frontier.  Lists are
-// then grouped by target (per-target CSR for the M2L and P2P kernels) and sorted by source
-// within each target.
+// pairs depends only on each pair, so here a few steps breadth first make a frontier of pairs
+// (k_trav_step), whose subtrees of pairs the blocks of one kernel then walk, each with a stack
+// of its own (k_traverse).  Counts beyond a buffer's size are reported and the walk is done
+// again on larger buffers.  Lists are then grouped by target (per-target CSR for the M2L and
+// P2P kernels) and sorted by source within each target.
 #include <algorithm>
 #include <climits>
 #include <vector>
 
-#include "fmm_grid.cuh"
 #include "fmm_solver.cuh"
 
 namespace fmmb200 {
@@ -98,7 +97,7 @@ __device__ __forceinline__ void part_bounds(const int* __restrict__ range, int& 
 // children) counts and three atomics per warp.  Writes beyond a buffer's capacity are
 // skipped but every slot below it is written and all are counted, so the host can tell an
 // overflow from the counts and run the traversal again on larger buffers.
-constexpr int kTravItems = 4, kTravBlocks = 3;
+constexpr int kTravItems = 4;
 constexpr int kTravMaxSteps = 2 * (kMaxLevel + 1) + 2;
 
 template <typename T> struct TravArgs {
@@ -109,11 +108,31 @@ template <typename T> struct TravArgs {
   int nspawn, mutual, ncells;
   T cycle;
   const int* range;  // the part's bodies, or null
-  // [0] M2L, [1] P2P, [2] bad index, [5 + l] frontier size after step l; zero at the start
+  // [0] M2L, [1] P2P, [2] bad index, [3] pairs of the last frontier taken by k_traverse's
+  // blocks, [4] a stack overflowed, [5 + l] frontier size after step l; zero at the start
   unsigned long long* ctr;
   unsigned long long *m2l, *p2p;
-  int* sync;  // barrier count and fault flag, zero at the start
+  int2* stacks;  // kTravStack pairs per block of k_traverse
 };
+
+// the first n pairs that a split of p puts in its place
+__device__ __forceinline__ void trav_children(const int4* __restrict__ info, int ty, int2 p, int n,
+                                              int2* out) {
+  const int4 fi = info[p.x], fj = info[pair_cell((unsigned)p.y)];
+  const int img = (int)((unsigned)p.y & ~kCellMask);
+  if (ty == PAIR_SPLIT_SELF) {
+    int w = 0;
+    for (int a = 0; a < fi.x; a++)
+      for (int b = a; b < fi.x; b++, w++)
+        if (w < n) out[w] = make_int2(fi.y + a, fi.y + b);
+  } else if (ty == PAIR_SPLIT_I) {
+    for (int i = 0; i < n; i++) out[i] = make_int2(fi.y + i, p.y);
+  } else if (ty == PAIR_SPLIT_J) {
+    for (int j = 0; j < n; j++) out[j] = make_int2(p.x, (fj.y + j) | img);
+  } else {
+    for (int i = 0; i < n; i++) out[i] = make_int2(fi.y + i / fj.x, (fj.y + i % fj.x) | img);
+  }
+}
 
 template <typename T>
 __device__ __forceinline__ void trav_step(const TravArgs<T>& g, const vec4<T>* __restrict__ X,
@@ -217,47 +236,10 @@ __device__ __forceinline__ void trav_step(const TravArgs<T>& g, const vec4<T>* _
         // every slot below the capacity is written (the next step reads up to it)
         const unsigned long long o = bn;
         const int kw = o >= next_cap ? 0 : (int)min((unsigned long long)k[u], next_cap - o);
-        const int cj = pair_cell((unsigned)p[u].y), img = (int)((unsigned)p[u].y & ~kCellMask);
-        if (ty[u] == PAIR_SPLIT_SELF) {
-          const int c0 = info[p[u].x].y, n = info[p[u].x].x;
-          int w = 0;
-          for (int a = 0; a < n; a++)
-            for (int b = a; b < n; b++, w++)
-              if (w < kw) next[o + w] = make_int2(c0 + a, c0 + b);
-        } else if (ty[u] == PAIR_SPLIT_I) {
-          const int c0 = info[p[u].x].y;
-          for (int i = 0; i < kw; i++) next[o + i] = make_int2(c0 + i, p[u].y);
-        } else if (ty[u] == PAIR_SPLIT_J) {
-          const int c0 = info[cj].y;
-          for (int j = 0; j < kw; j++) next[o + j] = make_int2(p[u].x, (c0 + j) | img);
-        } else {
-          const int ci0 = info[p[u].x].y, cj0 = info[cj].y, nj = info[cj].x;
-          for (int i = 0; i < kw; i++)
-            next[o + i] = make_int2(ci0 + i / nj, (cj0 + i % nj) | img);
-        }
+        trav_children(info, ty[u], p[u], kw, next + o);
         bn += k[u];
       }
     }
-  }
-}
-
-// All steps in one cooperative launch: a barrier between them, the frontiers taking turns in
-// two buffers, until a frontier is empty or larger than its buffer.
-template <typename T>
-__global__ void __launch_bounds__(256, kTravBlocks) k_traverse(TravArgs<T> g) {
-  GridBarrier bar{(unsigned*)&g.sync[0], &g.sync[1], 0};
-  int b0, b1;
-  part_bounds(g.range, b0, b1);
-  unsigned long long n = g.nfront0;
-  int2 *front = g.front, *next = g.front2;
-  for (int l = 0; l < kTravMaxSteps; l++) {
-    trav_step<T>(g, g.X, g.info, front, (long long)n, next, &g.ctr[5 + l], b0, b1);
-    if (!bar.sync()) return;
-    n = *(volatile unsigned long long*)&g.ctr[5 + l];
-    if (n == 0 || n > g.front_cap) return;
-    int2* const t = front;
-    front = next;
-    next = t;
   }
 }
 
@@ -269,6 +251,120 @@ __global__ void __launch_bounds__(256) k_trav_step(TravArgs<T> g, int l) {
   const unsigned long long n = l == 0 ? g.nfront0 : min(g.ctr[4 + l], g.front_cap);
   trav_step<T>(g, g.X, g.info, (l & 1) ? g.front2 : g.front, (long long)n,
                (l & 1) ? g.front : g.front2, &g.ctr[5 + l], b0, b1);
+}
+
+// The pairs below the frontier that l0 steps left.  A block takes pairs of the frontier a few
+// at a time and walks all that comes of them: up to kTravThreads pairs from the top of its
+// stack per round, one per thread, whose children go back on the stack and whose M2L and P2P
+// pairs go through shared memory to the lists a few hundred at a time.  No block waits for
+// another, and neither list's counter is touched once a warp: a launch per step cost 5-6 us
+// however few pairs it had, and on large trees its atomics (three per 128 pairs on three
+// addresses) and its frontiers' passage through memory.
+constexpr int kTravThreads = 128, kTravBlocks = 8;  // per block; blocks per SM
+constexpr int kTravBuf = 512;     // pairs of either list that a block holds back
+constexpr int kTravStack = 4096;  // pairs
+
+template <typename T>
+__global__ void __launch_bounds__(kTravThreads, kTravBlocks) k_traverse(TravArgs<T> g, int l0) {
+  __shared__ unsigned long long mbuf[kTravBuf], pbuf[kTravBuf], mat, pat, taken;
+  __shared__ int nm, np, kids[2];
+  const int tid = threadIdx.x, lane = lane_id();
+  int b0, b1;
+  part_bounds(g.range, b0, b1);
+  const int2* front = (l0 & 1) ? g.front2 : g.front;
+  const unsigned long long n = l0 == 0 ? g.nfront0 : min(g.ctr[4 + l0], g.front_cap);
+  // pairs taken at a time: few enough that every block comes to the frontier several times
+  const int chunk =
+      (int)min(n / (4 * gridDim.x) + 4, (unsigned long long)kTravThreads);
+  int2* stack = g.stacks + (size_t)blockIdx.x * kTravStack;
+  if (tid == 0) nm = np = kids[0] = kids[1] = 0;
+  auto flush = [&](int cm, int cp) {
+    __syncthreads();  // (all have read the counts)
+    if (tid == 0) {
+      mat = cm ? atomicAdd(&g.ctr[0], (unsigned long long)cm) : 0;
+      nm = 0;
+    }
+    if (tid == 32) {
+      pat = cp ? atomicAdd(&g.ctr[1], (unsigned long long)cp) : 0;
+      np = 0;
+    }
+    __syncthreads();
+    for (int i = tid; i < cm; i += kTravThreads)
+      if (mat + i < g.m2l_cap) g.m2l[mat + i] = mbuf[i];
+    for (int i = tid; i < cp; i += kTravThreads)
+      if (pat + i < g.p2p_cap) g.p2p[pat + i] = pbuf[i];
+  };
+  int top = 0;
+  bool more = true;
+  for (int it = 0;; it++) {
+    __syncthreads();
+    top = min(top + kids[(it + 1) & 1], kTravStack);
+    const int cm = nm, cp = np;
+    if (max(cm, cp) > kTravBuf - 2 * kTravThreads) flush(cm, cp);
+    int got = 0;
+    unsigned long long from = 0;
+    if (top < kTravThreads && more) {
+      const int want = min(chunk, kTravThreads - top);
+      if (tid == 0) taken = atomicAdd(&g.ctr[3], (unsigned long long)want);
+      __syncthreads();
+      from = taken;
+      got = from < n ? (int)min((unsigned long long)want, n - from) : 0;
+      more = from + want < n;
+    }
+    const int own = min(top, kTravThreads);
+    if (own + got == 0) {
+      if (max(cm, cp) <= kTravBuf - 2 * kTravThreads) flush(cm, cp);
+      return;
+    }
+    int2 p = make_int2(0, 0);
+    int ty = -1, k = 0;
+    if (tid < own + got) {
+      p = tid < own ? stack[top - 1 - tid] : front[from + (tid - own)];
+      const int cj = pair_cell((unsigned)p.y);
+      if ((unsigned)p.x < (unsigned)g.ncells && (unsigned)cj < (unsigned)g.ncells &&
+          pair_img((unsigned)p.y) < 27)
+        ty = classify_data<T>(p.x, p.y, g.X[p.x], g.X[cj], g.info[p.x], g.info[cj], g.nspawn,
+                              g.cycle, g.mutual, b0, b1, &k);
+      else
+        atomicOr(&g.ctr[2], 1ULL);  // never expected: reported to the host, pair skipped
+    }
+    top -= own;
+    // M2L in bits 0-7, P2P in 8-15, children in 16-31 (warp totals: <= 64, <= 64, <= 2048)
+    const unsigned v = ty == PAIR_M2L ? (unsigned)k
+                       : ty == PAIR_P2P ? (unsigned)k << 8
+                       : ty >= PAIR_SPLIT_I ? (unsigned)k << 16 : 0u;
+    unsigned incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned x = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += x;
+    }
+    __syncthreads();  // every thread has its pair
+    if (tid == 0) kids[(it + 1) & 1] = 0;
+    int bm = 0, bp = 0, bn = 0;
+    if (lane == 31) {
+      if (incl & 0xffu) bm = atomicAdd(&nm, (int)(incl & 0xffu));
+      if ((incl >> 8) & 0xffu) bp = atomicAdd(&np, (int)((incl >> 8) & 0xffu));
+      if (incl >> 16) bn = atomicAdd(&kids[it & 1], (int)(incl >> 16));
+    }
+    const unsigned excl = incl - v;
+    bm = __shfl_sync(0xffffffffu, bm, 31) + (int)(excl & 0xffu);
+    bp = __shfl_sync(0xffffffffu, bp, 31) + (int)((excl >> 8) & 0xffu);
+    bn = __shfl_sync(0xffffffffu, bn, 31) + (int)(excl >> 16) + top;
+    const unsigned long long packed = (unsigned long long)(unsigned)p.x << 32 | (unsigned)p.y;
+    const unsigned long long rev = (unsigned long long)(unsigned)p.y << 32 | (unsigned)p.x;
+    if (ty == PAIR_M2L) {
+      mbuf[bm] = packed;
+      if (k == 2) mbuf[bm + 1] = rev;
+    } else if (ty == PAIR_P2P) {
+      pbuf[bp] = packed;
+      if (k == 2) pbuf[bp + 1] = rev;
+    } else if (ty >= PAIR_SPLIT_I) {
+      const int room = min(k, kTravStack - bn);
+      if (room < k) g.ctr[4] = 1;
+      trav_children(g.info, ty, p, room, stack + bn);
+    }
+  }
 }
 
 // ---------------------------------------------------------------- grouping by target
@@ -582,31 +678,34 @@ template <typename T> static void upload_roots(Solver<T>& s) {
 }
 
 // The traversal on the handle's buffers, run again on larger ones while any was too small (the
-// buffers start from typical list lengths per cell).  Trees of up to kTravCoopCells cells, and
-// a handle's first one, run in one launch; larger ones as a launch per step, as many as the
-// last traversal took, two more per level that the tree has grown by since, and two to spare.
-// The one launch saves the 5-6 us that each small step costs (1,000 bodies 0.21 -> 0.18 ms,
-// uniform 250,007 0.30 -> 0.26 ms), but its blocks stay on every SM until it ends and keep the
-// upward expansions, which run beside the steps, waiting: Plummer 2^20 (64,000 cells) 0.97 ms
-// by steps, 1.10 ms in one launch.
-constexpr int kTravCoopCells = 8192;
+// buffers start from typical list lengths per cell).  Trees of up to kTravStackCells cells: steps
+// until the frontier is some four times as long as there are cells (a step makes about 20 pairs
+// of one; from a frontier a quarter as long the blocks' shares differ by far more: 30,003 bodies
+// in images 0.37 ms against 0.26), then k_traverse; should one of its stacks overflow, this and
+// the handle's later traversals take steps only.  Larger trees: steps only, as many as the last
+// traversal took, two more per level that the tree has grown by since, and two to spare (at
+// first as many as any tree needs).  Against all steps in one cooperative kernel with a barrier
+// between them the traverse phase of 1,000 bodies takes 0.16 instead of 0.19 ms, of 200,003 0.26
+// instead of 0.31, of 250,007 in the uniform tree 0.25 instead of 0.27; 2^20 bodies (64,000
+// cells) take 0.90 ms by steps and 1.03 in k_traverse, whose blocks end far apart there.
+constexpr int kTravStackCells = 8192;
 
 template <typename T>
 static void traverse_lists(Solver<T>& s, long long& nm2l, long long& np2p) {
   unsigned long long* ctr = (unsigned long long*)s.scal.p + 32;
   unsigned long long* hctr = (unsigned long long*)s.scal_host + 32;
-  constexpr int NC = kTravMaxSteps + 8;
-  int* sync = (int*)(ctr + NC);
+  constexpr int NC = kTravMaxSteps + 5;
   size_t m2l = 96 * (size_t)s.ncells + 1024, p2p = 24 * (size_t)s.ncells + 1024,
          front = 64 * (size_t)s.ncells + 1024;
-  bool coop = s.ncells <= kTravCoopCells || s.trav_steps == 0;
+  bool stacks = s.ncells <= kTravStackCells && !s.trav_by_steps, all = false;
+  const int blocks = std::max(16, std::min(148 * kTravBlocks, s.ncells / 2));
   for (;;) {
     s.m2l.ensure(m2l);
     s.p2p.ensure(p2p);
     s.front.ensure(front);
     s.front2.ensure(front);
     upload_roots(s);
-    FMM_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * (NC + 1), s.stream));
+    FMM_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * NC, s.stream));
     TravArgs<T> g{};
     g.front = s.front.p;
     g.front2 = s.front2.p;
@@ -624,49 +723,54 @@ static void traverse_lists(Solver<T>& s, long long& nm2l, long long& np2p) {
     g.ctr = ctr;
     g.m2l = s.m2l.p;
     g.p2p = s.p2p.p;
-    g.sync = sync;
     int steps = kTravMaxSteps;
-    if (coop) {
-      // fewer blocks make cheaper barriers: a thread for every sixteenth of a cell's pairs
-      const int blocks = std::max(8, std::min(148 * kTravBlocks, s.ncells / 16));
-      void* args[] = {&g};
-      FMM_CUDA(cudaLaunchCooperativeKernel((const void*)k_traverse<T>, dim3(blocks), dim3(256),
-                                           args, 0, s.stream));
-      FMM_LAUNCH_CHECK();
-    } else {
+    if (stacks) {
+      steps = 0;
+      for (long long e = std::max(s.nfront0, 1); e < 4LL * s.ncells; e *= 20) steps++;
+    } else if (s.trav_steps > 0 && !all) {
       steps = std::min(steps, s.trav_steps + 2 * std::max(0, s.maxlevel - s.trav_maxlevel) + 2);
-      for (int l = 0; l < steps; l++) {
-        k_trav_step<T><<<148 * 8, 256, 0, s.stream>>>(g, l);
-        FMM_LAUNCH_CHECK();
-      }
     }
-    FMM_CUDA(cudaMemcpyAsync(hctr, ctr, sizeof(unsigned long long) * (NC + 1),
-                             cudaMemcpyDeviceToHost, s.stream));
+    for (int l = 0; l < steps; l++) {
+      k_trav_step<T><<<std::min(148 * 8, std::max(1, s.ncells / 8)), 256, 0, s.stream>>>(g, l);
+      FMM_LAUNCH_CHECK();
+    }
+    if (stacks) {
+      s.trav_stacks.ensure((size_t)blocks * kTravStack);
+      g.stacks = s.trav_stacks.p;
+      k_traverse<T><<<blocks, kTravThreads, 0, s.stream>>>(g, steps);
+      FMM_LAUNCH_CHECK();
+    }
+    FMM_CUDA(cudaMemcpyAsync(hctr, ctr, sizeof(unsigned long long) * NC, cudaMemcpyDeviceToHost,
+                             s.stream));
     FMM_CUDA(cudaStreamSynchronize(s.stream));
-    if (((int*)(hctr + NC))[1])
-      throw FmmError(FMM_ERR_DEVICE, "the traversal's blocks lost one another");
     if (hctr[2]) throw FmmError(FMM_ERR_DEVICE, "traversal read a cell index out of range");
     bool fits = hctr[0] <= s.m2l.cap && hctr[1] <= s.p2p.cap;
     m2l = std::max<size_t>(s.m2l.cap, hctr[0]);  // (exact counts, or those up to the overflow)
     p2p = std::max<size_t>(s.p2p.cap, hctr[1]);
     front = g.front_cap;
     int used = 0;  // steps with pairs to classify
-    for (int l = 0; l < kTravMaxSteps; l++) {
+    for (int l = 0; l < steps; l++) {
       if (hctr[5 + l]) used = l + 2;
       if (hctr[5 + l] > g.front_cap) {
         fits = false;
         front = std::max<size_t>(2 * front, hctr[5 + l]);
       }
     }
-    if (hctr[5 + steps - 1]) {  // more steps than planned (the deepest pair takes fewer than all)
+    if (hctr[4]) {
+      fits = stacks = false;
+      s.trav_by_steps = true;
+    }
+    if (!stacks && hctr[4 + steps]) {  // more steps than planned
       fits = false;
-      coop = true;
+      all = true;
     }
     if (fits) {
+      if (!stacks) {
+        s.trav_steps = std::max(used, 1);
+        s.trav_maxlevel = s.maxlevel;
+      }
       nm2l = (long long)hctr[0];
       np2p = (long long)hctr[1];
-      s.trav_steps = std::max(used, 1);
-      s.trav_maxlevel = s.maxlevel;
       return;
     }
   }

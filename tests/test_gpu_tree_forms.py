@@ -1,6 +1,6 @@
 """The tree kernel at the sizes where it takes another form: leaves a warp ranks with two or four
 bodies per lane, or leaves to the sorts; node arrays that overflow; a tree deeper than the
-handle's last one; and the traversal in one launch and by steps.  Trees bit for bit the
+handle's last one; and the traversal with stacks and by steps.  Trees bit for bit the
 oracle's, radii of a whole solve bit for bit those of the stages, lists equal in both forms."""
 import importlib
 
@@ -70,8 +70,8 @@ def test_tree_forms(prec, ncrit):
 
 
 def test_traversal_forms():
-    """More cells than the one-launch traversal takes: the first solve of a handle runs it all the
-    same, the later ones by steps, after other bodies too."""
+    """More cells than the traversal with stacks takes: a handle's first solve by all steps, the
+    later ones by as many as the last took, with stacks in between."""
     rng = np.random.default_rng(3)
     s = fmm.Solver(P=4, theta=0.5, ncrit=16, use_ropt=0)
     first = {}
@@ -87,3 +87,24 @@ def test_traversal_forms():
                 assert n < 1000 or alone.num_cells()[0] > 8192
             for a, b in zip(lists, first[n]):
                 assert np.array_equal(a, b), (rep, kind)
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+def test_traversal_stack_overflow(prec):
+    """Eight distant clumps that no pair of cells is far from at this theta: the frontier stays at
+    64 pairs down to the clumps, then every pair becomes 64, more than a block's stack holds."""
+    rng = np.random.default_rng(8)
+    corner = np.array([[i & 1, i >> 1 & 1, i >> 2] for i in range(8)]) - 0.5
+    x = np.concatenate([c + rng.uniform(-1, 1, (768, 3)) * 5e-4 for c in corner])
+    q = rng.uniform(0.5, 1, len(x))
+    s = fmm.Solver(P=4, theta=1e-5, ncrit=16, precision=prec, use_ropt=0, nspawn=1)
+    y, w = bodies("cube", 500, rng, prec)
+    for rep in range(2):
+        s.solve(x, q)
+        c = s.cells()
+        leaves = np.flatnonzero(c["nchild"] == 0)
+        m2l, p2p = s.lists()
+        assert len(m2l) == 0
+        ref = (leaves[:, None].astype(np.uint64) << np.uint64(32) | leaves.astype(np.uint64)).ravel()
+        assert np.array_equal(p2p, ref)
+        s.solve(y, w)
