@@ -379,9 +379,25 @@ constexpr int kSegWarpCap = 1024;   // keys one warp sorts in its registers
 constexpr int kSegBlockCap = 8192;  // keys one block sorts; longer ranges: global sort
 constexpr int kSegWarps = 8;
 constexpr int kSegBlock = 512;
+constexpr int kSegBothCells = 2048;  // trees whose two lists are grouped together
 
-__global__ void k_seg_count(const unsigned long long* __restrict__ pairs, long long n,
-                            int* __restrict__ cnt) {
+struct SegList {
+  unsigned long long* pairs;
+  long long n;
+  int *cnt, *off;      // counts per target (zeros at the start), CSR offsets
+  unsigned* keys;      // n keys of scratch
+  int* overflow;       // set if a range is too long for k_seg_sort_block
+};
+struct SegLists {
+  SegList l[2];
+  __device__ __forceinline__ SegList at(int k) const { return k ? l[1] : l[0]; }
+};
+// (blockIdx.y: the list)
+
+__global__ void k_seg_count(SegLists g) {
+  const unsigned long long* __restrict__ pairs = g.at(blockIdx.y).pairs;
+  const long long n = g.at(blockIdx.y).n;
+  int* __restrict__ cnt = g.at(blockIdx.y).cnt;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long t0 = blockIdx.x * (long long)blockDim.x; t0 < n; t0 += stride) {
     const long long t = t0 + threadIdx.x;
@@ -395,9 +411,12 @@ __global__ void k_seg_count(const unsigned long long* __restrict__ pairs, long l
 
 // cnt holds the counts on entry and zeros on exit; each warp's pairs of one target take
 // consecutive slots from the top of the target's remaining range
-__global__ void k_seg_scatter(const unsigned long long* __restrict__ pairs, long long n,
-                              const int* __restrict__ off, int* __restrict__ cnt, int b,
-                              unsigned* __restrict__ keys) {
+__global__ void k_seg_scatter(SegLists g, int b) {
+  const unsigned long long* __restrict__ pairs = g.at(blockIdx.y).pairs;
+  const long long n = g.at(blockIdx.y).n;
+  const int* __restrict__ off = g.at(blockIdx.y).off;
+  int* __restrict__ cnt = g.at(blockIdx.y).cnt;
+  unsigned* __restrict__ keys = g.at(blockIdx.y).keys;
   const long long stride = (long long)gridDim.x * blockDim.x;
   const int lane = lane_id();
   for (long long t0 = blockIdx.x * (long long)blockDim.x; t0 < n; t0 += stride) {
@@ -486,8 +505,10 @@ __device__ __forceinline__ void warp_sort_range(const unsigned* __restrict__ key
 
 // one warp per target with at most kSegWarpCap pairs
 __global__ void __launch_bounds__(32 * kSegWarps, 5)
-    k_seg_sort_warp(int ncells, const int* __restrict__ off, const unsigned* __restrict__ keys,
-                    int b, unsigned long long* __restrict__ out) {
+    k_seg_sort_warp(int ncells, SegLists g, int b) {
+  const int* __restrict__ off = g.at(blockIdx.y).off;
+  const unsigned* __restrict__ keys = g.at(blockIdx.y).keys;
+  unsigned long long* __restrict__ out = g.at(blockIdx.y).pairs;
   const int c = blockIdx.x * kSegWarps + (threadIdx.x >> 5);
   if (c >= ncells) return;
   const int s0 = off[c], n = off[c + 1] - s0;
@@ -505,8 +526,11 @@ __global__ void __launch_bounds__(32 * kSegWarps, 5)
 // the longer ranges, one block at a time; a range above kSegBlockCap is written unsorted and
 // flagged for the global sort
 __global__ void __launch_bounds__(kSegBlock)
-    k_seg_sort_block(int ncells, const int* __restrict__ off, const unsigned* __restrict__ keys,
-                     int b, unsigned long long* __restrict__ out, int* __restrict__ overflow) {
+    k_seg_sort_block(int ncells, SegLists g, int b) {
+  const int* __restrict__ off = g.at(blockIdx.y).off;
+  const unsigned* __restrict__ keys = g.at(blockIdx.y).keys;
+  unsigned long long* __restrict__ out = g.at(blockIdx.y).pairs;
+  int* __restrict__ overflow = g.at(blockIdx.y).overflow;
   __shared__ unsigned a[kSegBlockCap];
   __shared__ int todo[kSegBlock];
   __shared__ int ntodo;
@@ -546,6 +570,10 @@ __global__ void __launch_bounds__(kSegBlock)
 // atomics, which saves the sort's launches, the Cartesian M2L of 2^22 bodies took 0.87 ms
 // instead of 0.79, the spherical one of 2^20 1.50 ms instead of 1.47.
 constexpr int kTgtKeyBits = 8, kTgtKeyMax = (1 << kTgtKeyBits) - 1;
+__device__ __forceinline__ unsigned tgt_key(int n, int shift) {
+  const int b = (n + (1 << shift) - 1) >> shift;
+  return n ? (unsigned)(kTgtKeyMax - 1 - min(kTgtKeyMax - 1, b)) : (unsigned)kTgtKeyMax;
+}
 __global__ void k_m2l_targets(int ncells, const int* __restrict__ off, int shift,
                               unsigned* __restrict__ key, int* __restrict__ cell,
                               int* __restrict__ count) {
@@ -554,9 +582,48 @@ __global__ void k_m2l_targets(int ncells, const int* __restrict__ off, int shift
   const unsigned m = __ballot_sync(0xffffffffu, n > 0);
   if (m && lane_id() == 0) atomicAdd(count, __popc(m));
   if (c >= ncells) return;
-  const int b = (n + (1 << shift) - 1) >> shift;
-  key[c] = n ? (unsigned)(kTgtKeyMax - 1 - min(kTgtKeyMax - 1, b)) : (unsigned)kTgtKeyMax;
+  key[c] = tgt_key(n, shift);
   cell[c] = c;
+}
+
+// Small trees: the offsets of both lists by a block each, and the M2L list's target keys as
+// k_m2l_targets writes them.
+constexpr int kScanThreads = 1024;
+__global__ void __launch_bounds__(kScanThreads)
+    k_seg_scan(int ncells, SegLists g, int shift, unsigned* __restrict__ key,
+               int* __restrict__ cell, int* __restrict__ count) {
+  __shared__ int wsum[kScanThreads / 32];
+  const int* __restrict__ cnt = g.at(blockIdx.x).cnt;
+  int* __restrict__ off = g.at(blockIdx.x).off;
+  const int lane = lane_id(), wl = threadIdx.x >> 5;
+  const int per = (ncells + kScanThreads) / kScanThreads;  // of ncells + 1 offsets
+  const int lo = min(ncells + 1, (int)threadIdx.x * per), hi = min(ncells + 1, lo + per);
+  int sum = 0, used = 0;
+  for (int i = lo; i < hi; i++) {
+    const int n = cnt[i];
+    sum += n;
+    if (blockIdx.x == 0 && i < ncells) {
+      used += n > 0;
+      key[i] = tgt_key(n, shift);
+      cell[i] = i;
+    }
+  }
+  int incl = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += u;
+  }
+  if (lane == 31) wsum[wl] = incl;
+  used = __reduce_add_sync(0xffffffffu, used);
+  if (lane == 0 && used) atomicAdd(count, used);
+  __syncthreads();
+  int run = incl - sum;
+  for (int k = 0; k < wl; k++) run += wsum[k];
+  for (int i = lo; i < hi; i++) {
+    off[i] = run;
+    run += cnt[i];
+  }
 }
 
 // body-pair count of the P2P list: sum over pairs of nbody(target) * nbody(source)
@@ -598,29 +665,35 @@ static int bits_for(int n) {
   return b;
 }
 
-// group a list by target (k_seg_*): CSR offsets into off[0, ncells], pairs sorted within
-// each target's range
-// scratch: segcnt (ncells + 1 ints), keys (n), tmp (CUB scan scratch, or s.cub_tmp if null)
-static void group_by_target(SolverBase& s, unsigned long long* lst, long long n, int b,
-                            int* off, int* overflow, int* segcnt, unsigned* keys,
-                            DevArr<char>* tmp) {
+// group a list, or both, by target (k_seg_*): CSR offsets into off[0, ncells], pairs sorted
+// within each target's range; `scan`: the counts into the offsets
+template <typename F>
+static void group_by_target(SolverBase& s, const SegLists& g, int lists, int b, F&& scan) {
   const int TB = 256;
-  FMM_CUDA(cudaMemsetAsync(segcnt, 0, (s.ncells + 1) * sizeof(int), s.stream));
-  const int grid = (int)std::max(1LL, std::min<long long>(ceil_div(n, TB), 148 * 16));
+  const long long n = lists == 1 ? g.l[0].n : std::max(g.l[0].n, g.l[1].n);
+  const dim3 grid((int)std::max(1LL, std::min<long long>(ceil_div(n, TB), 148 * 16)), lists);
   if (n > 0) {
-    k_seg_count<<<grid, TB, 0, s.stream>>>(lst, n, segcnt);
+    k_seg_count<<<grid, TB, 0, s.stream>>>(g);
     FMM_LAUNCH_CHECK();
   }
-  exclusive_sum_int(s, segcnt, off, s.ncells + 1, tmp);
+  scan();
   if (n == 0) return;
-  k_seg_scatter<<<grid, TB, 0, s.stream>>>(lst, n, off, segcnt, b, keys);
+  k_seg_scatter<<<grid, TB, 0, s.stream>>>(g, b);
   FMM_LAUNCH_CHECK();
-  k_seg_sort_warp<<<ceil_div(s.ncells, kSegWarps), 32 * kSegWarps, 0, s.stream>>>(s.ncells, off,
-                                                                                 keys, b, lst);
+  k_seg_sort_warp<<<dim3(ceil_div(s.ncells, kSegWarps), lists), 32 * kSegWarps, 0, s.stream>>>(
+      s.ncells, g, b);
   FMM_LAUNCH_CHECK();
-  k_seg_sort_block<<<std::min(ceil_div(s.ncells, kSegBlock), 148), kSegBlock, 0, s.stream>>>(
-      s.ncells, off, keys, b, lst, overflow);
+  // (a target has a pair per cell and image at most)
+  if ((long long)s.ncells * (s.cfg.images > 0 ? 27 : 1) <= kSegWarpCap) return;
+  k_seg_sort_block<<<dim3(std::min(ceil_div(s.ncells, kSegBlock), 148), lists), kSegBlock, 0,
+                     s.stream>>>(s.ncells, g, b);
   FMM_LAUNCH_CHECK();
+}
+// one list; scratch for the counts' scan: tmp, or s.cub_tmp if null
+static void group_one(SolverBase& s, const SegList& l, int b, DevArr<char>* tmp) {
+  FMM_CUDA(cudaMemsetAsync(l.cnt, 0, (s.ncells + 1) * sizeof(int), s.stream));
+  group_by_target(s, SegLists{{l, l}}, 1, b,
+                  [&] { exclusive_sum_int(s, l.cnt, l.off, s.ncells + 1, tmp); });
 }
 
 // a whole list sorted on (target << (b + ib) | image << b | source), 2 b + ib key bits:
@@ -813,25 +886,50 @@ template <typename T> void build_lists(Solver<T>& s, bool defer_p2p) {
   s.list_tmp.ensure(std::max<long long>(std::max(nm2l, np2p), 1));
   s.m2l_off.ensure(s.ncells + 1);
   s.p2p_off.ensure(s.ncells + 1);
-  s.seg_cnt.ensure(s.ncells + 1);
+  s.m2l_tgt.ensure(s.ncells);
+  s.tgt_key.ensure(2 * (size_t)s.ncells);
+  s.idx.ensure(s.ncells);
+  int* ntgt = (int*)(cnt + 4);
   int* overflow = (int*)(cnt + 5);  // per list: a target range too long for the blocks
-  FMM_CUDA(cudaMemsetAsync(overflow, 0, 2 * sizeof(int), s.stream));
-  group_by_target(s, s.m2l.p, nm2l, b, s.m2l_off.p, overflow, s.seg_cnt.p,
-                  (unsigned*)s.list_tmp.p, nullptr);
-  s.p2p_pending = defer_p2p && s.side != nullptr;
+  const int shift = s.cfg.basis == FMM_SPHERICAL ? 5 : 0;
+  FMM_CUDA(cudaMemsetAsync(cnt + 4, 0, 2 * sizeof(unsigned long long), s.stream));
+  // Small trees: both lists by the same launches, one after the other with the P2P order on the
+  // main stream.  Their kernels take 2-10 us, about what the host needs to queue them: 14
+  // launches and copies instead of 33 take 1,000 bodies from 0.49 to 0.44 ms, 16,384 in FP64
+  // from 0.66 to 0.61 (118 and 585 cells).  Larger ones group the P2P list beside the M2L:
+  // at 5,137 cells 1.60 ms against 1.63 together.
+  const bool both = s.ncells <= kSegBothCells;
+  s.seg_cnt.ensure((both ? 2 : 1) * (size_t)(s.ncells + 1));
+  const SegList lm{s.m2l.p, nm2l, s.seg_cnt.p, s.m2l_off.p, (unsigned*)s.list_tmp.p, overflow};
+  SegList lp{s.p2p.p, np2p, s.seg_cnt.p, s.p2p_off.p, (unsigned*)s.list_tmp.p, overflow + 1};
+  s.p2p_pending = !both && defer_p2p && s.side != nullptr;
+  if (both) {
+    lp.cnt += s.ncells + 1;
+    lp.keys += nm2l;
+    const SegLists g{{lm, lp}};
+    FMM_CUDA(cudaMemsetAsync(s.seg_cnt.p, 0, 2 * (size_t)(s.ncells + 1) * sizeof(int), s.stream));
+    group_by_target(s, g, 2, b, [&] {
+      k_seg_scan<<<2, kScanThreads, 0, s.stream>>>(s.ncells, g, shift, s.tgt_key.p, s.idx.p, ntgt);
+      FMM_LAUNCH_CHECK();
+    });
+    order_p2p_targets(s);
+  } else {
+    group_one(s, lm, b, nullptr);
+  }
   if (s.p2p_pending) {
     // the P2P list is grouped on the side stream with scratch of its own, beside M2L; its
     // overflow flag reaches the host through the pinned mirror (finish_p2p_list)
     s.seg_cnt2.ensure(s.ncells + 1);
     s.seg_keys2.ensure(std::max<long long>(np2p, 1));
+    lp.cnt = s.seg_cnt2.p;
+    lp.keys = s.seg_keys2.p;
     if (!s.p2p_ready) FMM_CUDA(cudaEventCreateWithFlags(&s.p2p_ready, cudaEventDisableTiming));
     FMM_CUDA(cudaEventRecord(s.fork, s.stream));
     FMM_CUDA(cudaStreamWaitEvent(s.side, s.fork, 0));
     cudaStream_t main = s.stream;
     s.stream = s.side;
     try {
-      group_by_target(s, s.p2p.p, np2p, b, s.p2p_off.p, overflow + 1, s.seg_cnt2.p,
-                      s.seg_keys2.p, &s.cub_tmp2);
+      group_one(s, lp, b, &s.cub_tmp2);
       order_p2p_targets(s);
       FMM_CUDA(cudaMemcpyAsync((int*)(hc + 5) + 1, overflow + 1, sizeof(int),
                                cudaMemcpyDeviceToHost, s.stream));
@@ -841,30 +939,22 @@ template <typename T> void build_lists(Solver<T>& s, bool defer_p2p) {
       throw;
     }
     s.stream = main;
-  } else {
-    group_by_target(s, s.p2p.p, np2p, b, s.p2p_off.p, overflow + 1, s.seg_cnt.p,
-                    (unsigned*)s.list_tmp.p, nullptr);
+  } else if (!both) {
+    group_one(s, lp, b, nullptr);
     order_p2p_targets(s);
   }
   // M2L target order: by descending pair count in buckets (stable in cell index)
-  {
-    int* ntgt = (int*)(cnt + 4);
-    s.m2l_tgt.ensure(s.ncells);
-    s.tgt_key.ensure(2 * (size_t)s.ncells);
-    s.idx.ensure(s.ncells);
-    FMM_CUDA(cudaMemsetAsync(ntgt, 0, sizeof(int), s.stream));
-    k_m2l_targets<<<ceil_div(s.ncells, TB), TB, 0, s.stream>>>(
-        s.ncells, s.m2l_off.p, s.cfg.basis == FMM_SPHERICAL ? 5 : 0, s.tgt_key.p, s.idx.p, ntgt);
+  if (!both) {
+    k_m2l_targets<<<ceil_div(s.ncells, TB), TB, 0, s.stream>>>(s.ncells, s.m2l_off.p, shift,
+                                                               s.tgt_key.p, s.idx.p, ntgt);
     FMM_LAUNCH_CHECK();
-    sort_pairs_u32(s, s.tgt_key.p, s.tgt_key.p + s.ncells, s.idx.p, s.m2l_tgt.p, s.ncells,
-                   kTgtKeyBits);
-    FMM_CUDA(cudaMemcpyAsync(s.scal_host + 12, ntgt, sizeof(int), cudaMemcpyDeviceToHost, s.stream));
   }
-  FMM_CUDA(cudaMemcpyAsync(hc + 3, cnt + 3, 2 * sizeof(unsigned long long) + sizeof(int),
+  sort_pairs_u32(s, s.tgt_key.p, s.tgt_key.p + s.ncells, s.idx.p, s.m2l_tgt.p, s.ncells,
+                 kTgtKeyBits);
+  // body pairs, targets and the overflow flags (the P2P list's on its own while it is pending)
+  FMM_CUDA(cudaMemcpyAsync(hc + 3, cnt + 3,
+                           2 * sizeof(unsigned long long) + (s.p2p_pending ? 1 : 2) * sizeof(int),
                            cudaMemcpyDeviceToHost, s.stream));
-  if (!s.p2p_pending)
-    FMM_CUDA(cudaMemcpyAsync((int*)(hc + 5) + 1, overflow + 1, sizeof(int),
-                             cudaMemcpyDeviceToHost, s.stream));
   FMM_CUDA(cudaStreamSynchronize(s.stream));
   const int* hflow = (const int*)(hc + 5);
   if (hflow[0] || (!s.p2p_pending && hflow[1])) {
@@ -876,7 +966,7 @@ template <typename T> void build_lists(Solver<T>& s, bool defer_p2p) {
     FMM_CUDA(cudaStreamSynchronize(s.stream));
   }
   s.p2p_body_pairs = -1;  // counted when asked for (count_p2p_body_pairs)
-  s.m2l_ntgt = s.scal_host[12];
+  s.m2l_ntgt = *(const int*)(hc + 4);
 }
 
 // the body pairs of the P2P list, for the statistics (not needed by the solve itself)

@@ -108,3 +108,21 @@ def test_traversal_stack_overflow(prec):
         ref = (leaves[:, None].astype(np.uint64) << np.uint64(32) | leaves.astype(np.uint64)).ravel()
         assert np.array_equal(p2p, ref)
         s.solve(y, w)
+
+
+@pytest.mark.parametrize("n", [300, 1000, 6000])
+def test_small_tree_grouping(n):
+    """Both lists of a small tree grouped together, with images and at a theta that no pair of
+    cells is far at: every leaf against every leaf in 27 images, from 200 to 14,000 sources a
+    target (a warp's, a block's and the global sort)."""
+    x, q = bodies("cube", n, np.random.default_rng(n), "f32")
+    s = fmm.Solver(P=4, theta=1e-5, ncrit=32, images=1, cycle=2.0, use_ropt=0)
+    s.solve(x, q)
+    c = s.cells()
+    assert len(c["nchild"]) <= 2048
+    leaves = np.flatnonzero(c["nchild"] == 0)
+    m2l, p2p = s.lists()
+    assert len(m2l) == 0
+    img = np.arange(27, dtype=np.int64)
+    ref = leaves[:, None, None] << 32 | img[None, :, None] << 27 | leaves[None, None, :]
+    assert np.array_equal(p2p, ref.ravel())
