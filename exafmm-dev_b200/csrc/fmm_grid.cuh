@@ -1,20 +1,27 @@
-// A barrier of all blocks of a cooperative launch (cudaLaunchCooperativeKernel: every block
-// resident), for the kernels that run many small dependent steps.
+// A barrier of all blocks of a launch whose blocks are resident together, for the kernels that
+// run many small dependent steps: a cooperative launch (cudaLaunchCooperativeKernel), or a launch
+// of one thread-block cluster.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace fmmb200 {
 
-// The barrier counts arrivals up; a block that waits longer than kSyncSpins polls (seconds)
-// sets *fault and every block leaves at its next barrier.
+// The barrier of a cooperative launch counts arrivals up; a block that waits longer than
+// kSyncSpins polls (seconds) sets *fault and every block leaves at its next barrier.  One
+// cluster's is the hardware's (0.3 us instead of 1.5-2).
 constexpr int kSyncSpins = 1 << 24;
 
 struct GridBarrier {
   unsigned* arrived;  // zero before the launch
   int* fault;
   unsigned epoch;
+  bool cluster;  // the launch is one cluster
   // all blocks' writes before it are visible to all blocks after it; false: leave the kernel
   __device__ __forceinline__ bool sync() {
+    if (cluster) {
+      asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+      return true;
+    }
     __shared__ int ok;
     __syncthreads();
     epoch += gridDim.x;
