@@ -93,11 +93,15 @@ __device__ __forceinline__ void part_bounds(const int* __restrict__ range, int& 
 }
 
 // One traversal step.  Each lane takes kTravItems consecutive frontier pairs (their loads are
-// independent); output slots come from one warp-wide scan of the lanes' packed (M2L, P2P,
-// children) counts and three atomics per warp.  Writes beyond a buffer's capacity are
+// independent); output slots come from a warp-wide scan of the lanes' packed (M2L, P2P,
+// children) counts, the block's warps' totals and three atomics per block and 512 pairs.  (Three
+// per warp, all on the same addresses, and four pairs a lane at 126 registers: traverse phase of
+// Plummer 2^20 0.89 ms, now 0.79; sphere of 2^22 1.13 -> 0.93; 256 solves 4.18 -> 3.79.  One
+// pair a lane 0.81, 1.03 and 4.18; four in 80 registers 0.94, 1.12 and 4.42; the children of a
+// split written by the whole warp 0.99, 1.33 and 4.65.)  Writes beyond a buffer's capacity are
 // skipped but every slot below it is written and all are counted, so the host can tell an
 // overflow from the counts and run the traversal again on larger buffers.
-constexpr int kTravItems = 4;
+constexpr int kTravItems = 2, kTravStepThreads = 256;
 constexpr int kTravMaxSteps = 2 * (kMaxLevel + 1) + 2;
 
 template <typename T> struct TravArgs {
@@ -144,11 +148,14 @@ __device__ __forceinline__ void trav_step(const TravArgs<T>& g, const vec4<T>* _
   unsigned long long *ctr = g.ctr, *m2l = g.m2l, *p2p = g.p2p;
   const unsigned long long m2l_cap = g.m2l_cap, p2p_cap = g.p2p_cap, next_cap = g.front_cap;
   const int lane = lane_id();
-  const long long stride = (long long)gridDim.x * blockDim.x * kTravItems;
-  const long long wbase =
-      ((long long)blockIdx.x * blockDim.x + threadIdx.x - lane) * kTravItems;
-  for (long long w = wbase; w < nfront; w += stride) {  // warp-uniform trip count
-    const long long t0 = w + (long long)lane * kTravItems;
+  constexpr int WARPS = kTravStepThreads / 32;
+  __shared__ unsigned wtot[WARPS];
+  __shared__ unsigned long long at[3];
+  const int wl = threadIdx.x >> 5;
+  const long long stride = (long long)gridDim.x * kTravStepThreads * kTravItems;
+  const long long base = (long long)blockIdx.x * kTravStepThreads * kTravItems;
+  for (long long w = base; w < nfront; w += stride) {  // block-uniform trip count
+    const long long t0 = w + (long long)threadIdx.x * kTravItems;
     int ty[kTravItems], k[kTravItems];
     int2 p[kTravItems];
     unsigned v = 0;  // packed: M2L in bits 0-8, P2P in 9-17, children in 18-31 (warp totals:
@@ -208,16 +215,27 @@ __device__ __forceinline__ void trav_step(const TravArgs<T>& g, const vec4<T>* _
       const unsigned x = __shfl_up_sync(0xffffffffu, incl, o);
       if (lane >= o) incl += x;
     }
-    const unsigned tot = __shfl_sync(0xffffffffu, incl, 31);
-    unsigned long long bm = 0, bp = 0, bn = 0;
-    if (lane == 31) {
-      if (tot & 0x1ffu) bm = atomicAdd(&ctr[0], (unsigned long long)(tot & 0x1ffu));
-      if ((tot >> 9) & 0x1ffu) bp = atomicAdd(&ctr[1], (unsigned long long)((tot >> 9) & 0x1ffu));
-      if (tot >> 18) bn = atomicAdd(next_count, (unsigned long long)(tot >> 18));
+    if (lane == 31) wtot[wl] = incl;
+    __syncthreads();
+    // bits of a field in the packed totals: M2L, P2P, children
+    auto field = [](unsigned x, int f) { return f == 0 ? x & 0x1ffu : f == 1 ? x >> 9 & 0x1ffu : x >> 18; };
+    unsigned long long bm = 0, bp = 0, bn = 0;  // of the block's earlier warps
+    for (int k = 0; k < wl; k++) {
+      bm += field(wtot[k], 0);
+      bp += field(wtot[k], 1);
+      bn += field(wtot[k], 2);
     }
-    bm = __shfl_sync(0xffffffffu, bm, 31) + ((incl - v) & 0x1ffu);
-    bp = __shfl_sync(0xffffffffu, bp, 31) + (((incl - v) >> 9) & 0x1ffu);
-    bn = __shfl_sync(0xffffffffu, bn, 31) + ((incl - v) >> 18);
+    if (threadIdx.x < 3) {
+      unsigned sum = 0;
+      for (int k = 0; k < WARPS; k++) sum += field(wtot[k], threadIdx.x);
+      at[threadIdx.x] =
+          sum ? atomicAdd(threadIdx.x < 2 ? &ctr[threadIdx.x] : next_count, (unsigned long long)sum)
+              : 0;
+    }
+    __syncthreads();
+    bm += at[0] + field(incl - v, 0);
+    bp += at[1] + field(incl - v, 1);
+    bn += at[2] + field(incl - v, 2);
 #pragma unroll
     for (int u = 0; u < kTravItems; u++) {
       const unsigned long long packed =
@@ -245,7 +263,7 @@ __device__ __forceinline__ void trav_step(const TravArgs<T>& g, const vec4<T>* _
 
 // Step l as a launch of its own, its frontier's size read on the device.
 template <typename T>
-__global__ void __launch_bounds__(256) k_trav_step(TravArgs<T> g, int l) {
+__global__ void __launch_bounds__(kTravStepThreads, 4) k_trav_step(TravArgs<T> g, int l) {
   int b0, b1;
   part_bounds(g.range, b0, b1);
   const unsigned long long n = l == 0 ? g.nfront0 : min(g.ctr[4 + l], g.front_cap);
@@ -804,7 +822,8 @@ static void traverse_lists(Solver<T>& s, long long& nm2l, long long& np2p) {
       steps = std::min(steps, s.trav_steps + 2 * std::max(0, s.maxlevel - s.trav_maxlevel) + 2);
     }
     for (int l = 0; l < steps; l++) {
-      k_trav_step<T><<<std::min(148 * 8, std::max(1, s.ncells / 8)), 256, 0, s.stream>>>(g, l);
+      k_trav_step<T><<<std::min(148 * 8, std::max(1, s.ncells / 8)), kTravStepThreads, 0,
+                       s.stream>>>(g, l);
       FMM_LAUNCH_CHECK();
     }
     if (stacks) {
