@@ -108,7 +108,8 @@ void set_bodies_host_t(Solver<T>& s, int n, const double* x, const double* q, in
     DevArr<double>& tmp = s.dtmp;
     tmp.ensure(4 * m);
     auto up = [&](double* dst, const double* src, size_t k) {
-      if (k) FMM_CUDA(cudaMemcpyAsync(dst, src, sizeof(double) * k, cudaMemcpyHostToDevice, s.stream));
+      if (k)
+        FMM_CUDA(cudaMemcpyAsync(dst, src, sizeof(double) * k, cudaMemcpyHostToDevice, s.stream));
     };
     up(tmp.p, x, 3 * (size_t)n);
     up(tmp.p + 3 * (size_t)n, x2, 3 * (size_t)n2);
@@ -496,7 +497,7 @@ int fmm_b200_create(const fmm_b200_config* cfg, fmm_b200_solver** out) {
     for (auto* a : ia) a->OP();                                                            \
     s_.keys.OP(); s_.keys2.OP(); s_.c_icell.OP(); s_.m2l.OP(); s_.fs_keys.OP();            \
     s_.c_info.OP(); s_.fs_root.OP(); s_.fs_root2.OP(); s_.tgt_key.OP();                                   \
-    s_.p2p.OP(); s_.list_tmp.OP(); s_.p2p_pairs_count.OP(); s_.p2p_order.OP();             \
+    s_.p2p.OP(); s_.list_tmp.OP(); s_.p2p_order.OP();             \
     s_.p2p_srcs.OP();                                                                      \
     s_.cub_tmp.OP(); s_.front.OP(); s_.front2.OP(); s_.trav_stacks.OP();                   \
     s_.seg_keys2.OP(); s_.cub_tmp2.OP(); s_.dtmp.OP();                                     \

@@ -52,11 +52,12 @@ __device__ __forceinline__ float rsqrt_ftz(float a) {
 __device__ __forceinline__ double rsqrt_ftz(double a) { return rsqrt(a); }
 
 // Most targets of a lane, and the lanes G that share one: 32 TPL / G slots for the leaf's
-// targets (64 at a time; FP32 without images: p2p_width).  FP32 at the default limits g4 = 8, g2 = 16: G = 8 up to 12 bodies, 4
-// up to 24, 2 up to 48, so slots come in steps of 4, 8 and 16 and few stay idle; FP64, whose
-// arithmetic and not its reads bounds it, takes G = 4, 2, 1 (fewer sums to merge).  So do solves
-// with periodic images, whose sums are also folded after every chunk by one warp per leaf: in
-// that order their results keep every bit they had (30,003 bodies: 0.05 ms either way).
+// targets (64 at a time; FP32 without images: p2p_width).  FP32 at the default limits g4 = 8,
+// g2 = 16: G = 8 up to 12 bodies, 4 up to 24, 2 up to 48, so slots come in steps of 4, 8 and 16
+// and few stay idle; FP64, whose arithmetic and not its reads bounds it, takes G = 4, 2, 1 (fewer
+// sums to merge).  So do solves with periodic images, whose sums are also folded after every
+// chunk by one warp per leaf: in that order their results keep every bit they had (30,003 bodies:
+// 0.05 ms either way).
 template <typename T> __host__ __device__ constexpr int p2p_tpl() { return sizeof(T) == 4 ? 3 : 2; }
 template <typename T> __device__ __forceinline__ int p2p_lanes(int nb, int g4, int g2, int images) {
   if (sizeof(T) == 8 || images) return nb <= g4 ? 4 : nb <= g2 ? 2 : 1;

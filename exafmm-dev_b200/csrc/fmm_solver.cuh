@@ -180,7 +180,6 @@ struct SolverBase {
   DevArr<unsigned long long> p2p_srcs;  // source leaves of the P2P pairs as k_p2p reads them
   bool p2p_ordered = false;
   int m2l_ntgt = 0;
-  DevArr<unsigned long long> p2p_pairs_count;
   DevArr<double> dtmp;  // host <-> device conversion scratch
   // phase timing
   cudaEvent_t ev[2 * FMM_NUM_PHASES] = {};
@@ -259,13 +258,9 @@ void sort_pairs_u64(SolverBase& s, const unsigned long long* kin, unsigned long 
 void sort_keys_u64(SolverBase& s, const unsigned long long* kin, unsigned long long* kout,
                    int n, int end_bit);
 void sort_pairs_u32(SolverBase& s, const unsigned* kin, unsigned* kout, const int* vin,
-                    int* vout, int n, int end_bit, DevArr<char>* tmp = nullptr);
+                    int* vout, int n, int end_bit);
 // scratch: s.cub_tmp, or tmp for a scan that may run beside other CUB calls of the solver
 void exclusive_sum_int(SolverBase& s, const int* in, int* out, int n,
                        DevArr<char>* tmp = nullptr);
-void segmented_sort_pairs_u64(SolverBase& s, const unsigned long long* kin,
-                              unsigned long long* kout, const int* vin, int* vout, int n,
-                              int nseg, const int* begin, const int* end, int end_bit);
-void sum_u64(SolverBase& s, const unsigned long long* in, unsigned long long* out, int n);
 
 }  // namespace fmmb200

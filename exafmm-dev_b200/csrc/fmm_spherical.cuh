@@ -257,7 +257,7 @@ __global__ void __launch_bounds__(tr_threads<T>())
 // instructions arrive at about one in eight cycles (35-45 us a level at P = 10 whatever its
 // cells): the folded form is under half as long.  One warp per block, so that a level of few
 // cells spreads over the SMs; the output orders in groups as the M2L's.  Upward phase of
-// 31,250 bodies at P = 10 0.10 -> 0.058 ms, M2M and P2M beside the traversal of 2^20 bodies
+// 31,607 bodies at P = 10 0.10 -> 0.058 ms, M2M and P2M beside the traversal of 2^20 bodies
 // 0.49-0.61 -> 0.28 ms, of 256 solves at P = 8 2.4-2.9 -> 2.05 ms; FP64 (P = 8) within the
 // spread.
 template <typename T> __host__ __device__ constexpr bool m2l_folds(int P) {
@@ -732,7 +732,7 @@ __device__ __forceinline__ void m2l_term(int P, int j, int k, const T* y, const 
 
 // L2P with one thread per body (tree order), its leaf from the map P2M wrote, the leaf's
 // local expansion read through L1 (the bodies of a warp share one to three leaves): every
-// lane busy whatever the leaf sizes; the arithmetic per body is that of k_l2p
+// lane busy whatever the leaf sizes
 template <typename T, int P>
 __global__ void __launch_bounds__(128)
     k_l2p_bodies(int n, const int* __restrict__ body_leaf, const vec4<T>* __restrict__ cX,

@@ -275,9 +275,7 @@ __global__ void __launch_bounds__(kTravStepThreads, 4) k_trav_step(TravArgs<T> g
 // at a time and walks all that comes of them: up to kTravThreads pairs from the top of its
 // stack per round, one per thread, whose children go back on the stack and whose M2L and P2P
 // pairs go through shared memory to the lists a few hundred at a time.  No block waits for
-// another, and neither list's counter is touched once a warp: a launch per step cost 5-6 us
-// however few pairs it had, and on large trees its atomics (three per 128 pairs on three
-// addresses) and its frontiers' passage through memory.
+// another: a launch per step costs 5-6 us however few pairs it has.
 constexpr int kTravThreads = 128, kTravBlocks = 8;  // per block; blocks per SM
 constexpr int kTravBuf = 512;     // pairs of either list that a block holds back
 constexpr int kTravStack = 4096;  // pairs
@@ -777,8 +775,9 @@ template <typename T> static void upload_roots(Solver<T>& s) {
 // traversal took, two more per level that the tree has grown by since, and two to spare (at
 // first as many as any tree needs).  Against all steps in one cooperative kernel with a barrier
 // between them the traverse phase of 1,000 bodies takes 0.16 instead of 0.19 ms, of 200,003 0.26
-// instead of 0.31, of 250,007 in the uniform tree 0.25 instead of 0.27; 2^20 bodies (64,000
-// cells) take 0.90 ms by steps and 1.03 in k_traverse, whose blocks end far apart there.
+// instead of 0.31, of 250,007 in the uniform tree 0.25 instead of 0.27; 2^22 on a sphere (361,000
+// cells) took 1.26 ms in k_traverse, whose blocks end far apart there, and 1.14 by steps (0.93
+// since).
 constexpr int kTravStackCells = 8192;
 
 template <typename T>

@@ -5,9 +5,10 @@
 // that each level moves by +-R0 / 2^(level+1) (:199-203).  Here every body walks that same
 // chain of centres once (k_keys), recording its octant at each of kMaxLevel levels as a
 // 63-bit path key; a stable radix sort by key then lays the bodies out in octant order, and
-// nodes are carved out of the sorted keys level by level (k_split / k_emit), each node's
-// octant sub-ranges found by binary search.  Bodies inside a leaf keep their input order,
-// as the stable partitions leave them, via a second stable sort by leaf-truncated key.
+// nodes are carved out of the sorted keys level by level (k_tree), each node's
+// octant sub-ranges found by binary search.  Bodies inside a leaf keep their input order, as
+// the stable partitions leave them: ranked by the leaf's warp (k_tree), or, with leaves above
+// kRankBodies, by a second stable sort by leaf-truncated key.
 // Cells take the reference's layout (Nodes2cells :250-294): root first, the children of a
 // cell contiguous, each child's subtree after the previous child's.
 #include <algorithm>
