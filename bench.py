@@ -17,8 +17,8 @@ use_rmax = use_ropt = 1, FP32 expansions with compensated potential/gradient sum
   event-timed duration; peak = the nominal FP32 rate 148 SMs x 128 lanes x 2 flops x the SM
   clock sampled during the timed solves (the FMA throughput measured by fmm_b200_fp32_peak
   is reported beside it).  The flops the kernel actually executes (the contraction in the
-  source's azimuthal frame: 4 sum (j+1)(P-j)^2 + 14 (P(P+1)/2 - P) + 2 P = 5,490 per pair
-  at P = 10) are reported as executed_tflops.
+  source's azimuthal frame with the +m and -m terms folded, and the rotations: 3,440 per pair at
+  P = 10, the harmonics apart) are reported as executed_tflops.
 * cpu_baseline: the reference exafmm-dev CPU FMM (oracle/_ref/perf, compiled from the
   reference's sources) on the same workload (N = 2^20) with all host threads, median of 3
   runs, per phase.
@@ -79,10 +79,17 @@ def m2l_flops_per_pair(P, basis="spherical"):
 
 
 def m2l_executed_flops_per_pair(P):
-    """Flops the spherical M2L kernel executes per pair: the contraction in the source's
-    azimuthal frame (two real multiply-adds per term) plus the source and output rotations."""
-    rot = P * (P + 1) // 2 - P
-    return 4 * sum((j + 1) * (P - j) ** 2 for j in range(P)) + 14 * rot + 2 * P
+    """Flops the spherical M2L kernel executes per pair beside the harmonics: the contraction in
+    the source's azimuthal frame with the +m and -m terms folded (per source order mu, target
+    order k and harmonic degree a: the two shared factors, then two real multiply-adds for each
+    of its coefficients) plus the source and output rotations."""
+    n = 14 * (P * (P + 1) // 2 - P) + 4 * P
+    for mu in range(P):
+        for k in range(P - mu):
+            for a in range(k + mu, P):
+                t = a - k - mu + 1
+                n += 4 * t if mu == 0 else 2 * t if k == 0 else 2 + 4 * t
+    return n
 
 
 def nominal_fp32_tflops(sm_mhz):
@@ -598,7 +605,7 @@ def bench_cartesian(fmm, datasets, torch, dev, stream, flush, device, steps, clk
            "l2": "256 MB flush before each timed solve"}
     if cpu_baseline:
         oracle, _ = reference_lib()
-        if oracle.have_reference(CART_REF_CONFIG, "perf"):
+        if oracle and oracle.have_reference(CART_REF_CONFIG, "perf"):
             ref = oracle.Reference(CART_REF_CONFIG, "perf")
             threads = os.cpu_count() or 1
             wall, ph = reference_median(ref, x, q, CART, threads)
