@@ -18,7 +18,8 @@ use_rmax = use_ropt = 1, FP32 expansions with compensated potential/gradient sum
   clock sampled during the timed solves (the FMA throughput measured by fmm_b200_fp32_peak
   is reported beside it).  The flops the kernel actually executes (the contraction in the
   source's azimuthal frame with the +m and -m terms folded, and the rotations: 3,440 per pair at
-  P = 10, the harmonics apart) are reported as executed_tflops.
+  P = 10, the harmonics apart) are reported as executed_tflops: fewer than the counted ones, so
+  frac may pass 1.
 * cpu_baseline: the reference exafmm-dev CPU FMM (oracle/_ref/perf, compiled from the
   reference's sources) on the same workload (N = 2^20) with all host threads, median of 3
   runs, per phase.
@@ -942,7 +943,7 @@ def main():
         "fp64_gpu": fp64,
         "e2e": {"value": e2e_value, "unit": "particles/s", "h2d_bytes_per_step": 32 * n,
                 "d2h_bytes_per_step": 32 * n, "ms_per_step": e2e_total / len(e2e_ms)},
-        "roofline": {"kernel": "M2L (k_m2l_reg<float,10>)", "bound": "fp32",
+        "roofline": {"kernel": "M2L (k_m2l_fold<float,10>)", "bound": "fp32",
                      "achieved": m2l_tflops, "peak": peak, "unit": "TFLOP/s",
                      "frac": m2l_tflops / peak, "traffic": traffic,
                      "flops_per_pair": m2l_flops_per_pair(WORKLOAD["P"]),
