@@ -405,8 +405,8 @@ __global__ void __launch_bounds__(32)
 // The multipoles are read from a copy by order (k_m2l_rows), 16 bytes a load: a load from 32
 // rows occupies the L1 nine cycles whatever its width.  Plummer N = 2^20, P = 10 (11.7 M
 // pairs, FP32) 2.31 -> 1.46 ms in one pass where two passes of k_m2l_reg ran before; 256 solves
-// at P = 8 8.5 -> 6.1 ms.  At P = 10 the FMA pipe is busy 44-47 % at 8 warps per SM; loads of the
-// rows (long scoreboard) are the largest stall.
+// at P = 8 8.5 -> 6.1 ms.  At P = 10 the FMA pipe is busy 52 % and the L1 data pipe
+// 71 % at 8 warps per SM; loads of the rows (long scoreboard) are the largest stall.
 // Measured and not kept: rows staged in shared memory by one bulk copy per lane (1.59 ms
 // against 1.47 ms), 12 warps per SM at 168 registers (2.7 ms: more columns, less L1).
 template <typename T> __host__ __device__ constexpr int m2l_words() {
