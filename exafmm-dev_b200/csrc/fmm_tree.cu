@@ -372,7 +372,13 @@ __device__ __forceinline__ void tree_node(const TreeArgs<T>& a, int lane, int v,
   const T R = div_rn(R0, (T)(1 << level));
   if (c <= 64) rank_leaf<T, 2>(a, lane, v, b, c, X0, X1, X2, R);
   else if (c <= kRankBodies) rank_leaf<T, kRankBodies / 32>(a, lane, v, b, c, X0, X1, X2, R);
-  else if (lane == 0) atomicExch(&a.ctl[TC_BIG], 1);
+  else if (lane == 0) {
+    atomicExch(&a.ctl[TC_BIG], 1);
+    if (a.radii) {  // (defined values for the cells above; the structure pass sets them anew)
+      a.nX[4 * v + 3] = R;
+      a.nM0[v] = 0;
+    }
+  }
 }
 
 // The subtree size (NNODE, include/build_tree_tbb.h:215-217) of a split node, and with radii
@@ -539,6 +545,16 @@ __global__ void k_leaf_levels(int nnodes, const int* __restrict__ nchildn,
   if (v >= nnodes || nchildn[v] != 0) return;
   int lev = nlevel[v];
   for (int b = nbegin[v]; b < nbegin[v] + ncount[v]; b++) blev[b] = lev;
+}
+
+// every cell's radius as before any solve sets it: the half side of its box (a tree kernel that
+// sets final radii leaves those of a tree with a leaf it could not rank unfinished)
+template <typename T>
+__global__ void k_box_radii(int nnodes, const int* __restrict__ nlevel,
+                            const int* __restrict__ nsid, const int* __restrict__ npos,
+                            const T* __restrict__ box, vec4<T>* __restrict__ cX) {
+  const int v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < nnodes) cX[npos[v]].w = div_rn(box[16 * nsid[v] + 3], (T)(1 << nlevel[v]));
 }
 
 // key truncated to the body's leaf, scattered back to input order
@@ -1012,6 +1028,11 @@ template <typename T> void build_tree(Solver<T>& s, bool radii) {
   if (rank && !hc[TC_BIG]) {
     s.radii_set = radii;
     return;
+  }
+  if (rank && radii) {  // (the structure pass then forms the radii from the boxes')
+    k_box_radii<T><<<ceil_div(nnodes, TB), TB, 0, s.stream>>>(nnodes, s.nlevel.p, s.nsid.p,
+                                                              s.npos.p, s.box.p, s.cX.p);
+    FMM_LAUNCH_CHECK();
   }
   // leaves of more bodies than a warp ranks: stable sort by leaf-truncated key from input order
   if (levels < kMaxLevel) {

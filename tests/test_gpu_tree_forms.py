@@ -126,3 +126,30 @@ def test_small_tree_grouping(n):
     img = np.arange(27, dtype=np.int64)
     ref = leaves[:, None, None] << 32 | img[None, :, None] << 27 | leaves[None, None, :]
     assert np.array_equal(p2p, ref.ravel())
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("use_rmax", [1, 0])
+@pytest.mark.parametrize("use_ropt", [0, 1])
+def test_coincident_bodies_radii(prec, use_rmax, use_ropt):
+    """More coincident bodies than a warp ranks, on a fresh handle and on one that has solved
+    before: radii and lists of a whole solve are those of the stages, results too."""
+    kw = dict(P=4, theta=0.5, ncrit=32, precision=prec, use_rmax=use_rmax, use_ropt=use_ropt)
+    x, q = bodies("same", 1600, np.random.default_rng(5), prec)
+    y, w = bodies("clump", 3000, np.random.default_rng(6), prec)
+    ref = fmm.Solver(**kw)
+    ref.set_bodies(x, q)
+    ref.build_tree()
+    ref.upward_pass()
+    ref.traverse()
+    ref.downward_pass()
+    R, lists, trg = ref.cells()["R"], ref.lists(), ref.trg()
+    s = fmm.Solver(**kw)
+    for rep in range(2):
+        got = s.solve(x, q)
+        assert s.cells()["level"].max() == 21
+        assert np.array_equal(s.cells()["R"], R), rep
+        for a, b in zip(s.lists(), lists):
+            assert np.array_equal(a, b), rep
+        assert np.array_equal(got, trg)
+        s.solve(y, w)
