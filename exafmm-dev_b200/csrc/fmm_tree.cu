@@ -18,6 +18,7 @@
 
 #include "fmm_grid.cuh"
 #include "fmm_solver.cuh"
+#include "fmm_tree_plan.cuh"
 
 namespace fmmb200 {
 
@@ -973,8 +974,7 @@ template <typename T> void build_tree(Solver<T>& s, bool radii) {
     t.nchild = s.c_nchild.p, t.ibody = s.c_ibody.p, t.nbody = s.c_nbody.p;
     t.clevel = s.c_level.p, t.croot = s.c_root.p, t.leaves = s.leaves.p, t.bodies = s.bodies.p;
     t.icell = s.c_icell.p, t.info = s.c_info.p, t.cX = s.cX.p, t.m0 = s.m0.p;
-    // a warp for every few nodes of the widest level: fewer blocks make cheaper barriers
-    int blocks = std::max(1, std::min(kTreeBlocks * 148, ceil_div(n, 4 * s.cfg.ncrit)));
+    int blocks = tree_blocks(n, s.cfg.ncrit, kTreeBlocks * 148);
     FMM_CUDA(cudaMemsetAsync(s.tree_ctl.p, 0, TC_INTS * sizeof(int), s.stream));
     void* args[] = {&t};
     if (blocks <= 2 * kTreeCluster) {

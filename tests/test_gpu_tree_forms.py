@@ -153,3 +153,16 @@ def test_coincident_bodies_radii(prec, use_rmax, use_ropt):
             assert np.array_equal(a, b), rep
         assert np.array_equal(got, trg)
         s.solve(y, w)
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("ncrit", [1 << 29, 1 << 30, 2 ** 31 - 1])
+def test_one_leaf(prec, ncrit):
+    """An ncrit as large as an int holds: one leaf, the direct sum.  FP32 sums of one sign: 2e-6
+    of the magnitudes as in the near-field tests, which the potentials are."""
+    x, q = bodies("cube", 777, np.random.default_rng(2), prec)
+    s = fmm.Solver(P=4, ncrit=ncrit, precision=prec, use_ropt=0)
+    t = s.solve(x, q)
+    assert s.num_cells() == (1, 0)
+    ref = fmm.direct(x, x, q)
+    assert (np.abs(t[:, 0] - ref[:, 0]) <= (2e-6 if prec == "f32" else 1e-13) * ref[:, 0]).all()
