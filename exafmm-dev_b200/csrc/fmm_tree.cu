@@ -925,10 +925,12 @@ template <typename T> void build_tree(Solver<T>& s, bool radii) {
   // whatever the order of their deeper digits.  A tree that turns out deeper is built again
   // with the keys sorted on every digit.
   int levels = s.tree_plan > 0 && rank ? std::min(s.tree_plan + 1, kMaxLevel) : kMaxLevel;
-  size_t cap = (size_t)std::max(1024, 4 * (n / std::max(1, s.cfg.ncrit)) + 64 + nroots);
+  size_t cap = tree_first_nodes(n, s.cfg.ncrit, nroots);
   int* hc = s.scal_host + kTreeHost;
   bool sorted = false;
   for (;;) {
+    if (cap == 0)
+      throw FmmError(FMM_ERR_NOT_SUPPORTED, "more than 2^27 - 1 cells (list pairs hold 27-bit cells)");
     if (!sorted) {
       k_keys<T><<<ceil_div(n, TB), TB, 0, s.stream>>>(s.bodies_in.p, n, s.box.p, s.root_first,
                                                       nroots, s.keys.p, s.idx.p);
@@ -940,7 +942,7 @@ template <typename T> void build_tree(Solver<T>& s, bool radii) {
     DevArr<int>* narr[] = {&s.nbegin, &s.ncount, &s.nparent, &s.nchildn, &s.nfirst, &s.nnode,
                            &s.npos, &s.ncb, &s.nlevel, &s.nsid, &s.c_iparent, &s.c_ichild,
                            &s.c_nchild, &s.c_ibody, &s.c_nbody, &s.c_level, &s.c_root, &s.leaves};
-    size_t ncap = (size_t)INT_MAX / 16;
+    size_t ncap = kTreeMaxNodes;
     for (auto* q : narr) {
       q->ensure(cap);
       ncap = std::min(ncap, q->cap);
@@ -1015,7 +1017,7 @@ template <typename T> void build_tree(Solver<T>& s, bool radii) {
       levels = kMaxLevel;
       sorted = false;
     }
-    if (full) cap = 2 * ncap;
+    if (full) cap = tree_more_nodes(ncap);
     if (!deep && !full) break;
   }
   s.level_lo.assign({0, nroots});

@@ -2,6 +2,7 @@
 // that they can be checked without a device.
 #pragma once
 #include <algorithm>
+#include <cstddef>
 
 namespace fmmb200 {
 
@@ -10,6 +11,19 @@ namespace fmmb200 {
 inline int tree_blocks(int n, int ncrit, int most) {
   const long long per = 4LL * ncrit, want = (n + per - 1) / per;
   return (int)std::max(1LL, std::min<long long>(want, most));
+}
+
+// Most nodes of a tree: the interaction lists hold 27-bit cells.
+constexpr size_t kTreeMaxNodes = (size_t{1} << 27) - 1;
+
+// Nodes to make room for at first; 0: more roots than a tree may have nodes.
+inline size_t tree_first_nodes(int n, int ncrit, int nroots, size_t most = kTreeMaxNodes) {
+  if ((size_t)nroots > most) return 0;
+  return std::min(most, std::max<size_t>(1024, 4 * (size_t)(n / ncrit) + 64 + nroots));
+}
+// and after a build that needed more than the `had` nodes there was room for; 0: it cannot be built
+inline size_t tree_more_nodes(size_t had, size_t most = kTreeMaxNodes) {
+  return had < most ? std::min(most, 2 * had) : 0;
 }
 
 }  // namespace fmmb200

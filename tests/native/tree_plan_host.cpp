@@ -4,4 +4,11 @@
 
 extern "C" {
 int tree_blocks(int n, int ncrit, int most) { return fmmb200::tree_blocks(n, ncrit, most); }
+unsigned long long tree_first_nodes(int n, int ncrit, int nroots, unsigned long long most) {
+  return most ? fmmb200::tree_first_nodes(n, ncrit, nroots, most)
+              : fmmb200::tree_first_nodes(n, ncrit, nroots);
+}
+unsigned long long tree_more_nodes(unsigned long long had, unsigned long long most) {
+  return most ? fmmb200::tree_more_nodes(had, most) : fmmb200::tree_more_nodes(had);
+}
 }

@@ -16,7 +16,11 @@ def lib(tmp_path_factory):
     subprocess.check_call(["/usr/bin/g++", "-O1", "-std=c++17", "-shared", "-fPIC", "-Wall",
                            "-I", os.path.join(ROOT, "exafmm-dev_b200", "csrc"),
                            os.path.join(ROOT, "tests", "native", "tree_plan_host.cpp"), "-o", str(out)])
-    return C.CDLL(str(out))
+    f = C.CDLL(str(out))
+    f.tree_first_nodes.argtypes = [C.c_int] * 3 + [C.c_ulonglong]
+    f.tree_more_nodes.argtypes = [C.c_ulonglong] * 2
+    f.tree_first_nodes.restype = f.tree_more_nodes.restype = C.c_ulonglong
+    return f
 
 
 @pytest.mark.parametrize("n", [1, 2, 1000, 1 << 20, 1 << 29, INT_MAX])
@@ -24,3 +28,24 @@ def lib(tmp_path_factory):
 def test_tree_blocks(n, ncrit, lib):
     for most in (1, 33, 444):
         assert lib.tree_blocks(n, ncrit, most) == max(1, min(most, -(-n // (4 * ncrit))))
+
+
+@pytest.mark.parametrize("n,ncrit,nroots", [(1, 1, 1), (1000, 64, 1), (1 << 29, 1, 1),
+                                            (INT_MAX, 1, 1), (INT_MAX, INT_MAX, 1000000)])
+@pytest.mark.parametrize("most", [0, 5000])
+def test_tree_nodes(n, ncrit, nroots, most, lib):
+    """Room for a tree that never fits: it grows to the limit (0: the builder's own, 2^27 - 1; or a
+    lower one), and then there is no more, so the rebuilds end."""
+    top = most or 2 ** 27 - 1
+    cap = lib.tree_first_nodes(n, ncrit, nroots, most)
+    if nroots > top:
+        assert cap == 0
+        return
+    assert cap == min(top, max(1024, 4 * (n // ncrit) + 64 + nroots))
+    for _ in range(30):
+        more = lib.tree_more_nodes(cap, most)
+        if more == 0:
+            break
+        assert cap < more <= top
+        cap = more
+    assert more == 0 and cap == top
