@@ -148,6 +148,7 @@ struct SolverBase {
   // (p2p_g4 <= 8 and p2p_g2 <= 16: a warp holds 32 / lanes targets); fmm_b200_autotune_p2p
   int p2p_g4 = 8, p2p_g2 = 16;
   DevArr<int> tree_ctl;     // control block of the tree kernel
+  int tree_most = 0;        // its blocks that the device holds at a time (0: not asked yet)
   bool radii_set = false;   // the tree kernel has set the cells' radii and monopoles
   // targets and sources in two trees (segments 0 and 1) on a common box, traversed from
   // (target root, source root) only (fmm_b200_solve_ij_*)

@@ -523,6 +523,18 @@ __global__ void __launch_bounds__(kTreeThreads, kTreeBlocks) k_tree(TreeArgs<T> 
   }
 }
 
+// Blocks of k_tree that this device (or this process's share of it) holds at a time: its launch
+// is refused with more.
+template <typename T> static int tree_resident(SolverBase& s) {
+  if (s.tree_most == 0) {
+    int sms = 0, per = 0;
+    FMM_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.cfg.device));
+    FMM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_tree<T>, kTreeThreads, 0));
+    s.tree_most = tree_most(sms, per, kTreeBlocks);
+  }
+  return s.tree_most;
+}
+
 // (NCHILD, ICHILD, NBODY, IBODY) of every cell in one 16-byte record, for the traversal
 __global__ void k_cell_info(int ncells, const int* __restrict__ nchild,
                             const int* __restrict__ ichild, const int* __restrict__ nbody,
@@ -976,7 +988,7 @@ template <typename T> void build_tree(Solver<T>& s, bool radii) {
     t.nchild = s.c_nchild.p, t.ibody = s.c_ibody.p, t.nbody = s.c_nbody.p;
     t.clevel = s.c_level.p, t.croot = s.c_root.p, t.leaves = s.leaves.p, t.bodies = s.bodies.p;
     t.icell = s.c_icell.p, t.info = s.c_info.p, t.cX = s.cX.p, t.m0 = s.m0.p;
-    int blocks = tree_blocks(n, s.cfg.ncrit, kTreeBlocks * 148);
+    int blocks = tree_blocks(n, s.cfg.ncrit, tree_resident<T>(s));
     FMM_CUDA(cudaMemsetAsync(s.tree_ctl.p, 0, TC_INTS * sizeof(int), s.stream));
     void* args[] = {&t};
     if (blocks <= 2 * kTreeCluster) {

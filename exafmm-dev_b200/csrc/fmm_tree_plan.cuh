@@ -6,6 +6,10 @@
 
 namespace fmmb200 {
 
+// Blocks of the tree kernel that are resident together on `sms` SMs that hold `per` of them each,
+// `want` of which each is to take at most (more make dearer barriers).
+inline int tree_most(int sms, int per, int want) { return std::max(1, sms * std::min(per, want)); }
+
 // Blocks of the tree kernel, at most `most`: a warp for every few nodes of the widest level
 // (fewer blocks make cheaper barriers).  Any ncrit that an int holds.
 inline int tree_blocks(int n, int ncrit, int most) {

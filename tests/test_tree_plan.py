@@ -49,3 +49,14 @@ def test_tree_nodes(n, ncrit, nroots, most, lib):
         assert cap < more <= top
         cap = more
     assert more == 0 and cap == top
+
+
+@pytest.mark.parametrize("sms", [1, 8, 18, 74, 132, 148])
+@pytest.mark.parametrize("per", [1, 2, 3, 4])
+def test_resident_blocks(sms, per, lib):
+    """A launch whose blocks wait on one another never has more than are resident together."""
+    most = lib.tree_most(sms, per, 3)
+    assert 1 <= most <= sms * per
+    for n in (1, 100000, INT_MAX):
+        assert 1 <= lib.tree_blocks(n, 1, most) <= sms * per
+    assert lib.tree_most(148, per, 3) == 148 * min(per, 3)
