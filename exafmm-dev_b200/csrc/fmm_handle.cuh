@@ -18,6 +18,15 @@ namespace fmmb200 {
 
 template <typename T> Solver<T>& S(fmm_b200_solver* h) { return *static_cast<Solver<T>*>(h->base); }
 
+// Waits for all that a failed call has queued: the handle's next call writes its pinned staging
+// buffers (the roots' bodies, the first frontier) and resizes its arrays without a wait of its
+// own, which every call that succeeds has had.
+inline void settle(SolverBase& s) {
+  (void)cudaStreamSynchronize(s.stream);
+  if (s.side) (void)cudaStreamSynchronize(s.side);
+  if (s.side_lo) (void)cudaStreamSynchronize(s.side_lo);
+}
+
 template <typename F> inline int guarded(fmm_b200_solver* h, F&& f) {
   if (!h || !h->base) return FMM_ERR_INVALID;
   try {
@@ -27,9 +36,11 @@ template <typename F> inline int guarded(fmm_b200_solver* h, F&& f) {
     return FMM_OK;
   } catch (const FmmError& e) {
     h->base->err = e.what();
+    settle(*h->base);
     return e.code;
   } catch (const std::exception& e) {
     h->base->err = e.what();
+    settle(*h->base);
     return FMM_ERR_INVALID;
   }
 }

@@ -881,7 +881,8 @@ template <typename T> void build_tree(Solver<T>& s, bool radii) {
   }
   // bounds per root over chunks of at most 4096 bodies (256 blocks at 2^20 bodies); the
   // roots' first bodies, the chunks' ranges and the roots' first chunks in one upload from
-  // pinned memory (the last solve's was waited for when its tree was read back)
+  // pinned memory (the last solve's was waited for when its tree was read back, a failed one's
+  // when it returned)
   const int CH = 4096;
   int nch = 0;
   for (int r = 0; r < nroots; r++) nch += ceil_div(rfirst[r + 1] - rfirst[r], CH);
