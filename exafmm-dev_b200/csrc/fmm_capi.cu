@@ -499,7 +499,7 @@ int fmm_b200_create(const fmm_b200_config* cfg, fmm_b200_solver** out) {
     s_.c_info.OP(); s_.fs_root.OP(); s_.fs_root2.OP(); s_.tgt_key.OP();                                   \
     s_.p2p.OP(); s_.list_tmp.OP(); s_.p2p_order.OP();             \
     s_.p2p_srcs.OP();                                                                      \
-    s_.cub_tmp.OP(); s_.front.OP(); s_.front2.OP(); s_.trav_stacks.OP();                   \
+    s_.cub_tmp.OP();                                                                       \
     s_.seg_keys2.OP(); s_.cub_tmp2.OP(); s_.dtmp.OP();                                     \
     if ((h)->precision == FMM_FP64) {                                                      \
       Solver<double>& d_ = *static_cast<Solver<double>*>((h)->base);                       \

@@ -52,12 +52,13 @@ template <typename U> struct DevArr {
     return *this;
   }
   ~DevArr() { release(); }
-  void ensure(size_t n) {
+  // spare = false: a first size that is an estimate already, or fixed, is taken as it is
+  void ensure(size_t n, bool spare = true) {
     if (n <= cap) return;
+    const size_t want = spare || p ? 2 * n + 256 : n;
     if (p) retired.push_back(p);
     p = nullptr;
     cap = 0;
-    size_t want = 2 * n + 256;
     g_device_allocs.fetch_add(1, std::memory_order_relaxed);
     cudaError_t e = cudaMalloc((void**)&p, want * sizeof(U));
     if (e != cudaSuccess) {
@@ -139,7 +140,6 @@ struct SolverBase {
   DevArr<int> fs_pos, fs_pos2;
   DevArr<unsigned long long> fs_keys;
   DevArr<int> fs_idx;
-  DevArr<int2> front, front2, trav_stacks;
   int trav_steps = 0, trav_maxlevel = 0;  // the last traversal's steps (0: none), its tree depth
   bool trav_by_steps = false;  // a traversal's stack has overflowed
   int tree_plan = 0;        // levels of the handle's last tree (0: none)
@@ -162,6 +162,7 @@ struct SolverBase {
   DevArr<int> part_range;
   const int* part_ptr() const { return nparts > 1 ? part_range.p : nullptr; }
   int nfront0 = 0;          // pairs of the first traversal step (roots x images)
+  // list_tmp: the traversal's frontiers and stacks, then the keys of the lists' grouping
   DevArr<unsigned long long> m2l, p2p, list_tmp;
   DevArr<int> m2l_off, p2p_off;
   DevArr<int> body_leaf;  // the leaf cell of each body (tree order), written by P2M

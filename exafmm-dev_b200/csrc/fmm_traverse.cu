@@ -731,7 +731,11 @@ static int mutual_of(const SolverBase& s) {
   return s.cfg.mutual && s.cfg.images == 0 && !s.ij ? 1 : 0;
 }
 
-template <typename T> static void upload_roots(Solver<T>& s) {
+// the first frontier (s.nfront0 pairs) to `front`, which root_count() pairs fit
+static int root_count(const SolverBase& s) {
+  return s.ij ? s.nroots == 2 : s.nroots * (s.cfg.images > 0 ? 27 : 1);
+}
+template <typename T> static void upload_roots(Solver<T>& s, int2* front) {
   // one (root, root) pair per solve of the batch (lists never cross solves); with periodic
   // images one per shift of the source tree, in the reference's image order (:250-260)
   std::vector<int2> roots;
@@ -751,7 +755,6 @@ template <typename T> static void upload_roots(Solver<T>& s) {
                                     s.root_cell[r] | (img_code(ix, iy, iz) << kImgShift)));
   }
   s.nfront0 = (int)roots.size();
-  s.front.ensure(std::max(s.nfront0, 1));
   if (roots.empty()) return;
   if (roots.size() > s.roots_cap) {
     if (s.roots_host) s.roots_retired.push_back(s.roots_host);
@@ -762,12 +765,17 @@ template <typename T> static void upload_roots(Solver<T>& s) {
     s.roots_cap = cap;
   }
   std::copy(roots.begin(), roots.end(), s.roots_host);
-  FMM_CUDA(cudaMemcpyAsync(s.front.p, s.roots_host, sizeof(int2) * roots.size(),
+  FMM_CUDA(cudaMemcpyAsync(front, s.roots_host, sizeof(int2) * roots.size(),
                            cudaMemcpyHostToDevice, s.stream));
 }
 
-// The traversal on the handle's buffers, run again on larger ones while any was too small (the
-// buffers start from typical list lengths per cell).  Trees of up to kTravStackCells cells: steps
+// The traversal on the handle's buffers, run again on larger ones while any was too small.  The
+// lists of small trees start at lengths per cell that most inputs stay below; on a larger tree a
+// handle's first traversal counts them.  The stacks and the frontiers lie in the array that the
+// grouping takes its keys from afterwards.  (With arrays of their own, twice as long as needed,
+// and lists sized by cells on every tree, a new handle held 111 MB after a solve of 31,607 bodies
+// and 3.28 GB after one of 2^22 on a sphere; now 63 MB and 2.49 GB, and the first solves take 5.0
+// instead of 6.6 ms and 21.4 instead of 21.6.)  Trees of up to kTravStackCells cells: steps
 // until the frontier is some four times as long as there are cells (a step makes about 20 pairs
 // of one; from a frontier a quarter as long the blocks' shares differ by far more: 30,003 bodies
 // in images 0.37 ms against 0.26), then k_traverse; should one of its stacks overflow, this and
@@ -785,21 +793,26 @@ static void traverse_lists(Solver<T>& s, long long& nm2l, long long& np2p) {
   unsigned long long* ctr = (unsigned long long*)s.scal.p + 32;
   unsigned long long* hctr = (unsigned long long*)s.scal_host + 32;
   constexpr int NC = kTravMaxSteps + 5;
-  size_t m2l = 96 * (size_t)s.ncells + 1024, p2p = 24 * (size_t)s.ncells + 1024,
-         front = 64 * (size_t)s.ncells + 1024;
-  bool stacks = s.ncells <= kTravStackCells && !s.trav_by_steps, all = false;
+  const bool small = s.ncells <= kTravStackCells;
+  size_t m2l = small ? 192 * (size_t)s.ncells + 1024 : 0;
+  size_t p2p = small ? 64 * (size_t)s.ncells + 1024 : 0;
+  size_t front = std::max((small ? 128 : 96) * (size_t)s.ncells + 1024, (size_t)root_count(s));
+  bool stacks = small && !s.trav_by_steps, all = false;
   const int blocks = std::max(16, std::min(148 * kTravBlocks, s.ncells / 2));
   for (;;) {
-    s.m2l.ensure(m2l);
-    s.p2p.ensure(p2p);
-    s.front.ensure(front);
-    s.front2.ensure(front);
-    upload_roots(s);
+    s.m2l.ensure(m2l, !small);
+    s.p2p.ensure(p2p, !small);
+    const size_t stack = stacks ? (size_t)blocks * kTravStack : 0;
+    s.list_tmp.ensure(stack + 2 * front, false);
+    int2* scratch = (int2*)s.list_tmp.p;
+    front = (s.list_tmp.cap - stack) / 2;
+    upload_roots(s, scratch + stack);
     FMM_CUDA(cudaMemsetAsync(ctr, 0, sizeof(unsigned long long) * NC, s.stream));
     TravArgs<T> g{};
-    g.front = s.front.p;
-    g.front2 = s.front2.p;
-    g.front_cap = std::min(s.front.cap, s.front2.cap);
+    g.stacks = scratch;
+    g.front = scratch + stack;
+    g.front2 = g.front + front;
+    g.front_cap = front;
     g.nfront0 = s.nfront0;
     g.m2l_cap = s.m2l.cap;
     g.p2p_cap = s.p2p.cap;
@@ -826,8 +839,6 @@ static void traverse_lists(Solver<T>& s, long long& nm2l, long long& np2p) {
       FMM_LAUNCH_CHECK();
     }
     if (stacks) {
-      s.trav_stacks.ensure((size_t)blocks * kTravStack);
-      g.stacks = s.trav_stacks.p;
       k_traverse<T><<<blocks, kTravThreads, 0, s.stream>>>(g, steps);
       FMM_LAUNCH_CHECK();
     }
@@ -835,35 +846,34 @@ static void traverse_lists(Solver<T>& s, long long& nm2l, long long& np2p) {
                              s.stream));
     FMM_CUDA(cudaStreamSynchronize(s.stream));
     if (hctr[2]) throw FmmError(FMM_ERR_DEVICE, "traversal read a cell index out of range");
-    bool fits = hctr[0] <= s.m2l.cap && hctr[1] <= s.p2p.cap;
-    m2l = std::max<size_t>(s.m2l.cap, hctr[0]);  // (exact counts, or those up to the overflow)
-    p2p = std::max<size_t>(s.p2p.cap, hctr[1]);
-    front = g.front_cap;
-    int used = 0;  // steps with pairs to classify
+    bool walked = true;  // to the end: the counts are exact
+    int used = 0;        // steps with pairs to classify
     for (int l = 0; l < steps; l++) {
       if (hctr[5 + l]) used = l + 2;
       if (hctr[5 + l] > g.front_cap) {
-        fits = false;
+        walked = false;
         front = std::max<size_t>(2 * front, hctr[5 + l]);
       }
     }
     if (hctr[4]) {
-      fits = stacks = false;
+      walked = stacks = false;
       s.trav_by_steps = true;
     }
     if (!stacks && hctr[4 + steps]) {  // more steps than planned
-      fits = false;
+      walked = false;
       all = true;
     }
-    if (fits) {
-      if (!stacks) {
-        s.trav_steps = std::max(used, 1);
-        s.trav_maxlevel = s.maxlevel;
-      }
+    if (walked && !stacks) {
+      s.trav_steps = std::max(used, 1);
+      s.trav_maxlevel = s.maxlevel;
+    }
+    if (walked && hctr[0] <= s.m2l.cap && hctr[1] <= s.p2p.cap) {
       nm2l = (long long)hctr[0];
       np2p = (long long)hctr[1];
       return;
     }
+    m2l = std::max<size_t>(s.m2l.cap, hctr[0]);
+    p2p = std::max<size_t>(s.p2p.cap, hctr[1]);
   }
 }
 
