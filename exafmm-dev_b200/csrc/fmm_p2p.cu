@@ -15,9 +15,9 @@
 // pairs.  Every lane reads every staged source, 16 bytes a source, and the shared-memory
 // pipe returns 128 bytes a cycle and SM: at one target per lane that return path would bound
 // the kernel, not the FMA pipe (4 cycles a source and warp against 3.25), so a source has to
-// serve several targets of its lane.  FP32 folds the sums of 32 of a lane's sources into a
-// compensated (TwoSum) accumulator, so the accumulation error does not grow with the length
-// of the list; FP64 sums plainly.
+// serve several targets of its lane.  FP32 folds the sums of up to 32 of a lane's sources
+// (p2p_folds) into a compensated (TwoSum) accumulator, so the accumulation error does not grow
+// with the length of the list; FP64 sums plainly.
 //
 // Bound: the FMA pipe (FP64: the FP64 pipe), 26 cycles a source pair and target, at 50-65 %
 // of it: the rest is idle target slots, the chunks' staging and latency at 16 warps per SM.
@@ -63,6 +63,15 @@ template <typename T> __device__ __forceinline__ int p2p_lanes(int nb, int g4, i
   if (sizeof(T) == 8 || images) return nb <= g4 ? 4 : nb <= g2 ? 2 : 1;
   constexpr int X = p2p_tpl<T>();
   return nb <= X * g4 / 2 ? 8 : nb <= X * g2 / 2 ? 4 : nb <= 16 * X ? 2 : 1;
+}
+
+// FP32: chunks of a leaf of nb bodies between folds.  A lane sums 32 sources plainly in between
+// (16 in each half of its packed sums), 8 and 16 for targets of leaves up to g4 and g2 bodies: as
+// many as when those had 4 and 2 lanes and every chunk was folded.  With 32 throughout, the near
+// field's error against 64 bits grew by a quarter (30,000 bodies of either sign, 7 a leaf:
+// potential 9.9e-8 of its norm against 7.8e-8).
+__device__ __forceinline__ int p2p_folds(int nb, int G, int g4, int g2) {
+  return G / (nb <= g4 ? 4 : nb <= g2 ? 2 : 1);
 }
 
 // FP32: targets of the next pass of a leaf with `left` to go, 96 at most, and as many as fill
@@ -420,7 +429,8 @@ __global__ void __launch_bounds__(32 * kP2PWarps, sizeof(T) == 4 ? 2 : 3)
   const int per = (ns + 32 * S - 1) / (32 * S) * 32;
   const int p0 = S == 1 ? 0 : min(ns, per * seg), p1 = S == 1 ? INT_MAX : min(ns, p0 + per);
   const int G = p2p_lanes<T>(nb, g4, g2, images);
-  P2PTeam w{0, G, s0, s1, S, p0, p1, images ? 1 : G};
+  P2PTeam w{0, G, s0, s1, S, p0, p1,
+            images ? 1 : sizeof(T) == 8 ? G : p2p_folds(nb, G, g4, g2)};
   const int team = wl / S, bar = 1 + team, thr = 32 * S;
   for (int base = 0, width = 64; base < nb; base += width) {
     if (sizeof(T) == 4 && !images && nb > 64) {
