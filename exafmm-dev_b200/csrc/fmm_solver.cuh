@@ -141,7 +141,7 @@ struct SolverBase {
   DevArr<unsigned long long> fs_keys;
   DevArr<int> fs_idx;
   int trav_steps = 0, trav_maxlevel = 0;  // the last traversal's steps (0: none), its tree depth
-  bool trav_by_steps = false;  // a traversal's stack has overflowed
+  int trav_by_steps = 0;  // traversals to take by steps, since a block's stack has overflowed
   int tree_plan = 0;        // levels of the handle's last tree (0: none)
   int write_r = 1;          // P2M / M2M set the cell radii (else the structure pass did)
   // P2P lanes per target by target leaf size: 4 up to p2p_g4 bodies, 2 up to p2p_g2, else 1

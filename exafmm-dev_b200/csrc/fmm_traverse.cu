@@ -779,7 +779,7 @@ template <typename T> static void upload_roots(Solver<T>& s, int2* front) {
 // until the frontier is some four times as long as there are cells (a step makes about 20 pairs
 // of one; from a frontier a quarter as long the blocks' shares differ by far more: 30,003 bodies
 // in images 0.37 ms against 0.26), then k_traverse; should one of its stacks overflow, this and
-// the handle's later traversals take steps only.  Larger trees: steps only, as many as the last
+// the handle's next kTravBySteps traversals take steps only.  Larger trees: steps only, as many as the last
 // traversal took, two more per level that the tree has grown by since, and two to spare (at
 // first as many as any tree needs).  Against all steps in one cooperative kernel with a barrier
 // between them the traverse phase of 1,000 bodies takes 0.16 instead of 0.19 ms, of 200,003 0.26
@@ -787,6 +787,7 @@ template <typename T> static void upload_roots(Solver<T>& s, int2* front) {
 // cells) took 1.26 ms in k_traverse, whose blocks end far apart there, and 1.14 by steps (0.93
 // since).
 constexpr int kTravStackCells = 8192;
+constexpr int kTravBySteps = 16;
 
 template <typename T>
 static void traverse_lists(Solver<T>& s, long long& nm2l, long long& np2p) {
@@ -797,7 +798,8 @@ static void traverse_lists(Solver<T>& s, long long& nm2l, long long& np2p) {
   size_t m2l = small ? 192 * (size_t)s.ncells + 1024 : 0;
   size_t p2p = small ? 64 * (size_t)s.ncells + 1024 : 0;
   size_t front = std::max((small ? 128 : 96) * (size_t)s.ncells + 1024, (size_t)root_count(s));
-  bool stacks = small && !s.trav_by_steps, all = false;
+  bool stacks = small && s.trav_by_steps == 0, all = false;
+  if (small && !stacks) s.trav_by_steps--;
   const int blocks = std::max(16, std::min(148 * kTravBlocks, s.ncells / 2));
   for (;;) {
     s.m2l.ensure(m2l, !small);
@@ -857,7 +859,7 @@ static void traverse_lists(Solver<T>& s, long long& nm2l, long long& np2p) {
     }
     if (hctr[4]) {
       walked = stacks = false;
-      s.trav_by_steps = true;
+      s.trav_by_steps = kTravBySteps;
     }
     if (!stacks && hctr[4 + steps]) {  // more steps than planned
       walked = false;

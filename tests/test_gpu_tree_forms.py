@@ -166,3 +166,30 @@ def test_one_leaf(prec, ncrit):
     assert s.num_cells() == (1, 0)
     ref = fmm.direct(x, x, q)
     assert (np.abs(t[:, 0] - ref[:, 0]) <= (2e-6 if prec == "f32" else 1e-13) * ref[:, 0]).all()
+
+
+def test_traversal_after_stack_overflow():
+    """A handle whose traversal has overflowed a block's stack takes steps for a while, for inputs
+    that would fit too, and then the stacks again: by the kernels that its solves launch."""
+    launches = fmm.load_library().fmm_b200_kernel_launches
+    rng = np.random.default_rng(9)
+    corner = np.array([[i & 1, i >> 1 & 1, i >> 2] for i in range(8)]) - 0.5
+    x = np.concatenate([c + rng.uniform(-1, 1, (768, 3)) * 5e-4 for c in corner])
+    y, w = bodies("cube", 500, rng, "f32")
+    kw = dict(P=4, theta=1e-5, ncrit=16, use_ropt=0, nspawn=1)
+
+    def count(s):
+        n = launches()
+        s.solve(y, w)
+        return launches() - n
+
+    fresh = fmm.Solver(**kw)
+    count(fresh)
+    few = count(fresh)
+    lists = fresh.lists()
+    s = fmm.Solver(**kw)
+    s.solve(x, np.ones(len(x)))
+    counts = [count(s) for _ in range(40)]
+    for a, b in zip(s.lists(), lists):
+        assert np.array_equal(a, b)
+    assert counts[0] > few and counts[-1] == few
