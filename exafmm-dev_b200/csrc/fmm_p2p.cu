@@ -602,7 +602,6 @@ void order_p2p_targets(SolverBase& s) {
   FMM_LAUNCH_CHECK();
   FMM_CUDA(cudaMemcpyAsync(s.scal_host + kP2PTeamsHost, teams, 4 * sizeof(int),
                            cudaMemcpyDeviceToHost, s.stream));
-  s.p2p_ordered = true;
 }
 
 template <typename T> void run_p2p(Solver<T>& s) {

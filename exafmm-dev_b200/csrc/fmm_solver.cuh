@@ -175,12 +175,11 @@ struct SolverBase {
   cudaEvent_t p2p_ready = nullptr;
   DevArr<int> m2l_tgt;       // M2L target cells by descending pair count
   DevArr<unsigned> tgt_key;  // scratch of their ordering
-  // P2P target leaves in launch order (valid while p2p_ordered: the lists of the last
-  // traversal), each with its source bodies; scratch of the ordering
+  // target leaves of the last P2P lists in launch order, each with its source bodies; scratch of
+  // the ordering
   DevArr<int4> p2p_order;
   DevArr<int> p2p_nsrc, p2p_bucket, p2p_work, p2p_hist;
   DevArr<unsigned long long> p2p_srcs;  // source leaves of the P2P pairs as k_p2p reads them
-  bool p2p_ordered = false;
   int m2l_ntgt = 0;
   DevArr<double> dtmp;  // host <-> device conversion scratch
   // phase timing

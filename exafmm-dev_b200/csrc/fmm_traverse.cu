@@ -900,7 +900,6 @@ void finish_p2p_list(SolverBase& s) {
 template <typename T> void build_lists(Solver<T>& s, bool defer_p2p) {
   const int TB = 256;
   s.nm2l = s.np2p = s.p2p_body_pairs = 0;
-  s.p2p_ordered = false;
   if (s.ncells == 0) return;
   if (s.ncells > (int)kCellMask)
     throw FmmError(FMM_ERR_NOT_SUPPORTED, "more than 2^27 - 1 cells (list pairs hold 27-bit cells)");

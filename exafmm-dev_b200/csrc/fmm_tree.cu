@@ -853,7 +853,6 @@ template <typename T> void build_tree(Solver<T>& s, bool radii) {
   const int n = s.n;
   const int TB = 256;
   s.kc_valid = false;  // the host copies of the cells' index fields are stale
-  s.p2p_ordered = false;  // so is the P2P target order of the last traversal
   s.radii_set = false;
   s.level_lo.clear();
   s.ncells = s.maxlevel = s.nleaves = 0;
