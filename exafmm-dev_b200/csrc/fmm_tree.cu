@@ -1049,12 +1049,8 @@ template <typename T> void build_tree(Solver<T>& s, bool radii) {
     FMM_LAUNCH_CHECK();
   }
   // leaves of more bodies than a warp ranks: stable sort by leaf-truncated key from input order
-  if (levels < kMaxLevel) {
-    k_keys<T><<<ceil_div(n, TB), TB, 0, s.stream>>>(s.bodies_in.p, n, s.box.p, s.root_first,
-                                                    nroots, s.keys.p, s.idx.p);
-    FMM_LAUNCH_CHECK();
-    forest_sort(s, s.keys.p, s.keys2.p, s.idx.p, s.idx2.p, n, nroots, 3 * kMaxLevel);
-  }
+  // (the keys are sorted on every digit here: such leaves come with a large ncrit, which plans no
+  // levels, or lie on the last level)
   int* blev = s.idx.p;
   k_leaf_levels<<<ceil_div(nnodes, TB), TB, 0, s.stream>>>(nnodes, s.nchildn.p, s.nbegin.p,
                                                            s.ncount.p, s.nlevel.p, blev);
