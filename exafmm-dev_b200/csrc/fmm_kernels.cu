@@ -408,28 +408,39 @@ void op_p2p(Solver<T>& s, int n, const int* ci, const int* cj, const int* image,
   if (L.pairs.empty() || !s.n) return;
   check_disjoint_bodies(s, L.targets, "P2P");
   const int nt = (int)L.targets.size();
-  upload_pairs(s, L, s.p2p, s.p2p_off);
-  upload_list(s, nt, L.targets.data());
+  finish(s);  // the solver's P2P lists are replaced
+  // A few pairs are put in launch order on the host; above the size of a copy that the driver
+  // takes without a wait (64 KB) the device does it from the uploaded pairs (5,000 leaves each on
+  // itself 1.68 ms a call, 1.90 on the host).
+  const bool few = L.pairs.size() + nt <= 4096;
+  if (few) {
+    order_p2p_pairs(s, L.pairs, L.off, L.targets);
+  } else {
+    upload_pairs(s, L, s.p2p, s.p2p_off);
+    upload_list(s, nt, L.targets.data());
+  }
   // save the targets, let the P2P write its sums, add the saved values back
   s.k_trg.ensure(2 * (size_t)s.n);
   FMM_CUDA(cudaMemcpyAsync(s.k_trg.p, s.trg_s.p, sizeof(vec4<T>) * s.n, cudaMemcpyDeviceToDevice,
                            s.stream));
   FMM_CUDA(cudaMemcpyAsync(s.k_trg.p + s.n, s.trg_e.p, sizeof(vec4<T>) * s.n,
                            cudaMemcpyDeviceToDevice, s.stream));
-  std::swap(s.leaves, s.k_list);
   const int nl = s.nleaves;
   const double e2 = s.cfg.eps2;
+  if (!few) std::swap(s.leaves, s.k_list);
   s.nleaves = nt;
   s.cfg.eps2 = eps2;
   auto restore = [&] {
-    std::swap(s.leaves, s.k_list);
+    if (!few) std::swap(s.leaves, s.k_list);
     s.nleaves = nl;
     s.cfg.eps2 = e2;
   };
   try {
     s.np2p = (long long)L.pairs.size();
-    order_p2p_targets(s);
-    FMM_CUDA(cudaStreamSynchronize(s.stream));  // its team counts
+    if (!few) {
+      order_p2p_targets(s);
+      FMM_CUDA(cudaStreamSynchronize(s.stream));  // its team counts
+    }
     run_p2p(s);
   } catch (...) {
     restore();
@@ -437,10 +448,10 @@ void op_p2p(Solver<T>& s, int n, const int* ci, const int* cj, const int* image,
   }
   restore();
   k_kmerge<T><<<ceil_div(32LL * nt, 256), 256, 0, s.stream>>>(
-      nt, s.k_list.p, s.c_ibody.p, s.c_nbody.p, s.k_trg.p, s.n, s.trg_s.p, s.trg_e.p);
+      nt, few ? s.p2p_nsrc.p + nt : s.k_list.p, s.c_ibody.p, s.c_nbody.p, s.k_trg.p, s.n,
+      s.trg_s.p, s.trg_e.p);
   FMM_LAUNCH_CHECK();
   s.np2p = 0;
-  finish(s);
 }
 
 }  // namespace

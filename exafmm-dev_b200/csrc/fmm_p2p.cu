@@ -37,6 +37,7 @@
 #include <algorithm>
 #include <climits>
 #include <type_traits>
+#include <vector>
 
 #include "fmm_solver.cuh"
 
@@ -230,9 +231,9 @@ __device__ __forceinline__ void p2p_fold(Target<T>* t, Accum<T, COMP>& acc, int 
 }
 
 // A source leaf as k_p2p reads it: first body in bits 0-30, image in 31-35, bodies above.
-__device__ __forceinline__ unsigned long long p2p_leaf(int4 info, int img) {
-  return (unsigned long long)(unsigned)info.w | (unsigned long long)img << 31 |
-         (unsigned long long)(unsigned)info.z << 36;
+__host__ __device__ __forceinline__ unsigned long long p2p_leaf(int body, int n, int img) {
+  return (unsigned long long)(unsigned)body | (unsigned long long)img << 31 |
+         (unsigned long long)(unsigned)n << 36;
 }
 
 // Positions [p0, p1) of the target leaf's source bodies (the bodies of its source leaves in
@@ -486,9 +487,9 @@ constexpr int kP2PBuckets = 4 * kSubBuckets;
 // `share` pairs per lane of a warp or more, so that the team's start and its merge (about 500
 // instructions a warp) stay small beside its pairs.  One warp for a count that no int holds, and
 // with periodic images (see p2p_lanes).
-__device__ __forceinline__ int p2p_class(unsigned long long src, int nb, int share) {
+__host__ __device__ __forceinline__ int p2p_class(unsigned long long src, int nb, int share) {
   if (src > INT_MAX / 2) return 3;
-  const unsigned long long w = src * (unsigned long long)min(64, (nb + 3) / 4 * 4) / 32;
+  const unsigned long long w = src * (unsigned long long)(nb < 61 ? (nb + 3) / 4 * 4 : 64) / 32;
   return w >= 8ULL * share ? 0 : w >= 4ULL * share ? 1 : w >= 2ULL * share ? 2 : 3;
 }
 
@@ -508,7 +509,7 @@ __global__ void __launch_bounds__(256)
       const unsigned p = (unsigned)pairs[k];
       const int4 f = info[pair_cell(p)];
       src += (unsigned)f.z;
-      srcs[k] = p2p_leaf(f, pair_img(p));
+      srcs[k] = p2p_leaf(f.w, f.z, pair_img(p));
     }
     src = warp_sum(src);
     if (lane == 0) {
@@ -578,6 +579,53 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+static int p2p_share(const SolverBase& s) {
+  return s.cfg.images > 0 ? INT_MAX : s.cfg.precision == FMM_FP32 ? 512 : 192;
+}
+
+// The launch order of a few pairs that the host lists (a single-operator call: CSR offsets per
+// cell, the cells' bodies in kc_ibody and kc_nbody), worked out there: no kernel and no wait for
+// the team counts (one pair of leaves 0.060 ms a call with the device's order, 0.038 now).  The
+// targets follow their source counts in p2p_nsrc; inside a team size they keep call order.
+void order_p2p_pairs(SolverBase& s, const std::vector<unsigned long long>& pairs,
+                     const std::vector<int>& off, const std::vector<int>& targets) {
+  const size_t np = pairs.size(), nt = targets.size();
+  std::vector<unsigned long long> srcs(np);
+  std::vector<int4> order(nt);
+  std::vector<int> nsrc(nt), cls(nt), sorted(2 * nt);
+  int* teams = s.scal_host + kP2PTeamsHost;
+  std::fill(teams, teams + 4, 0);
+  for (size_t t = 0; t < nt; t++) {
+    const int c = targets[t];
+    unsigned long long src = 0;
+    for (int k = off[c]; k < off[c + 1]; k++) {
+      const unsigned p = (unsigned)pairs[k];
+      const int j = pair_cell(p);
+      src += (unsigned)s.kc_nbody[j];
+      srcs[k] = p2p_leaf(s.kc_ibody[j], s.kc_nbody[j], pair_img(p));
+    }
+    cls[t] = p2p_class(src, s.kc_nbody[c], p2p_share(s));
+    nsrc[t] = (int)std::min<unsigned long long>(src, INT_MAX);
+    teams[cls[t]]++;
+  }
+  int at[4] = {0, teams[0], teams[0] + teams[1], teams[0] + teams[1] + teams[2]};
+  for (size_t t = 0; t < nt; t++) {
+    const int c = targets[t], i = at[cls[t]]++;
+    order[i] = make_int4(s.kc_ibody[c], s.kc_nbody[c], off[c], off[c + 1]);
+    sorted[i] = nsrc[t];
+    sorted[nt + t] = c;
+  }
+  s.p2p_srcs.ensure(np);
+  s.p2p_order.ensure(nt);
+  s.p2p_nsrc.ensure(2 * nt);
+  auto up = [&](void* dst, const void* src, size_t bytes) {
+    FMM_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s.stream));
+  };
+  up(s.p2p_srcs.p, srcs.data(), np * sizeof(srcs[0]));
+  up(s.p2p_order.p, order.data(), nt * sizeof(order[0]));
+  up(s.p2p_nsrc.p, sorted.data(), 2 * nt * sizeof(int));
+}
+
 // the launch order of the current P2P lists, on the solver's current stream; the team counts
 // reach s.scal_host (kP2PTeamsHost) once that stream has been waited for
 void order_p2p_targets(SolverBase& s) {
@@ -593,8 +641,7 @@ void order_p2p_targets(SolverBase& s) {
   FMM_CUDA(cudaMemsetAsync(hist, 0, 2 * kP2PBuckets * sizeof(int), s.stream));
   k_p2p_work<<<std::min(ceil_div(nl, 8), 148 * 4), 256, 0, s.stream>>>(
       nl, s.leaves.p, s.p2p_off.p, s.p2p.p, s.c_info.p, s.p2p_srcs.p,
-      s.p2p_bucket.p, s.p2p_work.p, hist,
-      s.cfg.images > 0 ? INT_MAX : s.cfg.precision == FMM_FP32 ? 512 : 192);
+      s.p2p_bucket.p, s.p2p_work.p, hist, p2p_share(s));
   FMM_LAUNCH_CHECK();
   k_p2p_place<<<std::min(ceil_div(nl, 256), 148 * 4), 256, 0, s.stream>>>(
       nl, s.leaves.p, s.p2p_bucket.p, s.p2p_work.p, hist, s.p2p_off.p, s.c_info.p, cursor, teams,

@@ -224,6 +224,8 @@ template <typename T> void downward_l2l(Solver<T>& s);        // fmm_passes.cu: 
 template <typename T> void downward_l2p(Solver<T>& s);        // fmm_passes.cu: L2P + output
 template <typename T> void build_lists(Solver<T>& s, bool defer_p2p = false);  // fmm_traverse.cu
 void order_p2p_targets(SolverBase& s);  // fmm_p2p.cu: launch order of the current P2P lists
+void order_p2p_pairs(SolverBase& s, const std::vector<unsigned long long>& pairs,
+                     const std::vector<int>& off, const std::vector<int>& targets);
 constexpr int kTreeHost = 320;           // scal_host: control block of the tree kernel
 constexpr int kP2PTeamsHost = 480;      // scal_host: its four team counts, after a wait
 void fill_cell_info(SolverBase& s);     // fmm_tree.cu: c_info from the cells' index fields

@@ -174,3 +174,27 @@ def test_operator_arguments_are_checked(datasets):
     s.kernel_p2m([1, 2])
     s.kernel_m2m([0])
     assert np.isfinite(s.expansion(0)).all()
+
+
+@pytest.mark.parametrize("images", [0, 1])
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("n,few", [(9001, False), (400, True)])
+def test_p2p_launch_order(n, few, prec, images):
+    """P2P over all pairs of a solve's lists as one operator call: bit for bit the solve's near
+    field (the same teams for the same lists).  A few pairs take two launches of this library's
+    kernels, the pairs' sums and the merge with the saved targets."""
+    rng = np.random.default_rng(4)
+    x = np.concatenate([rng.uniform(-1, 1, (n - n // 4, 3)), rng.uniform(-1, 1, (n // 4, 3)) * 0.02])
+    q = rng.uniform(-1, 1, n)
+    # an opening angle that no pair of cells meets: the solve is its near field
+    s = fmm.Solver(P=4, theta=1e-5, ncrit=80, precision=prec, use_ropt=0, images=images, cycle=2.0)
+    s.solve(x, q)
+    m2l, p2p = (np.asarray(a).astype(np.int64) for a in s.lists())
+    assert len(m2l) == 0
+    want = s.trg()[s.order()]
+    s.kernel_set_trg(None)
+    before = fmm.kernel_launches()
+    s.kernel_p2p(p2p >> 32, p2p & (2 ** 27 - 1), p2p >> 27 & 31)
+    assert (fmm.kernel_launches() - before == 2) == few
+    # (sums and error terms are added in double there, in the working precision by a solve)
+    assert np.array_equal(s.kernel_trg().astype(s.dtype), want.astype(s.dtype))
