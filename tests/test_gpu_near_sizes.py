@@ -4,8 +4,9 @@ up by hand, so sizes are exact.
 
 Tolerances.  FP64: sums of up to 1e4 terms of one sign for the potential, each within a few
 eps (2.2e-16): 1e-13 of the sum of magnitudes.  FP32: a term's relative error is at most about
-12 eps (6e-8; three rounded differences, r^2, a reciprocal square root within 2 ulp cubed), the
-compensated sum adds none: 2e-6 of the sum of magnitudes."""
+12 eps (6e-8; three rounded differences, r^2, a reciprocal square root within 2 ulp cubed); a lane
+adds up to 16 terms plainly in either half of its sums, and then the halves, before a compensated
+fold, which adds none: 16 eps more, 28 in all or 1.7e-6 of the sum of magnitudes: 2e-6."""
 import importlib
 
 import numpy as np

@@ -46,7 +46,15 @@ def test_tree_forms(prec, ncrit):
         x, q = bodies(kind, n, rng, prec)
         if kind == "same":
             # the reference recurses without end on coincident bodies: against the stages only
+            s.set_bodies(x, q)
+            s.build_tree()
+            s.upward_pass()
+            s.traverse()
+            R, lists = s.cells()["R"], s.lists()
             s.solve(x, q)
+            assert np.array_equal(s.cells()["R"], R)
+            for got, ref in zip(s.lists(), lists):
+                assert np.array_equal(got, ref)
             c = s.cells()
             assert c["nbody"][0] == n and c["level"].max() == 21
             leaf = c["nchild"] == 0
