@@ -11,15 +11,15 @@ use_rmax = use_ropt = 1, FP32 expansions with compensated potential/gradient sum
   outside its events.
 * e2e: the same solve through the host C ABI (fmm_b200_solve_host: pinned double x, q in,
   p, f out, host<->device copies inside the timed region).
-* roofline: the M2L kernel (the largest phase), FP32-pipe bound.  achieved = the algorithmic
-  flops of the reference's M2L loop, 8 sum_{j<P} (j+1)(P-j)^2 per cell pair (a complex
-  multiply-add = 8 flops; 9,680 at P = 10), times the run's M2L pairs, over the M2L phase's
-  event-timed duration; peak = the nominal FP32 rate 148 SMs x 128 lanes x 2 flops x the SM
-  clock sampled during the timed solves (the FMA throughput measured by fmm_b200_fp32_peak
-  is reported beside it).  The flops the kernel actually executes (the contraction in the
-  source's azimuthal frame with the +m and -m terms folded, and the rotations: 3,440 per pair at
-  P = 10, the harmonics apart) are reported as executed_tflops: fewer than the counted ones, so
-  frac may pass 1.
+* roofline: the M2L kernel (the largest phase), FP32-pipe bound.  achieved = the flops that the
+  kernel executes per cell pair (the contraction in the source's azimuthal frame with the +m and
+  -m terms folded, and the rotations: 3,440 at P = 10, the harmonics apart), times the run's M2L
+  pairs, over the M2L phase's event-timed duration; peak = the nominal FP32 rate 148 SMs x 128
+  lanes x 2 flops x the SM clock sampled during the timed solves (the FMA throughput measured by
+  fmm_b200_fp32_peak is reported beside it).  The rate in the flops of the reference's M2L loop,
+  8 sum_{j<P} (j+1)(P-j)^2 per pair (a complex multiply-add = 8 flops; 9,680 at P = 10), is
+  reported as reference_count_tflops: it compares M2L times with the reference's and is no
+  fraction of a peak.
 * cpu_baseline: the reference exafmm-dev CPU FMM (oracle/_ref/perf, compiled from the
   reference's sources) on the same workload (N = 2^20) with all host threads, median of 3
   runs, per phase.
@@ -892,8 +892,8 @@ def main():
                                                      local, args.steps, clk_mhz,
                                                      not args.no_cpu_baseline)
 
-    # roofline of M2L (the largest phase): algorithmic flops per pair of the reference's loop
-    # over the phase's event time, against the nominal FP32 rate at the sampled SM clock
+    # roofline of M2L (the largest phase): the kernel's flops per pair over the phase's event
+    # time, against the nominal FP32 rate at the sampled SM clock
     probe = fmm.fp32_peak_tflops(local)
     peak = nominal_fp32_tflops(clk_mhz)
     m2l_tflops = nm2l * m2l_flops_per_pair(WORKLOAD["P"]) / (phases["m2l"] * 1e-3) / 1e12
@@ -944,11 +944,11 @@ def main():
         "e2e": {"value": e2e_value, "unit": "particles/s", "h2d_bytes_per_step": 32 * n,
                 "d2h_bytes_per_step": 32 * n, "ms_per_step": e2e_total / len(e2e_ms)},
         "roofline": {"kernel": "M2L (k_m2l_fold<float,10>)", "bound": "fp32",
-                     "achieved": m2l_tflops, "peak": peak, "unit": "TFLOP/s",
-                     "frac": m2l_tflops / peak, "traffic": traffic,
-                     "flops_per_pair": m2l_flops_per_pair(WORKLOAD["P"]),
-                     "executed_tflops": m2l_exec, "probe_tflops": probe,
-                     "frac_of_probe": m2l_tflops / probe,
+                     "achieved": m2l_exec, "peak": peak, "unit": "TFLOP/s",
+                     "frac": m2l_exec / peak, "traffic": traffic,
+                     "flops_per_pair": m2l_executed_flops_per_pair(WORKLOAD["P"]),
+                     "reference_count_tflops": m2l_tflops, "probe_tflops": probe,
+                     "frac_of_probe": m2l_exec / probe,
                      "peak_source": "nominal FP32: 148 SMs x 128 lanes x 2 flops x %.0f MHz "
                                     "(SM clock sampled during the timed solves); "
                                     "MEASURED_PEAKS.json has no FP32 figure; probe_tflops = "
