@@ -315,8 +315,8 @@ static int autotune_ncrit_t(Solver<T>& s, const int* cand, int ncand, int repeat
 }
 
 // P2P lane-group autotuner: on the lists of the handle's last solve, each candidate pair of
-// leaf-size thresholds (4 lanes per target up to g4 bodies, 2 up to g2) runs the P2P
-// `repeats` times after one untimed run; the median device time decides.
+// leaf-size thresholds (SolverBase::p2p_g4, p2p_g2) runs the P2P `repeats` times after one
+// untimed run; the median device time decides.
 template <typename T>
 static int autotune_p2p_t(Solver<T>& s, const int* g4, const int* g2, int ncand, int repeats,
                           int* best, double* times_ms) {

@@ -22,9 +22,9 @@
 // Bound: the FMA pipe (FP64: the FP64 pipe), 26 cycles a source pair and target, at 50-65 %
 // of it: the rest is idle target slots, the chunks' staging and latency at 16 warps per SM.
 // FP32, one warp per leaf and one to two targets per lane before: Plummer 2^20, P = 10
-// (0.99 G pairs, 18 bodies a leaf) 1.08 -> 0.91 ms; 256 solves (14.4 G pairs) 14.4 -> 12.0 ms;
+// (0.99 G pairs, 18 bodies a leaf) 1.08 -> 0.89 ms; 256 solves (14.4 G pairs) 14.4 -> 12.1 ms;
 // cube of 200,003 (1.28 G, 49 a leaf) 1.19 -> 0.89 ms; sphere of 2^22 (1.23 G, 13 a leaf) 1.98
-// -> 1.82 ms.  Measured beside it on the 256 solves: four targets per lane 13.8 ms against
+// -> 1.90 ms.  Measured beside it on the 256 solves: four targets per lane 13.8 ms against
 // 13.6 (128 registers either way), two at 24 warps per SM 14.4 ms; accumulators in registers
 // 15.6 ms; chunks of 64 bodies 14.1 ms; teams twice as large 12.9 ms.
 //

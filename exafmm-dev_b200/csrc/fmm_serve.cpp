@@ -125,8 +125,11 @@ void copy_jobs(const std::vector<CopyJob>& jobs) {
   for (auto& t : ts) t.join();
 }
 
-// device memory of one solve in the batched solver (bodies, sort scratch, tree, expansions,
-// interaction lists), an upper-end estimate used for admission
+// What admission counts for one solve: bodies, sort scratch, tree, expansions and interaction
+// lists, each once and at typical lengths.  Not a bound: a handle keeps its arrays at up to twice
+// what its largest batch needed, with the traversal's frontiers and stacks and the kernels'
+// reordered copies beside them (256 solves of 9.2 M bodies at P = 8: 1.9 GB counted, 6.9 GB held),
+// so a budget wants room for four times as much on the device.
 size_t estimate_bytes(const fmm_b200_config& c, int n, int P) {
   const size_t ncoef = c.basis == FMM_SPHERICAL ? (size_t)P * (P + 1) : (size_t)P * (P + 1) * (P + 2) / 6;
   const size_t real = c.precision == FMM_FP64 ? 8 : 4;

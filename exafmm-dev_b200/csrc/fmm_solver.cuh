@@ -144,8 +144,9 @@ struct SolverBase {
   int trav_by_steps = 0;  // traversals to take by steps, since a block's stack has overflowed
   int tree_plan = 0;        // levels of the handle's last tree (0: none)
   int write_r = 1;          // P2M / M2M set the cell radii (else the structure pass did)
-  // P2P lanes per target by target leaf size: 4 up to p2p_g4 bodies, 2 up to p2p_g2, else 1
-  // (p2p_g4 <= 8 and p2p_g2 <= 16: a warp holds 32 / lanes targets); fmm_b200_autotune_p2p
+  // limits of the P2P lanes per target by target leaf size, p2p_g4 <= 8 and p2p_g2 <= 16
+  // (fmm_b200_autotune_p2p): 4 lanes up to p2p_g4 bodies, 2 up to p2p_g2, else 1; in FP32 without
+  // images 8 up to half as many again as p2p_g4, 4 up to that of p2p_g2, 2 up to 48, else 1
   int p2p_g4 = 8, p2p_g2 = 16;
   DevArr<int> tree_ctl;     // control block of the tree kernel
   int tree_most = 0;        // its blocks that the device holds at a time (0: not asked yet)

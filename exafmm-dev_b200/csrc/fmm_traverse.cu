@@ -159,7 +159,7 @@ __device__ __forceinline__ void trav_step(const TravArgs<T>& g, const vec4<T>* _
     int ty[kTravItems], k[kTravItems];
     int2 p[kTravItems];
     unsigned v = 0;  // packed: M2L in bits 0-8, P2P in 9-17, children in 18-31 (warp totals:
-                     // <= 256, <= 256, <= 8192)
+                     // <= 128, <= 128, <= 4096)
 #pragma unroll
     for (int u = 0; u < kTravItems; u++) {
       ty[u] = -1;
@@ -174,8 +174,8 @@ __device__ __forceinline__ void trav_step(const TravArgs<T>& g, const vec4<T>* _
                pair_img((unsigned)p[u].y) < 27;
     if constexpr (sizeof(T) == 4) {
       // FP32: all the items' cell data loaded before any is classified, so that the gathers
-      // of the four pairs are in flight together (FP64 cells take twice the registers: one
-      // pair at a time)
+      // of the pairs are in flight together (FP64 cells take twice the registers: one pair at
+      // a time)
       vec4<T> ca[kTravItems], cb[kTravItems];
       int4 fa[kTravItems], fb[kTravItems];
 #pragma unroll
@@ -779,8 +779,8 @@ template <typename T> static void upload_roots(Solver<T>& s, int2* front) {
 // until the frontier is some four times as long as there are cells (a step makes about 20 pairs
 // of one; from a frontier a quarter as long the blocks' shares differ by far more: 30,003 bodies
 // in images 0.37 ms against 0.26), then k_traverse; should one of its stacks overflow, this and
-// the handle's next kTravBySteps traversals take steps only.  Larger trees: steps only, as many as the last
-// traversal took, two more per level that the tree has grown by since, and two to spare (at
+// the handle's next kTravBySteps traversals take steps only.  Larger trees: steps only, as many as
+// the last traversal took, two more per level that the tree has grown by since, and two to spare (at
 // first as many as any tree needs).  Against all steps in one cooperative kernel with a barrier
 // between them the traverse phase of 1,000 bodies takes 0.16 instead of 0.19 ms, of 200,003 0.26
 // instead of 0.31, of 250,007 in the uniform tree 0.25 instead of 0.27; 2^22 on a sphere (361,000

@@ -25,7 +25,8 @@ namespace {
 // memory, the slices' in k_direct_sum, in slice order.  Bound by the FP64 pipe (about 22
 // operations a pair with the reciprocal square root).  The slices fill the GPU whatever the
 // number of targets: with a thread per target and no slices, 1,024 targets were four blocks
-// (2^20 sources: 183 ms; the whole call now takes 4.5 ms, 2.5 ms of it the copies).
+// (2^20 sources: 183 ms of kernel, now 2.0; the whole call takes 4.5 to 9 ms, the rest of it the
+// allocation and the copies of pageable host memory, whose time varies that much).
 constexpr int kDirTile = 256;
 constexpr int kDirTargets = 64;
 constexpr int kDirBlocks = 148 * 4;  // blocks wanted on the GPU: one wave at 4 per SM

@@ -291,7 +291,8 @@ int fmm_b200_autotune_p2p(fmm_b200_solver* s, const int* lanes4_max, const int* 
 /* ---- serving: continuous batching of independent solves ------------------------------ *
  * A server owns nworkers worker threads (one CUDA stream and one solver handle per order
  * each) and a scheduler that batches pending requests of equal order P, in arrival order,
- * within hbm_budget_bytes of estimated device memory, max_batch solves and 2^21 bodies
+ * within hbm_budget_bytes of estimated device memory (bodies, tree, expansions and lists once;
+ * handles hold up to four times that), max_batch solves and 2^21 bodies
  * per batch (a larger request rides alone).  Each worker holds pinned host staging for
  * 2^21 bodies (128 MB) from the start, and sizes each new handle (the first request of an
  * order on a worker) with two synthetic batches of 2^21 bodies before it takes requests, so
