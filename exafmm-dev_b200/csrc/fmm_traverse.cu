@@ -731,10 +731,11 @@ static int mutual_of(const SolverBase& s) {
   return s.cfg.mutual && s.cfg.images == 0 && !s.ij ? 1 : 0;
 }
 
-// the first frontier (s.nfront0 pairs) to `front`, which root_count() pairs fit
+// pairs of the first frontier at most
 static int root_count(const SolverBase& s) {
   return s.ij ? s.nroots == 2 : s.nroots * (s.cfg.images > 0 ? 27 : 1);
 }
+// the first frontier, s.nfront0 pairs, to `front`
 template <typename T> static void upload_roots(Solver<T>& s, int2* front) {
   // one (root, root) pair per solve of the batch (lists never cross solves); with periodic
   // images one per shift of the source tree, in the reference's image order (:250-260)
